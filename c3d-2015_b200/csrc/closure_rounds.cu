@@ -1094,7 +1094,12 @@ __global__ void __launch_bounds__(RWN * 32)
 }
 
 // ---------------------------------------------------------------- host side
+//
+// The file is compiled once per C3D_ROUNDS_PART (Makefile): part 0 holds the shared host code and
+// the dispatch, the other parts each instantiate rounds_t for a few orders, so that the
+// orders compile in parallel.
 
+#if C3D_ROUNDS_PART == 0
 template <int NT> static size_t state_bytes_t() { return sizeof(CellState<NT>); }
 
 size_t rounds_state_bytes(int nm)
@@ -1131,6 +1136,7 @@ size_t mixed_a_chunk_bytes(int nm2, int fmt)
     const int na = nm2p < 128 ? 128 : nm2p;
     return (size_t)na * QC * (fmt == 0 ? 2 : 8);
 }
+#endif
 
 template <int NT, int KIND, bool ZD> static size_t mixed_pass_smem(const ClosureParams &P, int nm2)
 {
@@ -1164,9 +1170,10 @@ struct TierHandles {
     cudaGraphConditionalHandle h[NLISTS];
 };
 
+#if C3D_ROUNDS_PART != 0
 // Picks each used list's launch size (SWITCH branch; NTIER = none) from its counter (bit l of
 // mask marks list l as used) and clears the counters of the lists the round fills.
-__global__ void rounds_tier_kernel(const Lists in, Lists out, TierHandles th, unsigned int mask,
+static __global__ void rounds_tier_kernel(const Lists in, Lists out, TierHandles th, unsigned int mask,
                                    long long cap, unsigned long long *launches)
 {
     if (threadIdx.x != 0)
@@ -1192,7 +1199,7 @@ __global__ void rounds_tier_kernel(const Lists in, Lists out, TierHandles th, un
 }
 
 // Entries past cap stay for the next round: appended to that round's list.
-__global__ void rounds_carry_kernel(const Lists in, Lists out, unsigned int mask, long long cap)
+static __global__ void rounds_carry_kernel(const Lists in, Lists out, unsigned int mask, long long cap)
 {
     __shared__ unsigned int base[NLISTS];
     for (int l = 0; l < NLISTS; ++l) {
@@ -1212,7 +1219,7 @@ __global__ void rounds_carry_kernel(const Lists in, Lists out, unsigned int mask
 
 // Loop condition after the body's two rounds: more work and the round limit not reached;
 // past the limit the closure stops with errorFlag 2 (c3d_sync: C3D_ERR_TIMEOUT).
-__global__ void rounds_cond_kernel(const Lists in, unsigned int mask, unsigned int *rounds,
+static __global__ void rounds_cond_kernel(const Lists in, unsigned int mask, unsigned int *rounds,
                                    long long maxRounds, int *errorFlag,
                                    cudaGraphConditionalHandle loop, unsigned long long *launches)
 {
@@ -1233,7 +1240,7 @@ __global__ void rounds_cond_kernel(const Lists in, unsigned int mask, unsigned i
     if (launches)
         atomicAdd(launches, 1ull);
 }
-
+#else
 // Appends a conditional node after the current dependencies of the graph being captured on st.
 cudaError_t capture_conditional(cudaStream_t st, cudaGraphConditionalHandle h,
                                        cudaGraphConditionalNodeType type, unsigned int size,
@@ -1270,6 +1277,7 @@ std::mutex &graph_build_mutex()
     static std::mutex m;
     return m;
 }
+#endif
 
 // The instantiated closure graphs of the last few configurations (a configuration is every
 // launch parameter; switching, e.g., between precisions reuses its graph), with the streams
@@ -1300,6 +1308,7 @@ template <class T> static void key_add(std::vector<unsigned char> &k, const T &v
     k.insert(k.end(), b, b + sizeof(T));
 }
 
+#if C3D_ROUNDS_PART == 0
 std::vector<unsigned char> rounds_graph_key(const RoundsLaunch &R, bool gaunt)
 {
     std::vector<unsigned char> k;
@@ -1322,8 +1331,9 @@ std::vector<unsigned char> rounds_graph_key(const RoundsLaunch &R, bool gaunt)
     key_add(k, gaunt);
     return k;
 }
+#endif
 
-template <int NT, int NT2, bool GAUNT> static cudaError_t rounds_t(const RoundsLaunch &R)
+template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &R)
 {
     const ClosureParams &P = *R.P;
     CellState<NT> *state = reinterpret_cast<CellState<NT> *>(R.state);
@@ -1343,7 +1353,7 @@ template <int NT, int NT2, bool GAUNT> static cudaError_t rounds_t(const RoundsL
     const bool probe = GAUNT && P.probe;
     const size_t probeSmem = RWN * sizeof(ProbeSlot<NT>);
     size_t passSmem, mixSmem[3] = {0, 0, 0};
-    if (GAUNT) {
+    if constexpr (GAUNT) {
         passSmem = GSTAGES * (size_t)(R.nm2 + 1) * QCP * 8 + (size_t)QC * CST2 * 8 +
                    (size_t)(RWP * P.nm + 1) * 8 + GSTAGES * 8;
         e = cudaFuncSetAttribute(rounds_pass_gaunt_kernel<NT, NT2>,
@@ -1438,7 +1448,7 @@ template <int NT, int NT2, bool GAUNT> static cudaError_t rounds_t(const RoundsL
                         nullptr, 0, FirstRound{});
             }
         } else {
-            if (GAUNT)
+            if constexpr (GAUNT)
                 rounds_pass_gaunt_kernel<NT, NT2>
                     <<<(unsigned)((nb + RWP - 1) / RWP), RW * 32, passSmem, s>>>(
                         P, R.chunks, R.nm2, la, nb, nDev, state, R.buf, R.errorFlag);
@@ -1662,6 +1672,46 @@ template <int NT, int NT2, bool GAUNT> static cudaError_t rounds_t(const RoundsL
     return cudaSuccess;
 }
 
+#if C3D_ROUNDS_PART == 0
+#define C3D_ROUNDS extern template
+#else
+#define C3D_ROUNDS template
+#endif
+#define C3D_ROUNDS_T(NT, NT2, G) C3D_ROUNDS cudaError_t rounds_t<NT, NT2, G>(const RoundsLaunch &);
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 1
+C3D_ROUNDS_T(1, 1, true)
+C3D_ROUNDS_T(1, 2, true)
+C3D_ROUNDS_T(2, 4, true)
+C3D_ROUNDS_T(2, 7, true)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 2
+C3D_ROUNDS_T(4, 11, true)
+C3D_ROUNDS_T(1, 1, false)
+C3D_ROUNDS_T(2, 1, false)
+C3D_ROUNDS_T(3, 1, false)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 3
+C3D_ROUNDS_T(5, 16, true)
+C3D_ROUNDS_T(4, 1, false)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 4
+C3D_ROUNDS_T(7, 22, true)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 5
+C3D_ROUNDS_T(8, 29, true)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 6
+C3D_ROUNDS_T(5, 1, false)
+C3D_ROUNDS_T(6, 1, false)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 7
+C3D_ROUNDS_T(7, 1, false)
+#endif
+#if C3D_ROUNDS_PART == 0 || C3D_ROUNDS_PART == 8
+C3D_ROUNDS_T(8, 1, false)
+#endif
+
+#if C3D_ROUNDS_PART == 0
 void *rounds_graph_new() { return new RoundsGraph(); }
 void rounds_graph_free(void *g) { delete reinterpret_cast<RoundsGraph *>(g); }
 
@@ -1700,5 +1750,6 @@ cudaError_t launch_closure_rounds(const RoundsLaunch &R, bool gaunt)
     default: return cudaErrorInvalidValue;
     }
 }
+#endif // C3D_ROUNDS_PART == 0
 
 } // namespace c3d
