@@ -482,7 +482,7 @@ __host__ __device__ constexpr int probe_entry_doubles(int nmp) { return nmp + 8;
 // ZD (the mixed closure's passes): the exponents of the chunk as a DMMA GEMM
 // Z[32 x 16] = M_chunk^T [32 x nm] alpha [nm x 16] (warp w: directions 8 (w % 4) .., cells
 // 8 (w / 4) ..) staged through shared memory, instead of the reference's unfused order.
-constexpr int ZS = 18; // row stride (cells) of the exponent tile: 16-byte pairs, 8-lane phases
+[[maybe_unused]] constexpr int ZS = 18; // row stride (cells) of the exponent tile: 16-byte pairs, 8-lane phases
                        // conflict-free
 
 // The first round of a closure with the convergence certificate: no list and no set-up
@@ -508,8 +508,8 @@ struct FirstRound {
     const int *psiValid;
     int gnx, gny, gnz;
 };
-constexpr int PSTR = 17; // row stride (cells) of the probe's psi tile
-constexpr int PRS = 3;   // stages of the mixed probe's psi read ring (chunks k .. k + 2)
+[[maybe_unused]] constexpr int PSTR = 17; // row stride (cells) of the probe's psi tile
+[[maybe_unused]] constexpr int PRS = 3;   // stages of the mixed probe's psi read ring (chunks k .. k + 2)
 
 // 8-byte asynchronous global -> shared copy (zero fill when !valid; src is not read then)
 __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid)
@@ -1333,6 +1333,7 @@ std::vector<unsigned char> rounds_graph_key(const RoundsLaunch &R, bool gaunt)
 }
 #endif
 
+#if C3D_ROUNDS_PART != 0
 template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &R)
 {
     const ClosureParams &P = *R.P;
@@ -1672,7 +1673,10 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
     return cudaSuccess;
 }
 
+#endif // C3D_ROUNDS_PART != 0
+
 #if C3D_ROUNDS_PART == 0
+template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &R);
 #define C3D_ROUNDS extern template
 #else
 #define C3D_ROUNDS template
