@@ -56,9 +56,18 @@ cudaError_t launch_kinetic_flux(const GridDims &g, const double *alpha, const do
                                 bool psiReady, double *flux, int *errorFlag,
                                 const int *wrapFlag, cudaStream_t st);
 bool kinetic_staged_used(const GridDims &g, int runLen);
-cudaError_t launch_psi_handoff(const GridDims &g, int nq, const double *M, const double *alpha,
-                               bool faceCopy, const int *refresh, const unsigned int *refreshCount,
-                               double *psi, int *psiValid, int numSMs, cudaStream_t st);
+cudaError_t launch_sym_ansatz(const SymTables &T, int deg, long long nall, const double *alpha,
+                              const long long *list, const unsigned int *count, int r0, int r1, int isPn,
+                              double *psi, int numSMs, cudaStream_t st);
+cudaError_t launch_sym_flux(const GridDims &g, int deg, const double *psi, const double *tab,
+                            const int *idx, int r0, int r1, double theta, double *flux,
+                            const int *wrapFlag, int numSMs, cudaStream_t st);
+cudaError_t launch_psi_face_copy(const GridDims &g, int nq, double *psi, cudaStream_t st);
+cudaError_t launch_psi_refresh(const GridDims &g, int nq, const double *M, const double *alpha,
+                               const long long *list, const unsigned int *count, double *psi,
+                               int numSMs, cudaStream_t st);
+cudaError_t launch_psi_groups(const GridDims &g, unsigned char *mark, long long *list,
+                              unsigned int *count, int numSMs, cudaStream_t st);
 size_t flux_frag_doubles(int nm, int nq, int which);
 cudaError_t launch_reproject(const GridDims &g, double *u, double *alpha, const double *mfA,
                              const double *mfP, int nq, int *errorFlag, cudaStream_t st);
@@ -146,7 +155,8 @@ struct c3d_ctx {
     bool psiReady = false;
     bool psiHandoffPending = false;     // the closure's probe wrote psi; completed in closure_grid
     bool handoff = true;                // c3d_set_ansatz_handoff
-    int *psiRefresh = nullptr;          // cells whose psi is rewritten after the closure
+    unsigned char *psiMark = nullptr;   // cells whose psi is rewritten after the closure,
+    long long *psiRefresh = nullptr;    // their groups of 8 cells
     unsigned int *psiRefreshCount = nullptr;
     // device flag: psi holds the ansatz of every cell but the face ghosts for the current
     // multipliers (set by a closure's hand-off, cleared by whatever may break that)
@@ -209,6 +219,12 @@ struct c3d_ctx {
     int *mirrorHost = nullptr;     // pinned
     bool mirror = true;
     long long mirroredClosures = 0;
+    // octant-symmetric quadrature (sym.cuh; no = 0: the general kernels): tables of the flux, of
+    // its ansatz, and (Gaunt form) of the closure's probe and Hessian passes
+    int deg = 0;
+    SymTables symPsi{}, symN{}, sym2{};
+    double *symFlux = nullptr;
+    double *symBuf[3] = {nullptr, nullptr, nullptr}; // allocations of symPsi, symN, sym2
     double *gChunksC = nullptr;    // work-list engine: chunks of nm2 M2 rows + the weight row
     GauntTerm *gStream = nullptr;  // tiled assembly streams of the work-list engine
     int gStreamLen = 0;
@@ -266,7 +282,8 @@ static void free_ctx(c3d_ctx *c)
                     c->rCounts, c->rBuf, c->mfA, c->mfP, c->cellMap, c->mirrorFlag,
                     c->gChunksC, c->cellGamma, c->cellErr, c->lineLog, c->mixF64,
                     c->mixA[0], c->mixA[1], c->cellCond, c->g0, c->psiRefresh,
-                    c->psiRefreshCount, c->xSplit[0], c->xSplit[1], c->psiValid};
+                    c->psiRefreshCount, c->psiMark, c->xSplit[0], c->xSplit[1], c->psiValid, c->symBuf[0],
+                    c->symBuf[1], c->symBuf[2]};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
@@ -288,6 +305,36 @@ static void free_ctx(c3d_ctx *c)
     if (c->ownStream && c->stream)
         cudaStreamDestroy(c->stream);
     delete c;
+}
+
+// Uploads the tables of a symmetric quadrature into one allocation, *buf (null: a failed
+// allocation; the previous one is freed).
+static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **buf)
+{
+    if (*buf)
+        cudaFree(*buf);
+    *buf = nullptr;
+    T = SymTables{};
+    std::vector<double> all;
+    auto add = [&](const void *src, size_t bytes) {
+        const size_t at = all.size(), n = (bytes + 127) / 128 * 16; // 128-byte aligned parts
+        all.resize(at + n);
+        std::memcpy(all.data() + at, src, bytes);
+        return at;
+    };
+    const size_t e = add(H.expo.data(), H.expo.size() * 8), p = add(H.proj.data(), H.proj.size() * 8),
+                 w = add(H.w.data(), H.w.size() * 8), s = add(H.stepIdx.data(), H.stepIdx.size() * 4),
+                 i = add(H.idx.data(), H.idx.size() * 4), f = add(H.flux.data(), H.flux.size() * 8);
+    if (cudaMalloc(buf, all.size() * 8) != cudaSuccess) {
+        cudaGetLastError();
+        *buf = nullptr;
+        return;
+    }
+    cudaMemcpy(*buf, all.data(), all.size() * 8, cudaMemcpyHostToDevice);
+    T = SymTables{H.no,     H.nb,     *buf + e, *buf + p,
+                  *buf + w, (const int *)(*buf + s), (const int *)(*buf + i)};
+    if (flux)
+        *flux = *buf + f;
 }
 
 // psi no longer matches the multipliers (or may not): the next hand-off closure writes all of it.
@@ -387,6 +434,11 @@ c3d_status c3d_create(const c3d_params *p, const double *M, const double *w, con
     flux_frags(nm, nq, M, w, xi, eta, mu, 1.0 / p->dx, 1.0 / p->dy, 1.0 / p->dz, mfA.data(),
                mfP.data());
     ok = ok && alloc((void **)&c->mfA, mfA.size() * 8) && alloc((void **)&c->mfP, mfP.size() * 8);
+    c->deg = sq - 1;
+    SymHost sh;
+    if (ok && sym_build(c->deg, c->deg, nq, M, w, xi, eta, mu, 1.0 / p->dx, 1.0 / p->dy,
+                        1.0 / p->dz, sh))
+        sym_upload(sh, c->symPsi, &c->symFlux, &c->symBuf[0]), ok = c->symBuf[0] != nullptr;
     if (ok && pnOps)
         ok = alloc((void **)&c->pnops, (size_t)6 * nm * nm * 8);
     if (!ok) {
@@ -573,6 +625,8 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
         R.nm2 = c->nm2;
         R.gstream = c->gStream;
         R.streamLen = c->gStreamLen;
+        R.symN = c->symN;
+        R.sym2 = c->sym2;
         R.m0 = c->m0;
         R.ncells = n;
         R.cellMap = cellMap;
@@ -620,13 +674,18 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
             R.launchDev = c->launchDev;
         }
         R.psi = nullptr;
-        if (gridRecords && c->cp.probe && c->handoff && c->solver == 1) {
+        // (a symmetric basis with asymmetric Gaunt tables: psi's row orders differ)
+        if (gridRecords && c->cp.probe && c->handoff && c->solver == 1 &&
+            (c->symN.no > 0) == (c->symPsi.no > 0)) {
             // hand the probe's ansatz to the kinetic flux when psi of every direction fits the
             // budget
             const size_t need = (size_t)c->nq * c->g.nall() * 8;
             if (need <= c->psiBytes) {
                 if (!c->psiRefresh) {
-                    C3D_CUDA(cudaMalloc(&c->psiRefresh, (size_t)c->g.nall() * sizeof(int)));
+                    const size_t groups = (size_t)(c->g.nall() + 7) / 8;
+                    C3D_CUDA(cudaMalloc(&c->psiMark, groups * 8));
+                    C3D_CUDA(cudaMemsetAsync(c->psiMark, 0, groups * 8, c->stream));
+                    C3D_CUDA(cudaMalloc(&c->psiRefresh, groups * sizeof(long long)));
                     C3D_CUDA(cudaMalloc(&c->psiRefreshCount, sizeof(unsigned int)));
                     C3D_CUDA(cudaMalloc(&c->psiValid, sizeof(int)));
                     C3D_CUDA(cudaMemset(c->psiValid, 0, sizeof(int)));
@@ -640,11 +699,9 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
                     c->psiAlloc = need;
                     C3D_CUDA(cudaMemset(c->psiValid, 0, sizeof(int)));
                 }
-                C3D_CUDA(cudaMemsetAsync(c->psiRefreshCount, 0, sizeof(unsigned int), st));
                 R.psi = c->psi;
                 R.psiNall = c->g.nall();
-                R.refresh = c->psiRefresh;
-                R.refreshCount = c->psiRefreshCount;
+                R.mark = c->psiMark;
                 R.psiValid = c->psiValid;
                 R.gnx = c->g.nx;
                 R.gny = c->g.ny;
@@ -742,6 +799,49 @@ c3d_status c3d_closure(c3d_ctx *c)
     return C3D_OK;
 }
 
+// The cells the closure marked get psi of their final multipliers; then (faceCopy) face ghosts
+// copy their images' -- in that order, so that they copy no stale values.
+static cudaError_t handoff_launch(c3d_ctx *c, bool faceCopy, cudaStream_t st)
+{
+    cudaError_t e = launch_psi_groups(c->g, c->psiMark, c->psiRefresh, c->psiRefreshCount,
+                                      c->numSMs, st);
+    if (e == cudaSuccess)
+        e = c->symPsi.no > 0
+            ? launch_sym_ansatz(c->symPsi, c->deg, c->g.nall(), c->alpha, c->psiRefresh,
+                                c->psiRefreshCount, 0, c->nq, 0, c->psi, c->numSMs, st)
+            : launch_psi_refresh(c->g, c->nq, c->M, c->alpha, c->psiRefresh, c->psiRefreshCount,
+                                 c->psi, c->numSMs, st);
+    // psi now holds every non-face-ghost cell's ansatz for the final multipliers
+    if (e == cudaSuccess && c->psiValid)
+        e = cudaMemsetAsync(c->psiValid, 1, sizeof(int), st);
+    if (e == cudaSuccess && faceCopy)
+        e = launch_psi_face_copy(c->g, c->nq, c->psi, st);
+    return e;
+}
+
+// The kinetic flux of a (device, grid layout): psi chunk by chunk of directions (all at once when
+// ready: the closure handed it over), stencil and projection.
+static cudaError_t flux_launch(c3d_ctx *c, const double *a, int isPn, bool ready,
+                               const int *wrapFlag, cudaStream_t st)
+{
+    if (c->symPsi.no == 0)
+        return launch_kinetic_flux(c->g, a, c->mfA, c->mfP, c->xi, c->eta, c->nq, c->qChunk,
+                                   c->runLen, c->theta, isPn, c->psi, ready, c->flux, c->errorFlag,
+                                   wrapFlag, st);
+    const int step = ready ? c->nq : c->qChunk;
+    cudaError_t e = cudaSuccess;
+    for (int r0 = 0; r0 < c->nq && e == cudaSuccess; r0 += step) {
+        const int r1 = std::min(c->nq, r0 + step);
+        if (!ready)
+            e = launch_sym_ansatz(c->symPsi, c->deg, c->g.nall(), a, nullptr, nullptr, r0, r1, isPn,
+                                  c->psi, c->numSMs, st);
+        if (e == cudaSuccess)
+            e = launch_sym_flux(c->g, c->deg, c->psi, c->symFlux, c->symPsi.idx, r0, r1, c->theta,
+                                c->flux, wrapFlag, c->numSMs, st);
+    }
+    return e;
+}
+
 // Completes the ansatz hand-off of a grid closure whose probe pass wrote psi: face ghosts
 // copied from their images (mirrored closures), the listed cells recomputed from their final
 // multipliers; the next kinetic flux then runs the stencil alone.
@@ -750,8 +850,7 @@ static c3d_status finish_handoff(c3d_ctx *c, bool faceCopy)
     if (!c->psiHandoffPending)
         return C3D_OK;
     c->psiHandoffPending = false;
-    C3D_CUDA(launch_psi_handoff(c->g, c->nq, c->M, c->alpha, faceCopy, c->psiRefresh,
-                                c->psiRefreshCount, c->psi, c->psiValid, c->numSMs, c->stream));
+    C3D_CUDA(handoff_launch(c, faceCopy, c->stream));
     c->launches += faceCopy ? 2 : 1;
     c->psiReady = true;
     return C3D_OK;
@@ -1099,6 +1198,23 @@ c3d_status c3d_set_gaunt(c3d_ctx *c, int nm2, const double *M2, const int *rowPt
     c3d_status s = build_mixed_chunks(c, nm2, M2, wh);
     if (s != C3D_OK)
         return s;
+    // octant-symmetric passes; the probe's tables come from the same columns of M2 as the
+    // Hessian passes', so that both form the same gradient
+    c->symN = c->sym2 = SymTables{};
+    std::vector<double> M1((size_t)nq * nm);
+    for (int q = 0; q < nq; ++q)
+        std::copy(M2 + (size_t)q * nm2, M2 + (size_t)q * nm2 + nm, M1.data() + (size_t)q * nm);
+    SymHost h1, h2;
+    if (c->symPsi.no > 0 &&
+        sym_build(c->deg, c->deg, nq, M1.data(), wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h1) &&
+        sym_build(2 * c->deg, c->deg, nq, M2, wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h2)) {
+        sym_upload(h1, c->symN, nullptr, &c->symBuf[1]);
+        sym_upload(h2, c->sym2, nullptr, &c->symBuf[2]);
+        if (!c->symBuf[1] || !c->symBuf[2]) {
+            c->symN = c->sym2 = SymTables{};
+            return fail(C3D_ERR_OOM, "c3d_set_gaunt: device allocation failed");
+        }
+    }
     return build_certificate(c, nm2, M2, wh, rowPtr, colInd, val);
 }
 
@@ -1401,9 +1517,7 @@ c3d_status c3d_flux_kinetic(c3d_ctx *c, int alphaIsU)
         psi_invalidate(c); // the ansatz kernel writes psi
     cudaEvent_t t0 = nullptr;
     timing_begin(c, &t0);
-    C3D_CUDA(launch_kinetic_flux(c->g, a, c->mfA, c->mfP, c->xi, c->eta, c->nq, c->qChunk,
-                                 c->runLen, c->theta, isPn, c->psi, ready, c->flux,
-                                 c->errorFlag, nullptr, c->stream));
+    C3D_CUDA(flux_launch(c, a, isPn, ready, nullptr, c->stream));
     timing_end(c, 1, t0);
     int nch = ceil_div(c->nq, c->qChunk);
     c->launches += ready ? 1 : 2 * nch;
@@ -1433,8 +1547,8 @@ c3d_status c3d_autotune(c3d_ctx *c, int *qChunk, int *runLen, double *msPerCall)
             qs.push_back(q);
     }
     std::vector<int> ls{0};
-    if (c->g.nz % 32 == 0 && c->g.nz > 32)
-        ls.push_back(32);
+    if (c->symPsi.no == 0 && c->g.nz % 32 == 0 && c->g.nz > 32)
+        ls.push_back(32); // (the symmetric stencil has one tile shape)
     const int q0 = c->qChunk, l0 = c->runLen;
     const bool timing = c->timing;
     c->psiReady = false; // every timed call forms the ansatz
@@ -1581,7 +1695,8 @@ static std::vector<unsigned char> stage_key(const c3d_ctx *c, int stage, double 
     skey(c->rBatchUse);
     const void *ptrs[] = {c->psi, c->rState, c->rBuf, c->rListA, c->rCounts, c->cellMap,
                           c->gChunksC, c->chunks, c->gStream, c->mixF64, c->mixA[0],
-                          c->mixA[1], c->g0, c->psiRefresh, c->launchDev, c->u, c->alpha};
+                          c->mixA[1], c->g0, c->psiRefresh, c->launchDev, c->u, c->alpha,
+                          c->symN.expo, c->sym2.expo};
     for (const void *p : ptrs)
         skey(p);
     return key;
@@ -1601,7 +1716,8 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
     // mirrored closure with the hand-off and the staged stencil: the face ghosts' psi is not
     // copied; the stencil reads their periodic images (the mirror flag tells it, on the device,
     // which closure body ran)
-    const bool wrap = mirrorPath && handoff && kinetic_staged_used(c->g, c->runLen);
+    const bool wrap = mirrorPath && handoff &&
+                      (c->symPsi.no > 0 || kinetic_staged_used(c->g, c->runLen));
     const long long l0 = c->launches;
     long long n = 0;
     cudaStream_t s0 = cs[0];
@@ -1642,8 +1758,7 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
                                         c->stats, c->numSMs, sk);
         }
         if (er == cudaSuccess && R.psi)
-            er = launch_psi_handoff(c->g, c->nq, c->M, c->alpha, mirrored && !wrap, c->psiRefresh,
-                                    c->psiRefreshCount, c->psi, c->psiValid, c->numSMs, sk);
+            er = handoff_launch(c, mirrored && !wrap, sk);
         return er;
     };
     if (ec == cudaSuccess && mirrorPath) {
@@ -1678,9 +1793,7 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
     if (ec == cudaSuccess && !handoff && c->psiValid) // the ansatz kernel writes psi
         ec = cudaMemsetAsync(c->psiValid, 0, sizeof(int), s0);
     if (ec == cudaSuccess)
-        ec = launch_kinetic_flux(c->g, c->alpha, c->mfA, c->mfP, c->xi, c->eta, c->nq, c->qChunk,
-                                 c->runLen, c->theta, 0, c->psi, handoff, c->flux, c->errorFlag,
-                                 wrap ? c->mirrorFlag : nullptr, s0);
+        ec = flux_launch(c, c->alpha, 0, handoff, wrap ? c->mirrorFlag : nullptr, s0);
     if (ec == cudaSuccess)
         ec = launch_euler(c->g, c->u, c->flux, c->sigT, c->sigS, dt, c->numSMs, s0);
     if (ec == cudaSuccess && stage == 1)

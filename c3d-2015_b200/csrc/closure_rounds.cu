@@ -20,6 +20,7 @@
 #include <mutex>
 #include <vector>
 #include "rounds_launch.h"
+#include "sym.cuh"
 #include "umma.cuh"
 
 #include <cuda_bf16.h>
@@ -496,12 +497,11 @@ struct FirstRound {
     const double *u, *alpha;
     // ansatz hand-off to the kinetic flux (grid closures with the certificate): the probe pass
     // writes psi[q nall + c] = exp(alpha_c . m_q) of every cell it solves, and the probe's
-    // Newton kernel lists in refresh the cells whose multipliers may still change (their psi is
+    // Newton kernel marks the cells whose multipliers may still change (their psi is
     // rewritten after the closure). Null psi: no hand-off.
     double *psi;
     long long nall;
-    int *refresh;
-    unsigned int *refreshCount;
+    unsigned char *mark;
     // nonzero: psi already holds the ansatz of every cell but the face ghosts for the closure's
     // starting multipliers (the previous closure's final ones), so the probe writes only the
     // face ghosts' (gnx, gny, gnz: the interior sizes that tell them)
@@ -909,6 +909,275 @@ __global__ void __launch_bounds__(RW * 32, KIND == 1 ? 1 : KIND == 2 ? 3 : 2)
     }
 }
 
+// ---------------------------------------------------------------- octant-symmetric passes
+// The passes of a context whose quadrature has the octant symmetry (sym.cuh). A warp owns 8
+// cells; per block of 8 octant directions a lane forms the 16 exponents of cell lane / 4 at 2
+// octant directions x 8 reflections (sym_expand, one DMMA per 4 multipliers of a parity
+// class), their exponentials and the class sums of w e^{alpha.m} (sym_wht), which the DMMAs of
+// sym_contract project onto the class members straight from registers. The tables of a block
+// are staged by bulk copies, SYM_STAGES deep, one barrier per block.
+
+constexpr int SYM_STAGES = 3;
+[[maybe_unused]] constexpr int SYM_PASS_WARPS = 4;
+[[maybe_unused]] constexpr int SYM_PROBE_WARPS = 8;
+
+// Degree of the basis of rounds_t<NT, NT2, true>.
+__host__ __device__ constexpr int sym_order(int nt2)
+{
+    return nt2 == 1 ? 0 : nt2 == 2 ? 1 : nt2 == 4 ? 2 : nt2 == 7 ? 3 : nt2 == 11 ? 4 : nt2 == 16 ? 5
+         : nt2 == 22 ? 6 : 7;
+}
+
+// Doubles of a staged block: expansion fragments of degree DEG, projection fragments of degree PD.
+template <int DEG, int PD> struct SymStage {
+    static constexpr int EXPO = SymCls<DEG>::STEPS * 32;
+    static constexpr int PROJ = 2 * SymCls<PD>::TILES * 32;
+    static constexpr int DOUBLES = EXPO + PROJ;
+};
+template <int DEG, int PD, int WARPS> constexpr size_t sym_smem()
+{
+    return (size_t)(SYM_STAGES * SymStage<DEG, PD>::DOUBLES + WARPS * SymCls<DEG>::STEPS * 32) * 8;
+}
+
+// Loads block b of the tables into stage b % SYM_STAGES (one thread).
+template <int DEG, int PD>
+__device__ __forceinline__ void sym_stage_load(const SymTables &T, int b, double *stage, uint64_t *full)
+{
+    using G = SymStage<DEG, PD>;
+    const int s = b % SYM_STAGES;
+    double *st = stage + s * G::DOUBLES;
+    mbar_expect_tx(&full[s], G::DOUBLES * 8);
+    bulk_g2s(st, T.expo + (size_t)b * G::EXPO, G::EXPO * 8, &full[s]);
+    bulk_g2s(st + G::EXPO, T.proj + (size_t)b * G::PROJ, G::PROJ * 8, &full[s]);
+}
+
+// What a trial pass computes besides f: with fused trials the moments at the trial point, which
+// the Newton kernel uses when it accepts the trial (the next iteration's Hessian visit then
+// needs no pass of its own). Not fused when that visit belongs to a reduced-precision list.
+__device__ __forceinline__ bool trial_fused(const ClosureParams &P, int fp64, int iter, double cnd)
+{
+    return !P.mixed || fp64 || iter + 1 > P.mixIterMax || cnd > P.condMixMax;
+}
+
+// Hessian and trial pass over the listed cells (the FP64 list): the nm2 extended moments of
+// cells that need them into momBuf (stride 8 NT2) and f's sum of trial cells into their state.
+template <int NT, int NT2>
+__global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
+    sym_pass_kernel(ClosureParams P, SymTables T, const int *__restrict__ list, int n,
+                    const unsigned int *nDev, CellState<NT> *state, double *__restrict__ momBuf,
+                    int *errorFlag)
+{
+    n = round_entries(n, nDev);
+    constexpr int WARPS = SYM_PASS_WARPS, DEG = sym_order(NT2), PD = 2 * DEG;
+    if (blockIdx.x * (8 * WARPS) >= n)
+        return;
+    using C = SymCls<DEG>;
+    using E = SymCls<PD>;
+    using G = SymStage<DEG, PD>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    double *stage = reinterpret_cast<double *>(smem_raw);
+    __shared__ uint64_t full[SYM_STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *aF = stage + SYM_STAGES * G::DOUBLES + warp * C::STEPS * 32;
+    if (tid == 0) {
+        for (int s = 0; s < SYM_STAGES; ++s)
+            mbar_init(&full[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        for (int b = 0; b < SYM_STAGES && b < T.nb; ++b)
+            sym_stage_load<DEG, PD>(T, b, stage, full);
+    }
+    const int pos = (blockIdx.x * WARPS + warp) * 8 + (lane >> 2);
+    long long cell = -1;
+    bool trial = false, wantH = false;
+    if (pos < n) {
+        cell = list[pos];
+        const SlotScalars &sc = state[cell].s;
+        trial = sc.need == NEED_TRIAL;
+        wantH = sc.need == NEED_H || (trial && trial_fused(P, sc.fp64, sc.iter, sc.cnd));
+    }
+#pragma unroll
+    for (int k = 0; k < C::STEPS; ++k) {
+        const int m = T.stepIdx[4 * k + (lane & 3)];
+        aF[k * 32 + lane] = cell >= 0 && m >= 0 ? state[cell].alpha[m] : 0.0;
+    }
+    const bool any = __any_sync(FULL_MASK, cell >= 0), anyH = __any_sync(FULL_MASK, wantH);
+    double acc[E::TILES][2];
+#pragma unroll
+    for (int t = 0; t < E::TILES; ++t)
+        acc[t][0] = acc[t][1] = 0.0;
+    double f = 0.0;
+    __syncthreads();
+    for (int b = 0; b < T.nb; ++b) {
+        const double *st = stage + (b % SYM_STAGES) * G::DOUBLES;
+        const bool ok = mbar_wait(&full[b % SYM_STAGES], (b / SYM_STAGES) & 1);
+        if (any) {
+            double v[2][8];
+            sym_expand<DEG>(aF, st, lane, v);
+            const double2 w = *reinterpret_cast<const double2 *>(T.w + SYM_BLK * b + 2 * (lane & 3));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    v[e][s] = (e == 0 ? w.x : w.y) * exp(v[e][s]);
+                sym_wht(v[e]);
+                f += v[e][0];
+                if (anyH)
+                    sym_contract<PD>(v[e], st + G::EXPO + e * (E::TILES * 32), lane, acc);
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0)
+                atomicExch(errorFlag, 1);
+            return;
+        }
+        if (tid == 0 && b + SYM_STAGES < T.nb)
+            sym_stage_load<DEG, PD>(T, b + SYM_STAGES, stage, full);
+    }
+    if (wantH) {
+        double *o = momBuf + (size_t)pos * (8 * NT2);
+#pragma unroll
+        for (int t = 0; t < E::TILES; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int m = T.idx[8 * t + 2 * (lane & 3) + e];
+                if (m >= 0)
+                    o[m] = acc[t][e];
+            }
+    }
+    f += __shfl_xor_sync(FULL_MASK, f, 1);
+    f += __shfl_xor_sync(FULL_MASK, f, 2);
+    if (trial && (lane & 3) == 0)
+        state[cell].s.fquad = f;
+}
+
+// Probe pass of a closure's first round (FirstRound; see rounds_pass_mixed_kernel for the
+// hand-off's psi and the certificate's entry): first-order moments, f's sum and bounds of
+// e^{alpha.m} per cell. It always forms e^{alpha.m}: reading psi / u_0 back instead was no faster
+// (11.9 against 10.8 ms per M_6 128^3 closure). e_min and e_max come from the high words of the values (rounded outwards by 2^-20: the
+// certificate keeps factors of 2 and 4 in hand).
+template <int NT, int NT2>
+__global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
+    sym_probe_kernel(ClosureParams P, SymTables T, int n, double *__restrict__ out, int *errorFlag,
+                     FirstRound first)
+{
+    constexpr int WARPS = SYM_PROBE_WARPS, DEG = sym_order(NT2), NMP = 8 * NT;
+    using C = SymCls<DEG>;
+    using G = SymStage<DEG, DEG>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    double *stage = reinterpret_cast<double *>(smem_raw);
+    __shared__ uint64_t full[SYM_STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nm = P.nm;
+    double *aF = stage + SYM_STAGES * G::DOUBLES + warp * C::STEPS * 32;
+    if (tid == 0) {
+        for (int s = 0; s < SYM_STAGES; ++s)
+            mbar_init(&full[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        for (int b = 0; b < SYM_STAGES && b < T.nb; ++b)
+            sym_stage_load<DEG, DEG>(T, b, stage, full);
+    }
+    const int pos = (blockIdx.x * WARPS + warp) * 8 + (lane >> 2);
+    const bool emit = first.psi != nullptr;
+    const bool valid = emit && first.psiValid && *first.psiValid != 0;
+    long long gc = -1;
+    double u0 = 1.0, ascale = 0.0;
+    bool write = false;
+    if (pos < n) {
+        const long long c = first.off + pos;
+        gc = first.cellMap ? first.cellMap[c] : c;
+        u0 = first.u[gc * nm];
+        ascale = log(u0) * 2.0 * sqrt(M_PI);
+        write = emit;
+        if (valid) {
+            // only a face ghost's psi may be missing (its image's was read instead)
+            const int gz = first.gnz + 4, gy = first.gny + 4;
+            const int k = (int)(gc % gz), j = (int)((gc / gz) % gy), i = (int)(gc / gz / gy);
+            write = (i >= 2 && i < first.gnx + 2) + (j >= 2 && j < first.gny + 2) +
+                        (k >= 2 && k < first.gnz + 2) == 2;
+        }
+    }
+    const bool any = __any_sync(FULL_MASK, gc >= 0);
+#pragma unroll
+    for (int k = 0; k < C::STEPS; ++k) {
+        const int m = T.stepIdx[4 * k + (lane & 3)];
+        double a = gc >= 0 && m >= 0 ? first.alpha[gc * nm + m] : 0.0;
+        if (m == 0)
+            a -= ascale;
+        aF[k * 32 + lane] = a;
+    }
+    double acc[C::TILES][2];
+#pragma unroll
+    for (int t = 0; t < C::TILES; ++t)
+        acc[t][0] = acc[t][1] = 0.0;
+    double f = 0.0;
+    int lo = 0x7fffffff, hi = 0;
+    __syncthreads();
+    for (int b = 0; b < T.nb; ++b) {
+        const double *st = stage + (b % SYM_STAGES) * G::DOUBLES;
+        const bool ok = mbar_wait(&full[b % SYM_STAGES], (b / SYM_STAGES) & 1);
+        if (any) {
+            double v[2][8];
+            sym_expand<DEG>(aF, st, lane, v);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int o = SYM_BLK * b + 2 * (lane & 3) + e;
+                double *p = first.psi + (long long)(8 * o) * first.nall + gc;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    v[e][s] = exp(v[e][s]);
+                    if (write && o < T.no)
+                        p[(long long)s * first.nall] = u0 * v[e][s];
+                }
+            }
+            const double2 w = *reinterpret_cast<const double2 *>(T.w + SYM_BLK * b + 2 * (lane & 3));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (SYM_BLK * b + 2 * (lane & 3) + e < T.no)
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        lo = min(lo, __double2hiint(v[e][s]));
+                        hi = max(hi, __double2hiint(v[e][s]));
+                    }
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    v[e][s] *= e == 0 ? w.x : w.y;
+                sym_wht(v[e]);
+                f += v[e][0];
+                sym_contract<DEG>(v[e], st + G::EXPO + e * (C::TILES * 32), lane, acc);
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0)
+                atomicExch(errorFlag, 1);
+            return;
+        }
+        if (tid == 0 && b + SYM_STAGES < T.nb)
+            sym_stage_load<DEG, DEG>(T, b + SYM_STAGES, stage, full);
+    }
+    f += __shfl_xor_sync(FULL_MASK, f, 1);
+    f += __shfl_xor_sync(FULL_MASK, f, 2);
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, o));
+        hi = max(hi, __shfl_xor_sync(FULL_MASK, hi, o));
+    }
+    if (gc < 0)
+        return;
+    double *o = out + (size_t)pos * probe_entry_doubles(NMP);
+#pragma unroll
+    for (int t = 0; t < C::TILES; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int m = T.idx[8 * t + 2 * (lane & 3) + e];
+            if (m >= 0)
+                o[m] = acc[t][e];
+        }
+    if ((lane & 3) == 0) {
+        o[NMP] = f;
+        o[NMP + 1] = __hiloint2double(lo, 0);
+        o[NMP + 2] = __hiloint2double(hi, -1);
+    }
+}
+
 // Newton logic for the listed cells: one warp per cell, RWN cells per CTA, state staged
 // in shared memory with H in the tiled layout (TSlot).
 // MODE 0: FP64 Hessians and trials. MODE 1: the list of a mixed-precision pass (entries of
@@ -929,7 +1198,7 @@ __global__ void __launch_bounds__(RWN * 32)
                          const double *__restrict__ buf,
                          const GauntTerm *__restrict__ stream, int streamLen,
                          Outputs Og, Lists out, int level, const GauntTerm *__restrict__ g0,
-                         int g0n, FirstRound first)
+                         int g0n, FirstRound first, bool fused)
 {
     n = round_entries(n, nDev);
     if (blockIdx.x * RWN >= n)
@@ -957,7 +1226,7 @@ __global__ void __launch_bounds__(RWN * 32)
     const int pos = blockIdx.x * RWN + warp;
     const bool active = pos < n;
     const long long cell = active ? (list ? list[pos] : first.off + pos) : -1;
-    const bool needH = MODE != 2 && active && state[cell].s.need == NEED_H;
+    bool needH = MODE != 2 && active && state[cell].s.need == NEED_H;
     SlotT &sl = slots[warp];
     // probe visits: the probe entry's loads go out before the cell's state is read, so the
     // two global round trips overlap
@@ -969,8 +1238,8 @@ __global__ void __launch_bounds__(RWN * 32)
             for (int r = 0; r < PMR; ++r)
                 pmr[r] = lane + 32 * r < BSTR ? buf[(size_t)pos * BSTR + lane + 32 * r] : 0.0;
     C3D_NCLK_DECL
-    long long gcell = -1; // probe visits: the grid cell, for the ansatz hand-off's refresh list
-    if (MODE == 2 && active && first.refresh)
+    long long gcell = -1; // probe visits: the grid cell, for the ansatz hand-off's marks
+    if (MODE == 2 && active && first.mark)
         gcell = !list ? (first.cellMap ? (long long)first.cellMap[cell] : cell) : state[cell].s.cell;
     if (active) {
         if (MODE == 2 && !list)
@@ -981,6 +1250,19 @@ __global__ void __launch_bounds__(RWN * 32)
         sl.s.need = NEED_NONE;
     }
     bool nonFinite = false;
+    // fused trials: the pass also formed the moments at the trial point, so an accepted trial
+    // goes on to the next iteration's Hessian visit here (unless that iteration regularised,
+    // which moves the multipliers)
+    bool tried = false;
+    if constexpr (MODE == 0 && GAUNT) {
+        if (fused && active && !needH && sl.s.need == NEED_TRIAL) {
+            tried = true;
+            const bool moments = trial_fused(P, sl.s.fp64, sl.s.iter, sl.s.cnd);
+            const int reg = sl.s.regIndex;
+            after_trial(sl, P, O, lane, sl.s.fquad);
+            needH = moments && sl.s.need == NEED_H && sl.s.regIndex == reg;
+        }
+    }
     if constexpr (MODE == 2) {
     } else if (GAUNT) {
         double *mom = sl.scratch(); // g, d, alphaOld, rinv: NM2P <= 4 NMP doubles
@@ -994,10 +1276,14 @@ __global__ void __launch_bounds__(RWN * 32)
             nonFinite = __any_sync(FULL_MASK, nf);
         }
         if (__syncthreads_or(needH)) {
+            __shared__ int sNeedH[RWN];
+            if (lane == 0)
+                sNeedH[warp] = needH;
+            __syncthreads();
             bool hw[RWN];
 #pragma unroll
             for (int w = 0; w < RWN; ++w)
-                hw[w] = slots[w].s.need == NEED_H;
+                hw[w] = sNeedH[w] != 0;
             static_assert(RWN * 32 == NEWTON_THREADS, "stream layout");
             double h[RWN];
 #pragma unroll
@@ -1044,7 +1330,7 @@ __global__ void __launch_bounds__(RWN * 32)
             __syncwarp();
             after_probe(sl, P, O, lane, m0, sl.pm, g0, g0n);
         }
-    } else if (sl.s.need == NEED_H) {
+    } else if (needH) {
         if (lane == 0) {
             sl.s.hprec = MIX ? level : 0;
             if (P.mixed && O.stats)
@@ -1064,7 +1350,7 @@ __global__ void __launch_bounds__(RWN * 32)
             after_hessian(sl, P, O, lane, m0);
         }
         C3D_NCLK(O.stats, 5, lane);
-    } else if (sl.s.need == NEED_TRIAL) {
+    } else if (!tried && sl.s.need == NEED_TRIAL) {
         after_trial(sl, P, O, lane, sl.s.fquad);
         C3D_NCLK(O.stats, 7, lane);
     }
@@ -1072,7 +1358,7 @@ __global__ void __launch_bounds__(RWN * 32)
         // a cell that goes on past its probe visit (or failed there) may end with other
         // multipliers than the probe's: its psi is rewritten after the closure
         if (gcell >= 0 && lane == 0 && (sl.s.need != NEED_NONE || sl.s.status != CELL_OK))
-            first.refresh[atomicAdd(first.refreshCount, 1u)] = (int)gcell;
+            first.mark[gcell] = 1;
     }
     // a finished cell's state is not read again
     if (sl.s.need != NEED_NONE)
@@ -1316,8 +1602,8 @@ std::vector<unsigned char> rounds_graph_key(const RoundsLaunch &R, bool gaunt)
     const void *ptrs[] = {R.chunks, R.gstream, R.cellMap, R.u, R.alpha, R.iters, R.iterGamma,
                           R.regIdx, R.status, R.failCount, R.stats, R.gamma, R.normG, R.cond,
                           R.state, R.listA, R.listB, R.counts, R.buf, R.mixF64, R.mixA[0],
-                          R.mixA[1], R.g0, R.errorFlag, R.psi, R.refresh, R.refreshCount,
-                          R.launchDev};
+                          R.mixA[1], R.g0, R.errorFlag, R.psi, R.mark, R.launchDev,
+                          R.symN.expo, R.sym2.expo};
     for (const void *p : ptrs)
         key_add(k, p);
     key_add(k, R.nm2);
@@ -1354,7 +1640,22 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
     const bool probe = GAUNT && P.probe;
     const size_t probeSmem = RWN * sizeof(ProbeSlot<NT>);
     size_t passSmem, mixSmem[3] = {0, 0, 0};
+    // octant-symmetric quadrature: the passes of sym.cuh
+    const bool sym = GAUNT && R.symN.no > 0;
+    constexpr int DEG = sym_order(NT2);
+    constexpr size_t symPassSmem = sym_smem<DEG, 2 * DEG, SYM_PASS_WARPS>(),
+                     symProbeSmem = sym_smem<DEG, DEG, SYM_PROBE_WARPS>();
     if constexpr (GAUNT) {
+        if (sym) {
+            e = cudaFuncSetAttribute(sym_pass_kernel<NT, NT2>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)symPassSmem);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(sym_probe_kernel<NT, NT2>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)symProbeSmem);
+            if (e != cudaSuccess)
+                return e;
+        }
         passSmem = GSTAGES * (size_t)(R.nm2 + 1) * QCP * 8 + (size_t)QC * CST2 * 8 +
                    (size_t)(RWP * P.nm + 1) * 8 + GSTAGES * 8;
         e = cudaFuncSetAttribute(rounds_pass_gaunt_kernel<NT, NT2>,
@@ -1429,7 +1730,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                 rounds_newton_kernel<NT, NT2, GAUNT, 2>
                     <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, probeSmem, s>>>(
                         P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, l,
-                        mixed ? nullptr : R.g0, R.g0n, FirstRound{});
+                        mixed ? nullptr : R.g0, R.g0n, FirstRound{}, false);
             }
         } else if (l > 0) {
             // mixed-precision Hessian passes (Gaunt form only)
@@ -1446,21 +1747,27 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                 rounds_newton_kernel<NT, NT2, GAUNT, 1>
                     <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, newtonSmem, s>>>(
                         P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, l,
-                        nullptr, 0, FirstRound{});
+                        nullptr, 0, FirstRound{}, false);
             }
         } else {
-            if constexpr (GAUNT)
-                rounds_pass_gaunt_kernel<NT, NT2>
-                    <<<(unsigned)((nb + RWP - 1) / RWP), RW * 32, passSmem, s>>>(
-                        P, R.chunks, R.nm2, la, nb, nDev, state, R.buf, R.errorFlag);
-            else
+            if constexpr (GAUNT) {
+                constexpr int per = 8 * SYM_PASS_WARPS;
+                if (sym)
+                    sym_pass_kernel<NT, NT2>
+                        <<<(unsigned)((nb + per - 1) / per), SYM_PASS_WARPS * 32, symPassSmem, s>>>(
+                            P, R.sym2, la, nb, nDev, state, R.buf, R.errorFlag);
+                else
+                    rounds_pass_gaunt_kernel<NT, NT2>
+                        <<<(unsigned)((nb + RWP - 1) / RWP), RW * 32, passSmem, s>>>(
+                            P, R.chunks, R.nm2, la, nb, nDev, state, R.buf, R.errorFlag);
+            } else
                 rounds_pass_direct_kernel<NT>
                     <<<(unsigned)((nb + RW - 1) / RW), RW * 32, passSmem, s>>>(
                         P, R.chunks, la, nb, nDev, state, R.buf, R.errorFlag);
             rounds_newton_kernel<NT, NT2, GAUNT, 0>
                 <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, newtonSmem, s>>>(
                     P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, 0, nullptr,
-                    0, FirstRound{});
+                    0, FirstRound{}, sym);
         }
         return cudaGetLastError();
     };
@@ -1475,10 +1782,15 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                 for (long long off = 0; off < R.ncells; off += R.batch) {
                     const int nb = (int)((R.ncells - off) < R.batch ? (R.ncells - off) : R.batch);
                     const FirstRound fr{off,       R.cellMap,      R.u,      R.alpha,
-                                        R.psi,     R.psiNall,      R.refresh, R.refreshCount,
+                                        R.psi,     R.psiNall,      R.mark,
                                         R.psiValid, R.gnx,         R.gny,    R.gnz};
                     const unsigned grid = (unsigned)((nb + MXC - 1) / MXC);
-                    if (mixed)
+                    constexpr int per = 8 * SYM_PROBE_WARPS;
+                    const unsigned gridS = (unsigned)((nb + per - 1) / per);
+                    if (sym)
+                        sym_probe_kernel<NT, NT2><<<gridS, SYM_PROBE_WARPS * 32, symProbeSmem, s>>>(
+                            P, R.symN, nb, R.buf, R.errorFlag, fr);
+                    else if (mixed)
                         rounds_pass_mixed_kernel<NT, NT2, 2, true><<<grid, RW * 32, mixSmem[2], s>>>(
                             P, R.mixF64, nullptr, nullptr, nb, nullptr, state, R.buf, R.errorFlag,
                             fr);
@@ -1489,7 +1801,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                     rounds_newton_kernel<NT, NT2, GAUNT, 2>
                         <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, probeSmem, s>>>(
                             P, m0, nullptr, nb, nullptr, state, R.buf, R.gstream, R.streamLen, O,
-                            A, 3, mixed ? nullptr : R.g0, R.g0n, fr);
+                            A, 3, mixed ? nullptr : R.g0, R.g0n, fr, false);
                     *R.launches += 2;
                 }
             }

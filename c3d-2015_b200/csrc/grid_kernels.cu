@@ -173,21 +173,44 @@ __global__ void psi_face_copy_kernel(GridDims g, int nq, int qPer, double *__res
     }
 }
 
-// psi[q nall + c] = exp(alpha_c . m_q) for the *count cells c of list (one warp per cell,
-// directions over the lanes; exponent summed in the reference's order, unfused): the cells
-// whose multipliers the closure changed after its probe pass had written their psi.
+// The groups of 8 consecutive cells with a marked cell, as entries (group << 8) | mask in any
+// order, *count of them (zero before); the marks are cleared for the next closure.
+__global__ void psi_groups_kernel(unsigned long long *mark, long long groups, long long *list,
+                                  unsigned int *count)
+{
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < groups;
+         g += (long long)gridDim.x * blockDim.x) {
+        const unsigned long long m = mark[g];
+        if (m == 0)
+            continue;
+        mark[g] = 0;
+        int mask = 0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            mask |= ((m >> (8 * r)) & 0xff) ? 1 << r : 0;
+        list[atomicAdd(count, 1u)] = g << 8 | mask;
+    }
+}
+
+// psi[q nall + c] = exp(alpha_c . m_q) for the marked cells c of the *count groups of list (one
+// warp per group, directions over the lanes; exponent summed in the reference's order, unfused):
+// the cells whose multipliers the closure changed after its probe pass had written their psi.
 __global__ void psi_refresh_kernel(GridDims g, int nq, const double *__restrict__ M,
-                                   const double *__restrict__ alpha, const int *__restrict__ list,
+                                   const double *__restrict__ alpha,
+                                   const long long *__restrict__ list,
                                    const unsigned int *__restrict__ count, double *__restrict__ psi)
 {
     const int nm = g.nm;
     const long long nall = g.nall();
-    const unsigned int n = *count;
+    const long long n = 8LL * *count;
     const int lane = threadIdx.x & 31;
     const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long i = w0; i < n; i += nw) {
-        const long long c = list[i];
+        const long long e = list[i >> 3];
+        if (!((e >> (i & 7)) & 1))
+            continue;
+        const long long c = (e >> 8) * 8 + (i & 7);
         const double *a = alpha + c * nm;
         for (int q = lane; q < nq; q += 32) {
             const double *m = M + (size_t)q * nm;
@@ -890,20 +913,28 @@ cudaError_t launch_ghost_mirror_check(const GridDims &g, const double *a, int *f
     return cudaGetLastError();
 }
 
-// The refresh comes first: a face ghost copies its image's final psi, and the image may be
-// one of the refreshed cells.
-// psiValid (may be null): set once psi holds every non-face-ghost cell's ansatz for the final
-// multipliers, so that the next closure's probe pass need not write it again.
-cudaError_t launch_psi_handoff(const GridDims &g, int nq, const double *M, const double *alpha,
-                               bool faceCopy, const int *refresh, const unsigned int *refreshCount,
-                               double *psi, int *psiValid, int numSMs, cudaStream_t st)
+cudaError_t launch_psi_groups(const GridDims &g, unsigned char *mark, long long *list,
+                              unsigned int *count, int numSMs, cudaStream_t st)
 {
-    psi_refresh_kernel<<<2 * numSMs, 256, 0, st>>>(g, nq, M, alpha, refresh, refreshCount, psi);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && psiValid)
-        e = cudaMemsetAsync(psiValid, 1, sizeof(int), st);
-    if (e != cudaSuccess || !faceCopy)
+    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned int), st);
+    if (e != cudaSuccess)
         return e;
+    const long long groups = (g.nall() + 7) / 8;
+    psi_groups_kernel<<<grid_for(groups, 256, numSMs), 256, 0, st>>>(
+        reinterpret_cast<unsigned long long *>(mark), groups, list, count);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_psi_refresh(const GridDims &g, int nq, const double *M, const double *alpha,
+                               const long long *list, const unsigned int *count, double *psi,
+                               int numSMs, cudaStream_t st)
+{
+    psi_refresh_kernel<<<2 * numSMs, 256, 0, st>>>(g, nq, M, alpha, list, count, psi);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_psi_face_copy(const GridDims &g, int nq, double *psi, cudaStream_t st)
+{
     constexpr int QPER = 64;
     const long long threads = 4LL * g.ny * g.nz + 4LL * g.nx * g.nz + 2LL * g.nx * g.ny;
     const dim3 grid((unsigned)((threads + 255) / 256), (unsigned)ceil_div(nq, QPER));

@@ -2,6 +2,7 @@
 // context code that fills it.
 #pragma once
 #include "c3d_common.cuh"
+#include "sym.cuh"
 
 #include <cstddef>
 #include <mutex>
@@ -15,6 +16,7 @@ struct RoundsLaunch {
     int nm2;                   // Gaunt: extended moments (chunk rows: nm2 + the weight row)
     const GauntTerm *gstream;  // Gaunt: assembly streams, entry s of thread t at s*128 + t
     int streamLen;             // entries per thread
+    SymTables symN, sym2;      // octant-symmetric quadrature: tables of degree N and 2N (no = 0: none)
     double m0;                 // M[0][0]
     long long ncells;
     const int *cellMap;        // closure cell i -> grid cell cellMap[i] (null: identity)
@@ -43,12 +45,10 @@ struct RoundsLaunch {
     long long *hostSyncs; // host-driven rounds: one wait per round
     long long maxRounds;
     // ansatz hand-off to the kinetic flux (null psi: none): psi[q psiNall + c] of every cell
-    // the probe solves, and the list (with its device count) of cells whose psi is rewritten
-    // after the closure
+    // the probe solves, and a mark (nonzero) on the cells whose psi is rewritten after the closure
     double *psi;
     long long psiNall;
-    int *refresh;
-    unsigned int *refreshCount;
+    unsigned char *mark;
     // device flag: psi holds every non-face-ghost cell's ansatz for the starting multipliers
     // (the probe then writes only face ghosts); gnx..gnz the grid's interior sizes
     const int *psiValid;
