@@ -85,7 +85,7 @@ void flux_frags(int nm, int nq, const double *M, const double *w, const double *
                 const double *eta, const double *mu, double rdx, double rdy, double rdz,
                 double *mfA, double *mfP);
 cudaError_t launch_moment_flux(const GridDims &g, const double *u, const double *ops, double dx,
-                               double dy, double dz, double *flux, cudaStream_t st);
+                               double dy, double dz, double *flux, int numSMs, cudaStream_t st);
 } // namespace c3d
 
 
@@ -1604,7 +1604,8 @@ c3d_status c3d_flux_moment(c3d_ctx *c)
         return fail(C3D_ERR_INVALID, "c3d_flux_moment: null context");
     if (!c->pnops)
         return fail(C3D_ERR_INVALID, "c3d_flux_moment: no P_N operators in this context");
-    C3D_CUDA(launch_moment_flux(c->g, c->u, c->pnops, c->dx, c->dy, c->dz, c->flux, c->stream));
+    C3D_CUDA(launch_moment_flux(c->g, c->u, c->pnops, c->dx, c->dy, c->dz, c->flux, c->numSMs,
+                                c->stream));
     c->launches += 1;
     return C3D_OK;
 }

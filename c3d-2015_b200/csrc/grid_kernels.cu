@@ -796,62 +796,100 @@ __global__ void __launch_bounds__(256, 3)
 
 // ---------------------------------------------------------------- P_N moment flux
 
-// One CTA handles CPB interior cells; phase 1 forms the six 4-point differences per
-// cell, phase 2 applies the six half-range operators row by row in the order of
-// mvProduct (src/flux_moment.cpp:15-24, :57-101).
-__global__ void moment_flux_kernel(GridDims g, const double *__restrict__ u,
-                                   const double *__restrict__ ops, double dx, double dy, double dz,
-                                   int cellsPerBlock, double *__restrict__ flux)
+// flux(c) = sum over the axes of (A+ tp + A- tm) / h, tp and tm the upwind differences of the
+// moments for either sign of the cosine (src/flux_moment.cpp:57-101), for interior cells.
+// The six nm x nm operators sit in shared memory as DMMA B fragments for the CTA's lifetime; a
+// warp takes 8 MT interior cells at a time, its lanes form the A fragments of tp and tm
+// (cell lane / 4, moment 4 k + lane % 4) from five neighbours, and per axis a sum over k-steps
+// of both halves is divided by the spacing and added to the flux. Bound by the FP64 tensor
+// pipe: 12 nm^2 FMA per cell padded to tiles of 8 x 4. P_5 on 64^3: 344 us per call, 2387 us
+// with scalar unfused sums, one operator row per thread.
+template <int NT, int MT>
+__global__ void __launch_bounds__(256, NT <= 5 ? 2 : 1)
+    moment_flux_kernel(GridDims g, const double *__restrict__ u, const double *__restrict__ ops,
+                       double dx, double dy, double dz, double *__restrict__ flux)
 {
-    extern __shared__ double sh[];
-    const int nm = g.nm;
-    double *T = sh; // cellsPerBlock x 6 x nm
-    const long long nint = g.ninterior();
-    long long n0 = (long long)blockIdx.x * cellsPerBlock;
-    const long long sx = (long long)g.nyg() * g.nzg(), sy = g.nzg(), sz = 1;
-    for (int e = threadIdx.x; e < cellsPerBlock * nm; e += blockDim.x) {
-        int cl = e / nm, m = e % nm;
-        long long n = n0 + cl;
-        if (n >= nint)
-            continue;
-        long long c = interior_cell(g, n);
-        const long long st[3] = {sx, sy, sz};
-        for (int ax = 0; ax < 3; ++ax) {
-            long long s = st[ax];
-#define UU(o) u[(c + (o) * s) * nm + m]
-            double tp = __dadd_rn(__dsub_rn(__dadd_rn(__dmul_rn(0.25, UU(1)), __dmul_rn(0.75, UU(0))),
-                                            __dmul_rn(1.25, UU(-1))),
-                                  __dmul_rn(0.25, UU(-2)));
-            double tm = __dsub_rn(__dsub_rn(__dadd_rn(__dmul_rn(-0.25, UU(2)), __dmul_rn(1.25, UU(1))),
-                                            __dmul_rn(0.75, UU(0))),
-                                  __dmul_rn(0.25, UU(-1)));
-#undef UU
-            T[(cl * 6 + 2 * ax + 0) * nm + m] = tp;
-            T[(cl * 6 + 2 * ax + 1) * nm + m] = tm;
-        }
+    constexpr int KS = 2 * NT, FRAGS = KS * NT * 32;
+    extern __shared__ __align__(128) double sOps[]; // [operator][k-step][tile][lane]
+    const int nm = g.nm, ks = (nm + 3) / 4;
+    for (int e = threadIdx.x; e < 6 * FRAGS; e += 256) {
+        const int l = e & 31, t = (e >> 5) % NT, k = (e / (32 * NT)) % KS, op = e / FRAGS;
+        const int row = 8 * t + l / 4, col = 4 * k + l % 4;
+        sOps[e] = row < nm && col < nm ? ops[((size_t)op * nm + row) * nm + col] : 0.0;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < cellsPerBlock * nm; e += blockDim.x) {
-        int cl = e / nm, i = e % nm;
-        long long n = n0 + cl;
-        if (n >= nint)
-            continue;
-        long long c = interior_cell(g, n);
-        double axf[3];
-        for (int ax = 0; ax < 3; ++ax) {
-            const double *Ap = ops + (2 * ax + 0) * (long long)nm * nm + (long long)i * nm;
-            const double *Am = ops + (2 * ax + 1) * (long long)nm * nm + (long long)i * nm;
-            const double *tp = T + (cl * 6 + 2 * ax + 0) * nm;
-            const double *tm = T + (cl * 6 + 2 * ax + 1) * nm;
-            double b = 0.0;
-            for (int j = 0; j < nm; ++j)
-                b = __dadd_rn(b, __dmul_rn(__ldg(Ap + j), tp[j]));
-            for (int j = 0; j < nm; ++j)
-                b = __dadd_rn(b, __dmul_rn(__ldg(Am + j), tm[j]));
-            axf[ax] = b;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long nint = g.ninterior(), step = (long long)gridDim.x * 8 * 8 * MT;
+    const long long st[3] = {(long long)g.nyg() * g.nzg(), g.nzg(), 1};
+    for (long long n0 = ((long long)blockIdx.x * 8 + warp) * 8 * MT; n0 < nint; n0 += step) {
+        long long c[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const long long n = n0 + 8 * m + (lane >> 2);
+            c[m] = n < nint ? interior_cell(g, n) : -1;
         }
-        flux[c * nm + i] = __dadd_rn(__dadd_rn(__ddiv_rn(axf[0], dx), __ddiv_rn(axf[1], dy)),
-                                     __ddiv_rn(axf[2], dz));
+        double total[MT][NT][2];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            double acc[MT][NT][2];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+                    acc[m][t][0] = acc[m][t][1] = 0.0;
+            const double *bp = sOps + (2 * ax) * FRAGS + lane, *bm = bp + FRAGS;
+            const long long s = st[ax] * nm;
+#pragma unroll 2
+            for (int k = 0; k < ks; ++k) {
+                const int col = 4 * k + (lane & 3);
+                double tp[MT], tm[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    tp[m] = tm[m] = 0.0;
+                    if (c[m] >= 0 && col < nm) {
+                        const double *v = u + c[m] * nm + col;
+                        const double v0 = v[0], p1 = v[s], p2 = v[2 * s], m1 = v[-s], m2 = v[-2 * s];
+                        tp[m] = 0.25 * p1 + 0.75 * v0 - 1.25 * m1 + 0.25 * m2;
+                        tm[m] = -0.25 * p2 + 1.25 * p1 - 0.75 * v0 - 0.25 * m1;
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const double b = bp[(k * NT + t) * 32];
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+                        dmma_g(acc[m][t][0], acc[m][t][1], tp[m], b);
+                }
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const double b = bm[(k * NT + t) * 32];
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+                        dmma_g(acc[m][t][0], acc[m][t][1], tm[m], b);
+                }
+            }
+            const double h = ax == 0 ? dx : ax == 1 ? dy : dz;
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const double f = acc[m][t][e] / h;
+                        total[m][t][e] = ax == 0 ? f : total[m][t][e] + f;
+                    }
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+            if (c[m] >= 0)
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int row = 8 * t + 2 * (lane & 3) + e;
+                        if (row < nm)
+                            flux[c[m] * nm + row] = total[m][t][e];
+                    }
     }
 }
 
@@ -1214,16 +1252,45 @@ cudaError_t launch_kinetic_flux(const GridDims &g, const double *alpha, const do
 #undef C3D_NT_CASE
 }
 
-cudaError_t launch_moment_flux(const GridDims &g, const double *u, const double *ops, double dx,
-                               double dy, double dz, double *flux, cudaStream_t st)
+template <int NT, int MT>
+static cudaError_t moment_flux_t(const GridDims &g, const double *u, const double *ops, double dx,
+                                 double dy, double dz, double *flux, int numSMs, cudaStream_t st)
 {
-    int cpb = 256 / g.nm;
-    if (cpb < 1)
-        cpb = 1;
-    size_t sm = (size_t)cpb * 6 * g.nm * sizeof(double);
-    long long blocks = (g.ninterior() + cpb - 1) / cpb;
-    moment_flux_kernel<<<(int)blocks, 256, sm, st>>>(g, u, ops, dx, dy, dz, cpb, flux);
+    const int smem = 6 * 2 * NT * NT * 32 * 8;
+    cudaError_t e = cudaFuncSetAttribute(moment_flux_kernel<NT, MT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess)
+        return e;
+    const long long blocks = (g.ninterior() + 64 * MT - 1) / (64 * MT);
+    const long long cap = (long long)numSMs * (NT <= 5 ? 2 : 1);
+    moment_flux_kernel<NT, MT><<<(unsigned)(blocks < cap ? blocks : cap), 256, smem, st>>>(
+        g, u, ops, dx, dy, dz, flux);
     return cudaGetLastError();
+}
+
+// Two tiles of 8 cells per warp share each operator fragment's load; small grids take one so
+// that more SMs get cells.
+cudaError_t launch_moment_flux(const GridDims &g, const double *u, const double *ops, double dx,
+                               double dy, double dz, double *flux, int numSMs, cudaStream_t st)
+{
+    const bool wide = g.ninterior() >= 256LL * numSMs;
+#define C3D_NT_CASE(NT)                                                                            \
+    case NT:                                                                                       \
+        return wide ? moment_flux_t<NT, 2>(g, u, ops, dx, dy, dz, flux, numSMs, st)                \
+                    : moment_flux_t<NT, 1>(g, u, ops, dx, dy, dz, flux, numSMs, st);
+    switch ((g.nm + 7) / 8) {
+        C3D_NT_CASE(1)
+        C3D_NT_CASE(2)
+        C3D_NT_CASE(3)
+        C3D_NT_CASE(4)
+        C3D_NT_CASE(5)
+        C3D_NT_CASE(6)
+        C3D_NT_CASE(7)
+        C3D_NT_CASE(8)
+    default:
+        return cudaErrorInvalidValue;
+    }
+#undef C3D_NT_CASE
 }
 
 } // namespace c3d
