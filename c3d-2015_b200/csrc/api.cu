@@ -47,9 +47,8 @@ cudaError_t launch_gaunt_batch(int nm, int nm2, int nm2p, int nchunks, const dou
 cudaError_t launch_ghost_fill(const GridDims &g, double *u, int numSMs, cudaStream_t st,
                               bool skipX = false);
 cudaError_t launch_euler(const GridDims &g, double *u, const double *flux, const double *sigT,
-                         const double *sigS, double dt, int numSMs, cudaStream_t st);
-cudaError_t launch_rk(const GridDims &g, double *u, double *uOld, int mode, int numSMs,
-                      cudaStream_t st);
+                         const double *sigS, double dt, double *uOld, int mode, cudaStream_t st);
+cudaError_t launch_rk_save(const GridDims &g, const double *u, double *uOld, cudaStream_t st);
 cudaError_t launch_kinetic_flux(const GridDims &g, const double *alpha, const double *mfA,
                                 const double *mfP, const double *xi, const double *eta, int nq,
                                 int qChunk, int runLen, double theta, int isPn, double *psi,
@@ -71,14 +70,15 @@ cudaError_t launch_psi_groups(const GridDims &g, unsigned char *mark, long long 
 size_t flux_frag_doubles(int nm, int nq, int which);
 cudaError_t launch_reproject(const GridDims &g, double *u, double *alpha, const double *mfA,
                              const double *mfP, int nq, int *errorFlag, cudaStream_t st);
-cudaError_t launch_ghost_fill_int(const GridDims &g, int *a, int numSMs, cudaStream_t st);
-cudaError_t launch_ghost_fill_1(const GridDims &g, double *a, int numSMs, cudaStream_t st);
+cudaError_t launch_ghost_mirror_copy(const GridDims &g, double *u, double *alpha, int *iters,
+                                     int *iterGamma, int *regIdx, int *status, double *gamma,
+                                     double *normG, unsigned long long *stats, int numSMs,
+                                     cudaStream_t st);
+
 cudaError_t launch_line_log(const GridDims &g, const ClosureParams &P, const int *iters,
                             const int *iterGamma, const int *regIdx, const double *gamma,
                             const double *normG, double *out, cudaStream_t st);
-cudaError_t launch_ghost_stats(const GridDims &g, const int *iters, const int *iterGamma,
-                               const int *regIdx, const int *status, unsigned long long *stats,
-                               int numSMs, cudaStream_t st);
+
 cudaError_t launch_ghost_mirror_check(const GridDims &g, const double *a, int *flag, int numSMs,
                                       cudaStream_t st);
 void flux_frags(int nm, int nq, const double *M, const double *w, const double *xi,
@@ -908,15 +908,10 @@ static c3d_status closure_grid(c3d_ctx *c)
                                        c->regIdx, c->status, c->cellMap, true);
             if (s != C3D_OK)
                 return s;
-            C3D_CUDA(launch_ghost_fill(c->g, c->alpha, c->numSMs, c->stream));
-            C3D_CUDA(launch_ghost_fill(c->g, c->u, c->numSMs, c->stream));
-            for (int *a : {c->iters, c->iterGamma, c->regIdx, c->status})
-                C3D_CUDA(launch_ghost_fill_int(c->g, a, c->numSMs, c->stream));
-            for (double *a : {c->cellGamma, c->cellErr})
-                C3D_CUDA(launch_ghost_fill_1(c->g, a, c->numSMs, c->stream));
-            C3D_CUDA(launch_ghost_stats(c->g, c->iters, c->iterGamma, c->regIdx, c->status,
-                                        c->stats, c->numSMs, c->stream));
-            c->launches += 9;
+            C3D_CUDA(launch_ghost_mirror_copy(c->g, c->u, c->alpha, c->iters, c->iterGamma,
+                                              c->regIdx, c->status, c->cellGamma, c->cellErr,
+                                              c->stats, c->numSMs, c->stream));
+            c->launches += 1;
             c->mirroredClosures++;
             return finish_handoff(c, true);
         }
@@ -1610,16 +1605,22 @@ c3d_status c3d_flux_moment(c3d_ctx *c)
     return C3D_OK;
 }
 
+// The Euler stage; mode 1 saves u first, mode 2 ends with the RK average (euler_kernel).
+static c3d_status euler_stage(c3d_ctx *c, double dt, int mode)
+{
+    cudaEvent_t t0 = nullptr;
+    timing_begin(c, &t0);
+    C3D_CUDA(launch_euler(c->g, c->u, c->flux, c->sigT, c->sigS, dt, c->uOld, mode, c->stream));
+    timing_end(c, 3, t0);
+    c->launches += 1;
+    return C3D_OK;
+}
+
 c3d_status c3d_euler(c3d_ctx *c, double dt)
 {
     if (!c)
         return fail(C3D_ERR_INVALID, "c3d_euler: null context");
-    cudaEvent_t t0 = nullptr;
-    timing_begin(c, &t0);
-    C3D_CUDA(launch_euler(c->g, c->u, c->flux, c->sigT, c->sigS, dt, c->numSMs, c->stream));
-    timing_end(c, 3, t0);
-    c->launches += 1;
-    return C3D_OK;
+    return euler_stage(c, dt, 0);
 }
 
 // Sets an IF node's condition: mirrored closure when no face ghost's multipliers differ from
@@ -1724,7 +1725,7 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
     cudaStream_t s0 = cs[0];
     cudaError_t ec = cudaSuccess;
     if (stage == 0)
-        ec = launch_rk(c->g, c->u, c->uOld, 0, c->numSMs, s0);
+        ec = launch_rk_save(c->g, c->u, c->uOld, s0);
     if (ec == cudaSuccess)
         ec = launch_ghost_fill(c->g, c->u, c->numSMs, s0, c->xHaloExternal);
     n += (stage == 0) + 1;
@@ -1745,18 +1746,9 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
         cudaError_t er = launch_closure_rounds(R, c->gaunt);
         cudaStream_t sk = cs[k];
         if (er == cudaSuccess && mirrored) {
-            er = launch_ghost_fill(c->g, c->alpha, c->numSMs, sk);
-            if (er == cudaSuccess)
-                er = launch_ghost_fill(c->g, c->u, c->numSMs, sk);
-            for (int *a : {c->iters, c->iterGamma, c->regIdx, c->status})
-                if (er == cudaSuccess)
-                    er = launch_ghost_fill_int(c->g, a, c->numSMs, sk);
-            for (double *a : {c->cellGamma, c->cellErr})
-                if (er == cudaSuccess)
-                    er = launch_ghost_fill_1(c->g, a, c->numSMs, sk);
-            if (er == cudaSuccess)
-                er = launch_ghost_stats(c->g, c->iters, c->iterGamma, c->regIdx, c->status,
-                                        c->stats, c->numSMs, sk);
+            er = launch_ghost_mirror_copy(c->g, c->u, c->alpha, c->iters, c->iterGamma, c->regIdx,
+                                          c->status, c->cellGamma, c->cellErr, c->stats,
+                                          c->numSMs, sk);
         }
         if (er == cudaSuccess && R.psi)
             er = handoff_launch(c, mirrored && !wrap, sk);
@@ -1787,7 +1779,7 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
                     ec = eb;
             }
         }
-        n += 3 + 9;
+        n += 3 + 1;
     } else if (ec == cudaSuccess) {
         ec = closure(false, 0);
     }
@@ -1796,10 +1788,8 @@ static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff,
     if (ec == cudaSuccess)
         ec = flux_launch(c, c->alpha, 0, handoff, wrap ? c->mirrorFlag : nullptr, s0);
     if (ec == cudaSuccess)
-        ec = launch_euler(c->g, c->u, c->flux, c->sigT, c->sigS, dt, c->numSMs, s0);
-    if (ec == cudaSuccess && stage == 1)
-        ec = launch_rk(c->g, c->u, c->uOld, 1, c->numSMs, s0);
-    n += (handoff ? 1 + (wrap ? 1 : 2) : 2 * ceil_div(c->nq, c->qChunk)) + 1 + (stage == 1);
+        ec = launch_euler(c->g, c->u, c->flux, c->sigT, c->sigS, dt, c->uOld, stage == 1 ? 2 : 0, s0);
+    n += (handoff ? 2 + (wrap ? 1 : 2) : 2 * ceil_div(c->nq, c->qChunk)) + 1;
     *launches = n + (c->launches - l0); // the closure counted its round 0
     c->launches = l0;
     return ec;
@@ -1984,8 +1974,10 @@ c3d_status c3d_stage(c3d_ctx *c, int stage, double dt)
         return s;
     if (used)
         return C3D_OK;
-    if (stage == 0) {
-        C3D_CUDA(launch_rk(c->g, c->u, c->uOld, 0, c->numSMs, c->stream));
+    // the closure may change u between the save and the Euler stage; the P_N path does not
+    const bool saveInEuler = c->solver == 0 && stage == 0;
+    if (stage == 0 && !saveInEuler) {
+        C3D_CUDA(launch_rk_save(c->g, c->u, c->uOld, c->stream));
         c->launches += 1;
     }
     if ((s = c3d_ghost_fill(c)) != C3D_OK)
@@ -2002,13 +1994,7 @@ c3d_status c3d_stage(c3d_ctx *c, int stage, double dt)
         if ((s = c3d_flux_kinetic(c, 1)) != C3D_OK)
             return s;
     }
-    if ((s = c3d_euler(c, dt)) != C3D_OK)
-        return s;
-    if (stage == 1) {
-        C3D_CUDA(launch_rk(c->g, c->u, c->uOld, 1, c->numSMs, c->stream));
-        c->launches += 1;
-    }
-    return C3D_OK;
+    return euler_stage(c, dt, stage == 1 ? 2 : saveInEuler ? 1 : 0);
 }
 
 // The cells of the x-slab split: x is the slowest index of the I3D layout, so each x-plane is
@@ -2050,7 +2036,7 @@ c3d_status c3d_stage_part(c3d_ctx *c, int stage, double dt, int part)
         return s;
     if (part == 0) {
         if (stage == 0) {
-            C3D_CUDA(launch_rk(c->g, c->u, c->uOld, 0, c->numSMs, c->stream));
+            C3D_CUDA(launch_rk_save(c->g, c->u, c->uOld, c->stream));
             c->launches += 1;
         }
         if ((s = c3d_ghost_fill(c)) != C3D_OK) // the y and z faces
@@ -2084,13 +2070,7 @@ c3d_status c3d_stage_part(c3d_ctx *c, int stage, double dt, int part)
         return C3D_OK;
     if ((s = c3d_flux_kinetic(c, 0)) != C3D_OK)
         return s;
-    if ((s = c3d_euler(c, dt)) != C3D_OK)
-        return s;
-    if (stage == 1) {
-        C3D_CUDA(launch_rk(c->g, c->u, c->uOld, 1, c->numSMs, c->stream));
-        c->launches += 1;
-    }
-    return C3D_OK;
+    return euler_stage(c, dt, stage == 1 ? 2 : 0);
 }
 
 c3d_status c3d_step(c3d_ctx *c, double dt)

@@ -26,61 +26,86 @@ namespace c3d {
 
 // Two periodic ghost layers per face over interior ranges of the other two axes
 // (no edges or corners). The three face groups read only interior cells, so
-// they run as one launch. T: double state arrays (ncomp = nm) or int per-cell records.
-// f0 > 0 skips the first f0 faces: f0 = 4 ny nz leaves the x faces to the caller (x-slab
-// decomposition, whose x ghosts come from the neighbouring slabs).
-template <typename T>
-__global__ void ghost_fill_kernel(GridDims g, T *__restrict__ u, int ncomp, long long f0)
+// they run as one launch. f0 > 0 skips the first f0 faces: f0 = 4 ny nz leaves the x faces to
+// the caller (x-slab decomposition, whose x ghosts come from the neighbouring slabs). One warp
+// per ghost cell: the cell indices cost several 64-bit divisions.
+__global__ void ghost_fill_kernel(GridDims g, double *__restrict__ u, long long f0)
 {
-    const long long total = (ghost_faces(g) - f0) * ncomp;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        int m = (int)(e % ncomp);
+    const int lane = threadIdx.x & 31, nm = g.nm;
+    const long long total = ghost_faces(g), warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long f = f0 + (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); f < total;
+         f += warps) {
         long long dst, src;
-        ghost_pair(g, f0 + e / ncomp, dst, src);
-        u[dst * ncomp + m] = u[src * ncomp + m];
+        ghost_pair(g, f, dst, src);
+        for (int m = lane; m < nm; m += 32)
+            u[dst * nm + m] = u[src * nm + m];
     }
 }
 
-// Closure statistics of the face ghosts whose records a mirrored closure copied from their
-// images: the same counters a solve adds (finalize, closure_core.cuh), so that the totals
-// equal those of solving every cell.
-__global__ void ghost_stats_kernel(GridDims g, const int *__restrict__ iters,
-                                   const int *__restrict__ iterGamma,
-                                   const int *__restrict__ regIdx, const int *__restrict__ status,
-                                   unsigned long long *stats)
+// What a mirrored closure copies from the periodic images to the face ghosts.
+struct MirrorCopy {
+    double *u, *alpha;
+    int *iters, *iterGamma, *regIdx, *status;
+    double *gamma, *normG;
+    unsigned long long *stats;
+};
+
+// The face ghosts of a mirrored closure, one warp per ghost cell: multipliers, moments and
+// records of the image, and the closure statistics a solve of the ghost would have added
+// (finalize, closure_core.cuh), so that the totals equal those of solving every cell. The CTA's
+// counters are 32-bit in shared memory (native atomics) and go to the context's once per CTA.
+__global__ void ghost_mirror_copy_kernel(GridDims g, MirrorCopy C)
 {
-    // the CTA's counters in shared memory, added to the context's once per CTA
-    __shared__ unsigned long long sStat[STAT_COUNT];
+    __shared__ unsigned int sStat[STAT_COUNT];
+    __shared__ unsigned long long sIters, sIterGamma;
     for (int q = threadIdx.x; q < STAT_COUNT; q += blockDim.x)
         sStat[q] = 0;
+    if (threadIdx.x == 0)
+        sIters = sIterGamma = 0;
     __syncthreads();
-    const long long total = ghost_faces(g);
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < total;
-         f += (long long)gridDim.x * blockDim.x) {
+    unsigned long long iters = 0, iterGamma = 0;
+    const int lane = threadIdx.x & 31, nm = g.nm;
+    const long long total = ghost_faces(g), warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long f = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < total; f += warps) {
         long long dst, src;
         ghost_pair(g, f, dst, src);
-        const unsigned long long it = (unsigned long long)iters[dst];
-        const unsigned long long ig = (unsigned long long)iterGamma[dst];
-        atomicAdd(&sStat[STAT_CELLS], 1ull);
-        atomicAdd(&sStat[STAT_ITERS], it);
-        atomicAdd(&sStat[STAT_ITER_GAMMA], ig);
-        atomicMax(&sStat[STAT_MAX_ITER], it);
-        atomicMax(&sStat[STAT_MAX_ITER_GAMMA], ig);
-        if (status[dst] != CELL_OK)
-            atomicAdd(&sStat[STAT_FAILED], 1ull);
-        atomicAdd(&sStat[STAT_REG_HIST + (regIdx[dst] & 15)], 1ull);
-        atomicAdd(&sStat[STAT_ITER_HIST + (it < 63 ? it : 63)], 1ull);
+        for (int m = lane; m < nm; m += 32) {
+            C.alpha[dst * nm + m] = C.alpha[src * nm + m];
+            C.u[dst * nm + m] = C.u[src * nm + m];
+        }
+        if (lane == 0) {
+            const int it = C.iters[src], ig = C.iterGamma[src], rg = C.regIdx[src], st = C.status[src];
+            C.iters[dst] = it;
+            C.iterGamma[dst] = ig;
+            C.regIdx[dst] = rg;
+            C.status[dst] = st;
+            C.gamma[dst] = C.gamma[src];
+            C.normG[dst] = C.normG[src];
+            atomicAdd(&sStat[STAT_CELLS], 1u);
+            iters += (unsigned long long)it;
+            iterGamma += (unsigned long long)ig;
+            atomicMax(&sStat[STAT_MAX_ITER], (unsigned int)it);
+            atomicMax(&sStat[STAT_MAX_ITER_GAMMA], (unsigned int)ig);
+            if (st != CELL_OK)
+                atomicAdd(&sStat[STAT_FAILED], 1u);
+            atomicAdd(&sStat[STAT_REG_HIST + (rg & 15)], 1u);
+            atomicAdd(&sStat[STAT_ITER_HIST + (it < 63 ? it : 63)], 1u);
+        }
+    }
+    if (iters) {
+        atomicAdd(&sIters, iters);
+        atomicAdd(&sIterGamma, iterGamma);
     }
     __syncthreads();
     for (int q = threadIdx.x; q < STAT_COUNT; q += blockDim.x) {
-        const unsigned long long v = sStat[q];
+        const unsigned long long v =
+            q == STAT_ITERS ? sIters : q == STAT_ITER_GAMMA ? sIterGamma : sStat[q];
         if (v == 0)
             continue;
         if (q == STAT_MAX_ITER || q == STAT_MAX_ITER_GAMMA)
-            atomicMax(&stats[q], v);
+            atomicMax(&C.stats[q], v);
         else
-            atomicAdd(&stats[q], v);
+            atomicAdd(&C.stats[q], v);
     }
 }
 
@@ -105,18 +130,17 @@ __global__ void line_log_kernel(GridDims g, ClosureParams P, const int *__restri
 }
 
 // *flag = 1 if any face ghost of a differs (bitwise) from its periodic image.
-__global__ void ghost_mirror_check_kernel(GridDims g, const double *__restrict__ a, int ncomp,
-                                          int *flag)
+__global__ void ghost_mirror_check_kernel(GridDims g, const double *__restrict__ a, int *flag)
 {
-    const long long total = ghost_faces(g) * ncomp;
+    const int lane = threadIdx.x & 31, nm = g.nm;
+    const long long total = ghost_faces(g), warps = ((long long)gridDim.x * blockDim.x) >> 5;
     const unsigned long long *b = reinterpret_cast<const unsigned long long *>(a);
     bool diff = false;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        int m = (int)(e % ncomp);
+    for (long long f = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < total; f += warps) {
         long long dst, src;
-        ghost_pair(g, e / ncomp, dst, src);
-        diff |= b[dst * ncomp + m] != b[src * ncomp + m];
+        ghost_pair(g, f, dst, src);
+        for (int m = lane; m < nm; m += 32)
+            diff |= b[dst * nm + m] != b[src * nm + m];
     }
     if (__syncthreads_or(diff) && threadIdx.x == 0)
         atomicExch(flag, 1);
@@ -224,52 +248,46 @@ __global__ void psi_refresh_kernel(GridDims g, int nq, const double *__restrict_
 
 // ---------------------------------------------------------------- Euler / RK
 
-__device__ __forceinline__ bool interior(const GridDims &g, long long c, int &i, int &j, int &k)
+// The interior cells of a z line are nz nm consecutive doubles, so the elementwise stages walk
+// lines (blockIdx.y strided) with 32-bit indices inside one.
+// Calls f(x, c, m) for every element x of moment m of interior cell c.
+template <class F> __device__ __forceinline__ void for_interior(const GridDims &g, F &&f)
 {
-    k = (int)(c % g.nzg());
-    long long r = c / g.nzg();
-    j = (int)(r % g.nyg());
-    i = (int)(r / g.nyg());
-    return i >= 2 && i < g.nx + 2 && j >= 2 && j < g.ny + 2 && k >= 2 && k < g.nz + 2;
+    const int nm = g.nm, len = g.nz * nm, lines = g.nx * g.ny;
+    for (int l = blockIdx.y; l < lines; l += gridDim.y) {
+        const long long c0 = g.cell(2 + l / g.ny, 2 + l % g.ny, 2);
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < len; t += gridDim.x * blockDim.x)
+            f(c0 * nm + t, c0 + t / nm, t % nm);
+    }
 }
 
-
+// Euler stage. MODE 0: u <- E(u); 1: uOld <- u, then u <- E(u) (the save of the first RK stage,
+// where nothing changes u in between); 2: u <- 0.5 (E(u) + uOld) (the last RK stage). E rounds
+// as the reference's expressions, unfused.
+template <int MODE>
 __global__ void euler_kernel(GridDims g, double *__restrict__ u, const double *__restrict__ flux,
                              const double *__restrict__ sigT, const double *__restrict__ sigS,
-                             double dt)
+                             double dt, double *__restrict__ uOld)
 {
-    const int nm = g.nm;
-    const long long total = g.ninterior() * nm;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        int m = (int)(e % nm);
-        long long c = interior_cell(g, e / nm);
-        long long x = c * nm + m;
-        double st = sigT[c];
+    for_interior(g, [&](long long x, long long c, int m) {
+        const double st = sigT[c], u0 = u[x];
         double v;
         if (m == 0) {
             double fac = __dsub_rn(__dadd_rn(1.0, __dmul_rn(dt, sigS[c])), __dmul_rn(dt, st));
-            v = __dsub_rn(__dmul_rn(u[x], fac), __dmul_rn(dt, flux[x]));
+            v = __dsub_rn(__dmul_rn(u0, fac), __dmul_rn(dt, flux[x]));
         } else {
-            v = __dsub_rn(__dmul_rn(u[x], __dsub_rn(1.0, __dmul_rn(dt, st))), __dmul_rn(dt, flux[x]));
+            v = __dsub_rn(__dmul_rn(u0, __dsub_rn(1.0, __dmul_rn(dt, st))), __dmul_rn(dt, flux[x]));
         }
-        u[x] = v;
-    }
+        if (MODE == 1)
+            uOld[x] = u0;
+        u[x] = MODE == 2 ? __dmul_rn(0.5, __dadd_rn(v, uOld[x])) : v;
+    });
 }
 
-// mode 0: uOld <- u ; mode 1: u <- 0.5 (u + uOld)   (interior cells only)
-__global__ void rk_kernel(GridDims g, double *__restrict__ u, double *__restrict__ uOld, int mode)
+// uOld <- u (interior cells only)
+__global__ void rk_save_kernel(GridDims g, const double *__restrict__ u, double *__restrict__ uOld)
 {
-    const int nm = g.nm;
-    const long long total = g.ninterior() * nm;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        long long x = interior_cell(g, e / nm) * nm + (e % nm);
-        if (mode == 0)
-            uOld[x] = u[x];
-        else
-            u[x] = __dmul_rn(0.5, __dadd_rn(u[x], uOld[x]));
-    }
+    for_interior(g, [&](long long x, long long, int) { uOld[x] = u[x]; });
 }
 
 // ---------------------------------------------------------------- kinetic flux on the tensor pipe
@@ -908,20 +926,7 @@ cudaError_t launch_ghost_fill(const GridDims &g, double *u, int numSMs, cudaStre
                               bool skipX)
 {
     const long long f0 = skipX ? 4LL * g.ny * g.nz : 0;
-    ghost_fill_kernel<double><<<grid_for((ghost_faces(g) - f0) * g.nm, 256, numSMs), 256, 0, st>>>(
-        g, u, g.nm, f0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_ghost_fill_int(const GridDims &g, int *a, int numSMs, cudaStream_t st)
-{
-    ghost_fill_kernel<int><<<grid_for(ghost_faces(g), 256, numSMs), 256, 0, st>>>(g, a, 1, 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_ghost_fill_1(const GridDims &g, double *a, int numSMs, cudaStream_t st)
-{
-    ghost_fill_kernel<double><<<grid_for(ghost_faces(g), 256, numSMs), 256, 0, st>>>(g, a, 1, 0);
+    ghost_fill_kernel<<<grid_for((ghost_faces(g) - f0) * 32, 256, numSMs), 256, 0, st>>>(g, u, f0);
     return cudaGetLastError();
 }
 
@@ -934,20 +939,20 @@ cudaError_t launch_line_log(const GridDims &g, const ClosureParams &P, const int
     return cudaGetLastError();
 }
 
-cudaError_t launch_ghost_stats(const GridDims &g, const int *iters, const int *iterGamma,
-                               const int *regIdx, const int *status, unsigned long long *stats,
-                               int numSMs, cudaStream_t st)
+cudaError_t launch_ghost_mirror_copy(const GridDims &g, double *u, double *alpha, int *iters,
+                                     int *iterGamma, int *regIdx, int *status, double *gamma,
+                                     double *normG, unsigned long long *stats, int numSMs,
+                                     cudaStream_t st)
 {
-    ghost_stats_kernel<<<grid_for(ghost_faces(g), 256, numSMs), 256, 0, st>>>(
-        g, iters, iterGamma, regIdx, status, stats);
+    ghost_mirror_copy_kernel<<<grid_for(ghost_faces(g) * 32, 256, numSMs), 256, 0, st>>>(
+        g, MirrorCopy{u, alpha, iters, iterGamma, regIdx, status, gamma, normG, stats});
     return cudaGetLastError();
 }
 
 cudaError_t launch_ghost_mirror_check(const GridDims &g, const double *a, int *flag, int numSMs,
                                       cudaStream_t st)
 {
-    ghost_mirror_check_kernel<<<grid_for(ghost_faces(g) * g.nm, 256, numSMs), 256, 0, st>>>(
-        g, a, g.nm, flag);
+    ghost_mirror_check_kernel<<<grid_for(ghost_faces(g) * 32, 256, numSMs), 256, 0, st>>>(g, a, flag);
     return cudaGetLastError();
 }
 
@@ -980,18 +985,29 @@ cudaError_t launch_psi_face_copy(const GridDims &g, int nq, double *psi, cudaStr
     return cudaGetLastError();
 }
 
-cudaError_t launch_euler(const GridDims &g, double *u, const double *flux, const double *sigT,
-                         const double *sigS, double dt, int numSMs, cudaStream_t st)
+static dim3 interior_grid(const GridDims &g)
 {
-    euler_kernel<<<grid_for(g.ninterior() * g.nm, 256, numSMs), 256, 0, st>>>(g, u, flux, sigT, sigS,
-                                                                              dt);
+    const long long lines = (long long)g.nx * g.ny;
+    return dim3((unsigned)(((long long)g.nz * g.nm + 255) / 256), (unsigned)(lines < 65535 ? lines : 65535));
+}
+
+// mode as euler_kernel's (uOld may be null in mode 0)
+cudaError_t launch_euler(const GridDims &g, double *u, const double *flux, const double *sigT,
+                         const double *sigS, double dt, double *uOld, int mode, cudaStream_t st)
+{
+    const dim3 grid = interior_grid(g);
+    if (mode == 0)
+        euler_kernel<0><<<grid, 256, 0, st>>>(g, u, flux, sigT, sigS, dt, uOld);
+    else if (mode == 1)
+        euler_kernel<1><<<grid, 256, 0, st>>>(g, u, flux, sigT, sigS, dt, uOld);
+    else
+        euler_kernel<2><<<grid, 256, 0, st>>>(g, u, flux, sigT, sigS, dt, uOld);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rk(const GridDims &g, double *u, double *uOld, int mode, int numSMs,
-                      cudaStream_t st)
+cudaError_t launch_rk_save(const GridDims &g, const double *u, double *uOld, cudaStream_t st)
 {
-    rk_kernel<<<grid_for(g.ninterior() * g.nm, 256, numSMs), 256, 0, st>>>(g, u, uOld, mode);
+    rk_save_kernel<<<interior_grid(g), 256, 0, st>>>(g, u, uOld);
     return cudaGetLastError();
 }
 
