@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -1125,39 +1126,37 @@ c3d_status c3d_set_gaunt(c3d_ctx *c, int nm2, const double *M2, const int *rowPt
     cudaMemcpy(dchc, chc.data(), chc.size() * 8, cudaMemcpyHostToDevice);
     if (c->gChunksC) cudaFree(c->gChunksC);
     c->gChunksC = dchc;
-    // assembly streams of the tiled Hessian (work-list engine). Thread t of the Newton
-    // kernel's CTA owns the tile slots e = t + 128 i of the lower triangle of 8x8 tiles; its
-    // stream lists, slot after slot, the CSR terms of beta for that slot's (row >= col)
-    // element in the reference's order, the last one marked with the slot (a slot without
-    // terms gets one zero term; identity padding slots one col = -1 entry). Streams are
-    // padded to a common length with no-op entries and interleaved across threads
-    // (entry s of thread t at s * 128 + t) so that a warp's loads coalesce.
-    const int nt = (nm + 7) / 8, ls = 64 * nt * (nt + 1) / 2;
+    // assembly streams of the tiled Hessian (work-list engine): the elements of the lower
+    // triangle are dealt to the threads of the Newton kernel's CTA, longest first to the thread
+    // with the fewest terms; a stream lists, element after element, its CSR terms of beta in
+    // the reference's order, the last one marked with the element's tile slot (an element
+    // without terms gets one zero term). Streams are padded to a common length with no-op
+    // entries and interleaved across threads (entry s of thread t at s * 128 + t) so that a
+    // warp's loads coalesce. The kernel fills the identity padding itself.
+    std::vector<std::pair<int, int>> elems; // (terms, i * nm + j)
+    for (int i = 0; i < nm; ++i)
+        for (int j = 0; j <= i; ++j)
+            elems.push_back({std::max(1, rowPtr[j * nm + i + 1] - rowPtr[j * nm + i]), i * nm + j});
+    std::stable_sort(elems.begin(), elems.end(),
+                     [](const auto &a, const auto &b) { return a.first > b.first; });
     std::vector<std::vector<GauntTerm>> lists(NEWTON_THREADS);
-    for (int e = 0; e < ls; ++e) {
-        std::vector<GauntTerm> &st = lists[e % NEWTON_THREADS];
-        // storage offset e & 63 inside tile e >> 6 -> element (rr, cc), the inverse of toff
-        const int t = e >> 6, rr = (e >> 3) & 7;
-        const int cc = 2 * (((e >> 1) & 3) ^ ((rr >> 1) & 3)) + (e & 1);
-        int ib = 0;
-        while ((ib + 1) * (ib + 2) / 2 <= t)
-            ++ib;
-        const int jb = t - ib * (ib + 1) / 2;
-        const int i = 8 * ib + rr, j = 8 * jb + cc;
-        const size_t first = st.size();
-        if (!(ib == jb && cc > rr)) {
-            if (i >= nm || j >= nm) {
-                if (i == j)
-                    st.push_back(GauntTerm{1.0, -1, -1});
-            } else {
-                const int idx = j * nm + i;
-                for (int k = rowPtr[idx]; k < rowPtr[idx + 1]; ++k)
-                    st.push_back(GauntTerm{val[k], colInd[k], -1});
-            }
-        }
-        if (st.size() == first)
+    std::vector<std::pair<size_t, int>> load; // min-heap of (terms, thread)
+    for (int t = 0; t < NEWTON_THREADS; ++t)
+        load.push_back({0, t});
+    for (const auto &el : elems) {
+        std::pop_heap(load.begin(), load.end(), std::greater<>());
+        std::vector<GauntTerm> &st = lists[load.back().second];
+        const int i = el.second / nm, j = el.second % nm, idx = j * nm + i;
+        for (int k = rowPtr[idx]; k < rowPtr[idx + 1]; ++k)
+            st.push_back(GauntTerm{val[k], colInd[k], -1});
+        if (rowPtr[idx + 1] == rowPtr[idx])
             st.push_back(GauntTerm{0.0, 0, -1});
-        st.back().slot = e;
+        // tile (i / 8, j / 8), element offset as toff (closure_core.cuh)
+        const int ib = i / 8, jb = j / 8, r = i % 8, c2 = j % 8;
+        st.back().slot = 64 * (ib * (ib + 1) / 2 + jb) + 8 * r +
+                         2 * ((c2 >> 1) ^ ((r >> 1) & 3)) + (c2 & 1);
+        load.back().first = st.size();
+        std::push_heap(load.begin(), load.end(), std::greater<>());
     }
     size_t len = 0;
     for (auto &st : lists)

@@ -84,8 +84,8 @@ struct ClosureParams {
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // One entry of the Gaunt-form Hessian assembly stream (src/opt/fobj.cpp:81-99): the
-// running H element += v * moment[col] (col = -1: the element is 1, an identity padding
-// slot); slot >= 0 ends tile slot `slot`, which then receives the element.
+// running H element += v * moment[col]; slot >= 0 ends tile slot `slot`, which then receives
+// the element.
 struct __align__(16) GauntTerm {
     double v;
     int col;

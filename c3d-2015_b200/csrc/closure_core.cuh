@@ -246,12 +246,14 @@ __device__ int warp_cholesky_packed(S &sl, int n, int lane)
 }
 
 // Blocked Cholesky of the tiled lower triangle (Slot<NT, true>); returns LAPACK info.
-// Per tile column kb: the 8 columns of the panel (diagonal tile and the tiles below it,
-// in registers, lane l holding elements 2l, 2l+1 of each) are factored right-looking with
-// warp shuffles; the trailing tiles (ib, jb), kb < jb <= ib, then receive
-// -L(ib,kb) L(jb,kb)^T as two m8n8k4 DMMAs each (the panel tiles in operand layout:
-// lane l holds L[l/4][4s + l%4] for k-step s, which is the A fragment of L(ib,kb) and the
-// B fragment of L(jb,kb)^T).
+// Per tile column kb: lane l holds row l % 8 of the diagonal tile (the four octets repeat each
+// other) and the 8 columns are factored with shuffles inside the tile; then each lane solves
+// rows of the panel below against that tile, one row of 8 elements at a time, and the trailing
+// tiles (ib, jb), kb < jb <= ib, receive -L(ib,kb) L(jb,kb)^T as two m8n8k4 DMMAs each (lane l
+// holds L[l/4][4s + l%4] for k-step s, which is the A fragment of L(ib,kb) and the B fragment
+// of L(jb,kb)^T). Every element sees the operations of the column-by-column form in its order.
+// The chain of pivots (square root and reciprocal) bounds it; the loop over tile columns stays
+// rolled so that the code fits the instruction cache.
 template <class S>
 __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
 {
@@ -259,81 +261,94 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
     static_assert(sizeof(S) % 16 == 0 && (8 * 8 * S::NMP) % 16 == 0,
                   "tiles must be 16-byte aligned in every slot");
     double *A = sl.L;
-    const int r = lane >> 2, q = lane & 3;
-    const int c0 = 2 * q, c1 = 2 * q + 1;
     int info = 0;
-#pragma unroll
+#pragma unroll 1
     for (int kb = 0; kb < T; ++kb) {
-        double p0[T], p1[T];
+        double *D = A + 64 * tix(kb, kb);
+        const int row = lane & 7;
+        double v[8], rj[8];
 #pragma unroll
-        for (int t = kb; t < T; ++t) {
-            double2 v = *reinterpret_cast<const double2 *>(&A[64 * tix(t, kb) + tpair(lane)]);
-            p0[t] = v.x;
-            p1[t] = v.y;
+        for (int q = 0; q < 4; ++q) {
+            const double2 x = *reinterpret_cast<const double2 *>(&D[toff(row, 2 * q)]);
+            v[2 * q] = x.x;
+            v[2 * q + 1] = x.y;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            // padding columns (identity rows, zero couplings) would leave their entries
-            // unchanged: skip them (warp-uniform)
-            if (8 * kb + j >= n)
-                break;
-            const int src = 4 * j + (j >> 1);
-            double ajj = __shfl_sync(FULL_MASK, (j & 1) ? p1[kb] : p0[kb], src);
-            // warp-uniform; padding pivots are 1. The loops run to the end (and then hold
-            // NaNs) so that they unroll completely and the panel stays in registers.
-            if (!(ajj > 0.0) && info == 0)
-                info = 8 * kb + j + 1;
-            double ljj = sqrt(ajj);
-            double rj = 1.0 / ljj;
-            // column j: the pivot, then the rows below it scaled by 1/L_jj
-            if (q == (j >> 1)) {
-                double &dv = (j & 1) ? p1[kb] : p0[kb];
-                if (r == j)
-                    dv = ljj;
-                else if (r > j)
-                    dv *= rj;
+            rj[j] = 1.0;
+            // padding columns (identity rows, zero couplings, last tile only) stay as they are
+            if (8 * kb + j < n) {
+                const double ajj = __shfl_sync(FULL_MASK, v[j], j);
+                if (!(ajj > 0.0) && info == 0)
+                    info = 8 * kb + j + 1;
+                // root and reciprocal both from the pivot, so that neither waits for the other
+                const double ljj = sqrt(ajj);
+                rj[j] = rsqrt(ajj);
+                if (row == j)
+                    v[j] = ljj;
+                else if (row > j)
+                    v[j] *= rj[j];
 #pragma unroll
-                for (int t = kb + 1; t < T; ++t) {
-                    double &v = (j & 1) ? p1[t] : p0[t];
-                    v *= rj;
+                for (int c = j + 1; c < 8; ++c) {
+                    const double lc = __shfl_sync(FULL_MASK, v[j], c);
+                    if (row >= c)
+                        v[c] = fma(-v[j], lc, v[c]);
                 }
             }
-            // L(c, j) of the diagonal tile for this lane's columns c0, c1
-            double lc0 = __shfl_sync(FULL_MASK, (j & 1) ? p1[kb] : p0[kb], 4 * c0 + (j >> 1));
-            double lc1 = __shfl_sync(FULL_MASK, (j & 1) ? p1[kb] : p0[kb], 4 * c1 + (j >> 1));
+        }
+        __syncwarp();
+        if (lane < 8) {
 #pragma unroll
-            for (int t = kb; t < T; ++t) {
-                double lrj = __shfl_sync(FULL_MASK, (j & 1) ? p1[t] : p0[t], 4 * r + (j >> 1));
-                bool ok0 = c0 > j && (t > kb || c0 <= r);
-                bool ok1 = c1 > j && (t > kb || c1 <= r);
-                if (ok0)
-                    p0[t] = fma(-lrj, lc0, p0[t]);
-                if (ok1)
-                    p1[t] = fma(-lrj, lc1, p1[t]);
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<double2 *>(&D[toff(row, 2 * q)]) =
+                    make_double2(v[2 * q], v[2 * q + 1]);
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<double2 *>(&sl.rinv[8 * kb + 2 * q]) =
+                    make_double2(rj[2 * q], rj[2 * q + 1]);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int i = lane; i < 8 * (T - 1 - kb); i += 32) {
+            double *P = A + 64 * tix(kb + 1 + (i >> 3), kb);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double2 x = *reinterpret_cast<const double2 *>(&P[toff(i & 7, 2 * q)]);
+                v[2 * q] = x.x;
+                v[2 * q + 1] = x.y;
             }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] *= rj[j];
+#pragma unroll
+                for (int c = j + 1; c < 8; ++c)
+                    v[c] = fma(-v[j], D[toff(c, j)], v[c]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<double2 *>(&P[toff(i & 7, 2 * q)]) =
+                    make_double2(v[2 * q], v[2 * q + 1]);
         }
-        double f0[T], f1[T];
-#pragma unroll
-        for (int t = kb; t < T; ++t) {
-            *reinterpret_cast<double2 *>(&A[64 * tix(t, kb) + tpair(lane)]) =
-                make_double2(p0[t], p1[t]);
-            double x0 = __shfl_sync(FULL_MASK, p0[t], 4 * r + (q >> 1));
-            double x1 = __shfl_sync(FULL_MASK, p1[t], 4 * r + (q >> 1));
-            double y0 = __shfl_sync(FULL_MASK, p0[t], 4 * r + 2 + (q >> 1));
-            double y1 = __shfl_sync(FULL_MASK, p1[t], 4 * r + 2 + (q >> 1));
-            f0[t] = (q & 1) ? x1 : x0;
-            f1[t] = (q & 1) ? y1 : y0;
-        }
-#pragma unroll
-        for (int jb = kb + 1; jb < T; ++jb)
-#pragma unroll
+        __syncwarp();
+        const int f0 = toff(lane >> 2, lane & 3), f1 = toff(lane >> 2, 4 + (lane & 3));
+#pragma unroll 1
+        for (int jb = kb + 1; jb < T; ++jb) {
+            const double *Bt = A + 64 * tix(jb, kb);
+            const double b0 = Bt[f0], b1 = Bt[f1];
+            // (four tiles at a time with loads first took 126 registers instead of 96 and was
+            // 4% slower on the standalone orders, whose warps per SM it lowers)
+#pragma unroll 2
             for (int ib = jb; ib < T; ++ib) {
+                const double *At = A + 64 * tix(ib, kb);
                 double2 *cp = reinterpret_cast<double2 *>(&A[64 * tix(ib, jb) + tpair(lane)]);
                 double2 c = *cp;
-                dmma(c.x, c.y, -f0[ib], f0[jb]);
-                dmma(c.x, c.y, -f1[ib], f1[jb]);
+                dmma(c.x, c.y, -At[f0], b0);
+                dmma(c.x, c.y, -At[f1], b1);
                 *cp = c;
             }
+        }
         __syncwarp();
     }
     return info;
@@ -354,18 +369,18 @@ __device__ __forceinline__ int warp_cholesky(S &sl, int n, int lane)
 // precomputed reciprocal.
 template <class S>
 __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, double &x0,
-                                                         double &x1, double r0, double r1);
+                                                         double &x1);
 
 template <class S>
 __device__ void warp_apply_inverse(const S &sl, int n, int lane, double &x0, double &x1,
-                                   bool exactDiv, double r0 = 0.0, double r1 = 0.0)
+                                   bool exactDiv)
 {
     if constexpr (S::tiled) {
         // the reciprocals serve both the estimate and the direction here: the blocked
         // factor already rounds differently from the reference's unblocked one
         (void)n;
         (void)exactDiv;
-        warp_apply_inverse_tiled(sl, lane, x0, x1, r0, r1);
+        warp_apply_inverse_tiled(sl, lane, x0, x1);
         return;
     }
     const double *P = sl.L;
@@ -401,92 +416,103 @@ __device__ void warp_apply_inverse(const S &sl, int n, int lane, double &x0, dou
     }
 }
 
-// x <- (L L^T)^{-1} x on the tiled factor: tile-blocked substitution. Inside the diagonal
-// tile the steps are those of the column-oriented form with the reciprocal pivots r0, r1
-// of this lane's rows (lane, lane + 32), held in registers: the row's owner scales it and
-// broadcasts the result;
-// the tiles off the diagonal act as 8-column mat-vec updates of the rows below (forward) or
-// above (backward). Padding rows (L = I there, reciprocal 1) keep finite values and never feed
-// the real rows.
+// x <- (L L^T)^{-1} x on the tiled factor: tile-blocked substitution. Every lane solves the
+// diagonal tile's 8 rows (gathered by shuffles) in its own registers with the reciprocal
+// pivots sl.rinv, in the order of the column-oriented form; the tiles off the diagonal act as
+// 8-column mat-vec updates of the rows below (forward) or above (backward). Padding rows (L = I
+// there, reciprocal 1) keep finite values and never feed the real rows. (One shuffle per row
+// instead: 18.3k clocks per solve at n = 64.)
 template <class S>
 __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, double &x0,
-                                                         double &x1, double r0, double r1)
+                                                         double &x1)
 {
     constexpr int T = S::nt;
     constexpr int NMP = S::NMP;
     const double *A = sl.L;
+    const int own = lane & 7;
+    // the block's values and reciprocals; the lane's own row takes its value back
+    auto gather = [&](int kb, double (&y)[8], double (&r)[8]) {
+        const double v = kb < 4 ? x0 : x1;
 #pragma unroll
+        for (int i = 0; i < 8; ++i)
+            y[i] = __shfl_sync(FULL_MASK, v, (8 * kb + i) & 31);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double2 t = *reinterpret_cast<const double2 *>(&sl.rinv[8 * kb + 2 * q]);
+            r[2 * q] = t.x;
+            r[2 * q + 1] = t.y;
+        }
+    };
+    auto scatter = [&](int kb, const double (&y)[8]) {
+        double v = y[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i)
+            v = own == i ? y[i] : v;
+        if ((lane >> 3) == (kb & 3)) {
+            if (kb < 4)
+                x0 = v;
+            else
+                x1 = v;
+        }
+    };
+#pragma unroll 1
     for (int kb = 0; kb < T; ++kb) {
         const double *D = A + 64 * tix(kb, kb);
+        double y[8], r[8];
+        gather(kb, y, r);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int row = 8 * kb + i;
-            const double xi = __shfl_sync(FULL_MASK, row < 32 ? x0 * r0 : x1 * r1, row & 31);
-            if (lane == (row & 31)) {
-                if (row < 32)
-                    x0 = xi;
-                else
-                    x1 = xi;
-            }
-            if (lane > row && lane < 8 * kb + 8)
-                x0 = fma(-D[toff(lane - 8 * kb, i)], xi, x0);
-            if (lane + 32 > row && lane + 32 < 8 * kb + 8)
-                x1 = fma(-D[toff(lane + 32 - 8 * kb, i)], xi, x1);
-        }
-        if (kb + 1 < T) {
-            double y[8];
+            y[i] *= r[i];
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-                y[c] = __shfl_sync(FULL_MASK, 8 * kb + c < 32 ? x0 : x1, (8 * kb + c) & 31);
+            for (int k = i + 1; k < 8; ++k)
+                y[k] = fma(-D[toff(k, i)], y[i], y[k]);
+        }
+        scatter(kb, y);
+        if (kb + 1 < T) {
             if (lane >= 8 * kb + 8 && lane < NMP) {
                 const double *Lt = A + 64 * tix(lane >> 3, kb);
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    x0 = fma(-Lt[toff(lane & 7, c)], y[c], x0);
+                for (int q = 0; q < 4; ++q) {
+                    const double2 l = *reinterpret_cast<const double2 *>(&Lt[toff(own, 2 * q)]);
+                    x0 = fma(-l.x, y[2 * q], x0);
+                    x0 = fma(-l.y, y[2 * q + 1], x0);
+                }
             }
-            if (lane + 32 >= 8 * kb + 8 && lane + 32 < NMP) {
+            if (NMP > 32 && lane + 32 >= 8 * kb + 8 && lane + 32 < NMP) {
                 const double *Lt = A + 64 * tix((lane + 32) >> 3, kb);
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    x1 = fma(-Lt[toff(lane & 7, c)], y[c], x1);
+                for (int q = 0; q < 4; ++q) {
+                    const double2 l = *reinterpret_cast<const double2 *>(&Lt[toff(own, 2 * q)]);
+                    x1 = fma(-l.x, y[2 * q], x1);
+                    x1 = fma(-l.y, y[2 * q + 1], x1);
+                }
             }
         }
     }
-#pragma unroll
+#pragma unroll 1
     for (int kb = T - 1; kb >= 0; --kb) {
         const double *D = A + 64 * tix(kb, kb);
+        double y[8], r[8];
+        gather(kb, y, r);
 #pragma unroll
         for (int i = 7; i >= 0; --i) {
-            const int row = 8 * kb + i;
-            const double xi = __shfl_sync(FULL_MASK, row < 32 ? x0 * r0 : x1 * r1, row & 31);
-            if (lane == (row & 31)) {
-                if (row < 32)
-                    x0 = xi;
-                else
-                    x1 = xi;
-            }
-            if (lane >= 8 * kb && lane < row)
-                x0 = fma(-D[toff(i, lane - 8 * kb)], xi, x0);
-            if (lane + 32 >= 8 * kb && lane + 32 < row)
-                x1 = fma(-D[toff(i, lane + 32 - 8 * kb)], xi, x1);
+            y[i] *= r[i];
+#pragma unroll
+            for (int k = 0; k < i; ++k)
+                y[k] = fma(-D[toff(i, k)], y[i], y[k]);
         }
-        if (kb > 0) {
-            double y[8];
+        scatter(kb, y);
+        if (lane < 8 * kb) {
+            const double *Lt = A + 64 * tix(kb, lane >> 3);
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-                y[c] = __shfl_sync(FULL_MASK, 8 * kb + c < 32 ? x0 : x1, (8 * kb + c) & 31);
-            if (lane < 8 * kb) {
-                const double *Lt = A + 64 * tix(kb, lane >> 3);
+                x0 = fma(-Lt[toff(c, own)], y[c], x0);
+        }
+        if (NMP > 32 && lane + 32 < 8 * kb) {
+            const double *Lt = A + 64 * tix(kb, (lane + 32) >> 3);
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    x0 = fma(-Lt[toff(c, lane & 7)], y[c], x0);
-            }
-            if (lane + 32 < 8 * kb) {
-                const double *Lt = A + 64 * tix(kb, (lane + 32) >> 3);
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    x1 = fma(-Lt[toff(c, lane & 7)], y[c], x1);
-            }
+            for (int c = 0; c < 8; ++c)
+                x1 = fma(-Lt[toff(c, own)], y[c], x1);
         }
     }
 }
@@ -501,13 +527,12 @@ __device__ __forceinline__ double vsum_abs(double x0, double x1, int lane, int n
 // 381-396, Alg. 4.1 -- the algorithm of LAPACK's dlacn2 as driven by dpocon).
 // Returns 1/rcond with rcond = (1/est)/anorm.
 template <class S>
-__device__ double warp_condest(const S &sl, int n, int lane, double anorm, double r0 = 0.0,
-                               double r1 = 0.0)
+__device__ double warp_condest(const S &sl, int n, int lane, double anorm)
 {
     if (anorm == 0.0)
         return 1.0 / 0.0;
     double x0 = 1.0 / (double)n, x1 = 1.0 / (double)n;
-    warp_apply_inverse(sl, n, lane, x0, x1, false, r0, r1);
+    warp_apply_inverse(sl, n, lane, x0, x1, false);
     double est;
     if (n == 1) {
         est = fabs(__shfl_sync(FULL_MASK, x0, 0));
@@ -516,13 +541,13 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm, doubl
         int s0 = x0 >= 0.0 ? 1 : -1, s1 = x1 >= 0.0 ? 1 : -1;
         x0 = (double)s0;
         x1 = (double)s1;
-        warp_apply_inverse(sl, n, lane, x0, x1, false, r0, r1);
+        warp_apply_inverse(sl, n, lane, x0, x1, false);
         int j = warp_iamax(x0, x1, lane, n);
         int iter = 2;
         for (;;) {
             x0 = (lane == j) ? 1.0 : 0.0;
             x1 = (lane + 32 == j) ? 1.0 : 0.0;
-            warp_apply_inverse(sl, n, lane, x0, x1, false, r0, r1);
+            warp_apply_inverse(sl, n, lane, x0, x1, false);
             double estold = est;
             est = vsum_abs(x0, x1, lane, n);
             bool diff = (lane < n && (x0 >= 0.0 ? 1 : -1) != s0) ||
@@ -534,7 +559,7 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm, doubl
             s1 = x1 >= 0.0 ? 1 : -1;
             x0 = (double)s0;
             x1 = (double)s1;
-            warp_apply_inverse(sl, n, lane, x0, x1, false, r0, r1);
+            warp_apply_inverse(sl, n, lane, x0, x1, false);
             int jlast = j;
             j = warp_iamax(x0, x1, lane, n);
             double xjl = __shfl_sync(FULL_MASK, jlast < 32 ? x0 : x1, jlast & 31);
@@ -547,7 +572,7 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm, doubl
         }
         x0 = ((lane & 1) ? -1.0 : 1.0) * (1.0 + (double)lane / (double)(n - 1));
         x1 = (((lane + 32) & 1) ? -1.0 : 1.0) * (1.0 + (double)(lane + 32) / (double)(n - 1));
-        warp_apply_inverse(sl, n, lane, x0, x1, false, r0, r1);
+        warp_apply_inverse(sl, n, lane, x0, x1, false);
         double temp = 2.0 * (vsum_abs(x0, x1, lane, n) / (double)(3 * n));
         if (temp > est)
             est = temp;
@@ -814,9 +839,11 @@ __device__ void escalate_fp64(S &sl, const Outputs &O, int lane)
 
 // gext (mixed precision): the FP64 moments <m_i e^{alpha.m}> and fqext = <e^{alpha.m}> of
 // the pass, from which g and f are formed instead of from row 0 of the reduced-precision H.
+// emin: a lower bound of e^{alpha.m} over the quadrature (0: none).
 template <class S>
 __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, int lane,
-                              double m0, const double *gext = nullptr, double fqext = 0.0)
+                              double m0, const double *gext = nullptr, double fqext = 0.0,
+                              double emin = 0.0)
 {
     const int nm = P.nm;
     C3D_NCLK_DECL
@@ -875,28 +902,28 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     // 1-norm condition number is at most norm1 sqrt(n)/gmin. The Hager estimate can only be
     // smaller, so if this bound is below condHMax/2 the reference's test `condest > condHMax`
     // is false whatever the estimate; the estimate is then skipped.
+    // H >= e_min G bounds the smallest eigenvalue too (after_probe), halved for rounding, which
+    // must be far below it. The mixed closure routes by the record, so there only the Gershgorin
+    // bound replaces the estimate.
+    const double lam = 0.5 * emin * P.gramLo;
+    if (!P.mixed && lam > 1e-12 * norm1)
+        gmin = fmax(gmin, lam);
     bool condSure = gmin > 0.0 && norm1 * sqrt((double)nm) / gmin <= 0.5 * P.condHMax;
-    if (lane == 0) // the condition record: the Gershgorin bound, or the estimate below
+    if (lane == 0) // the condition record: the bound, or the estimate below
         sl.s.cnd = condSure ? norm1 * sqrt((double)nm) / gmin : 0.0;
     __syncwarp();
     C3D_NCLK(O.stats, 1, lane);
     int info = warp_cholesky(sl, nm, lane);
     C3D_NCLK(O.stats, 2, lane);
     double cond = 0.0;
-    double r0 = 1.0, r1 = 1.0; // tiled: reciprocal pivots of rows lane, lane + 32
     if (info == 0) {
-        if constexpr (S::tiled) {
-            if (lane < S::NMP)
-                r0 = 1.0 / sl.L[S::lx(lane, lane)];
-            if (lane + 32 < S::NMP)
-                r1 = 1.0 / sl.L[S::lx(lane + 32, lane + 32)];
-        } else {
+        // reciprocal pivots (the tiled factorisation leaves them in rinv)
+        if constexpr (!S::tiled)
             for (int i = lane; i < nm; i += 32)
                 sl.rinv[i] = 1.0 / sl.L[S::lx(i, i)];
-        }
         __syncwarp();
         if (!condSure)
-            cond = warp_condest(sl, nm, lane, norm1, r0, r1);
+            cond = warp_condest(sl, nm, lane, norm1);
     }
     __syncwarp();
     C3D_NCLK(O.stats, 3, lane);
@@ -943,7 +970,7 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     // d = -H^{-1} g
     double x0 = lane < nm ? sl.g[lane] : 0.0;
     double x1 = lane + 32 < nm ? sl.g[lane + 32] : 0.0;
-    warp_apply_inverse(sl, nm, lane, x0, x1, true, r0, r1);
+    warp_apply_inverse(sl, nm, lane, x0, x1, true);
     if (lane < nm)
         sl.d[lane] = -x0;
     if (lane + 32 < nm)

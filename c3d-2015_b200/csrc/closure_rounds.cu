@@ -39,6 +39,14 @@ template <int NT> struct CellState {
 
 namespace {
 
+__device__ __forceinline__ void copy_scalars(SlotScalars &dst, const SlotScalars &src, int lane)
+{
+    static_assert(sizeof(SlotScalars) % 8 == 0 && sizeof(SlotScalars) <= 256, "one word per lane");
+    if (lane < (int)sizeof(SlotScalars) / 8)
+        reinterpret_cast<unsigned long long *>(&dst)[lane] =
+            reinterpret_cast<const unsigned long long *>(&src)[lane];
+}
+
 // lineSearch = false skips d and alphaOld, which a Hessian visit recomputes before use.
 template <int NT, class S>
 __device__ void state_to_slot(const CellState<NT> &st, S &sl, int lane, bool lineSearch = true)
@@ -54,8 +62,7 @@ __device__ void state_to_slot(const CellState<NT> &st, S &sl, int lane, bool lin
             sl.alphaOld[i] = st.alphaOld[i];
         }
     }
-    if (lane == 0)
-        sl.s = st.s;
+    copy_scalars(sl.s, st.s, lane);
     __syncwarp();
 }
 
@@ -72,8 +79,7 @@ __device__ void slot_to_state(const S &sl, CellState<NT> &st, int lane)
         st.d[i] = sl.d[i];
         st.alphaOld[i] = sl.alphaOld[i];
     }
-    if (lane == 0)
-        st.s = sl.s;
+    copy_scalars(st.s, sl.s, lane);
 }
 
 // The work lists of one round: 0 trials and FP64 Hessian passes, 1 BF16 Hessian passes,
@@ -960,7 +966,8 @@ __device__ __forceinline__ bool trial_fused(const ClosureParams &P, int fp64, in
 }
 
 // Hessian and trial pass over the listed cells (the FP64 list): the nm2 extended moments of
-// cells that need them into momBuf (stride 8 NT2) and f's sum of trial cells into their state.
+// cells that need them into momBuf (stride 8 NT2), followed by a lower bound of e^{alpha.m} (the
+// smallest high word), and f's sum of trial cells into their state.
 template <int NT, int NT2>
 __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
     sym_pass_kernel(ClosureParams P, SymTables T, const int *__restrict__ list, int n,
@@ -1006,6 +1013,7 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
     for (int t = 0; t < E::TILES; ++t)
         acc[t][0] = acc[t][1] = 0.0;
     double f = 0.0;
+    int lo = 0x7fffffff;
     __syncthreads();
     for (int b = 0; b < T.nb; ++b) {
         const double *st = stage + (b % SYM_STAGES) * G::DOUBLES;
@@ -1017,8 +1025,12 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    v[e][s] = (e == 0 ? w.x : w.y) * exp(v[e][s]);
+                for (int s = 0; s < 8; ++s) {
+                    const double ez = exp(v[e][s]);
+                    // (directions past the last have exponent 0: they only lower the bound)
+                    lo = min(lo, __double2hiint(ez));
+                    v[e][s] = (e == 0 ? w.x : w.y) * ez;
+                }
                 sym_wht(v[e]);
                 f += v[e][0];
                 if (anyH)
@@ -1033,8 +1045,13 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
         if (tid == 0 && b + SYM_STAGES < T.nb)
             sym_stage_load<DEG, PD>(T, b + SYM_STAGES, stage, full);
     }
+    lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, 1));
+    lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, 2));
     if (wantH) {
         double *o = momBuf + (size_t)pos * (8 * NT2);
+        static_assert((PD + 1) * (PD + 1) < 8 * NT2, "room for the bound");
+        if ((lane & 3) == 0)
+            o[(PD + 1) * (PD + 1)] = __hiloint2double(lo, 0);
 #pragma unroll
         for (int t = 0; t < E::TILES; ++t)
 #pragma unroll
@@ -1189,7 +1206,7 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
 // GAUNT: the CTA assembles H_ij = sum_k beta_ijk mom_k (i >= j, the CSR terms of beta in
 // the order of src/opt/fobj.cpp:81-99, laid out per tile slot by c3d_set_gaunt) for its
 // cells that need a Hessian in one sweep over the tile slots, so that each term is read once
-// for RWN cells. A cell's moments sit in its slot's g..rinv vectors, which a Hessian visit
+// for RWN cells. The cells' moments sit in the slots' g..rinv vectors, which a Hessian visit
 // recomputes afterwards. Otherwise the pass wrote H in tiles to hBuf.
 template <int NT, int NT2, bool GAUNT, int MODE>
 __global__ void __launch_bounds__(RWN * 32)
@@ -1250,32 +1267,50 @@ __global__ void __launch_bounds__(RWN * 32)
         sl.s.need = NEED_NONE;
     }
     bool nonFinite = false;
-    // fused trials: the pass also formed the moments at the trial point, so an accepted trial
-    // goes on to the next iteration's Hessian visit here (unless that iteration regularised,
-    // which moves the multipliers)
+    // Trials come first. Fused: the pass also formed the moments at the trial point, so an
+    // accepted trial goes on to the next iteration's Hessian visit here (unless that iteration
+    // regularised, which moves the multipliers).
     bool tried = false;
     if constexpr (MODE == 0 && GAUNT) {
-        if (fused && active && !needH && sl.s.need == NEED_TRIAL) {
+        if (active && !needH && sl.s.need == NEED_TRIAL) {
             tried = true;
-            const bool moments = trial_fused(P, sl.s.fp64, sl.s.iter, sl.s.cnd);
+            const bool moments = fused && trial_fused(P, sl.s.fp64, sl.s.iter, sl.s.cnd);
             const int reg = sl.s.regIndex;
             after_trial(sl, P, O, lane, sl.s.fquad);
             needH = moments && sl.s.need == NEED_H && sl.s.regIndex == reg;
+            if (!needH) {
+                // on to another pass (or finished): stored before the assembly takes the scratch
+                if (sl.s.need != NEED_NONE)
+                    slot_to_state(sl, state[cell], lane);
+                append_if_needed(sl, P, cell, lane, out);
+            }
         }
     }
     if constexpr (MODE == 2) {
     } else if (GAUNT) {
-        double *mom = sl.scratch(); // g, d, alphaOld, rinv: NM2P <= 4 NMP doubles
-        if (needH) {
+        if (__syncthreads_or(needH)) {
+            // The CTA's moments, cells innermost, so that a term's loads for all cells are two
+            // 16-byte accesses: moment k of cell w at offset 4 (k / 4) + w of slot k % 4's scratch
+            // (g, d, alphaOld, rinv: NM2P <= 4 NMP doubles). Slots whose cell needs no Hessian
+            // hold nothing in theirs any more.
+            static_assert(RWN == 4, "moment layout");
             bool nf = false;
             for (int k = lane; k < NM2P; k += 32) {
-                const double v = buf[(size_t)pos * BSTR + k];
+                const double v = needH ? buf[(size_t)pos * BSTR + k] : 0.0;
                 nf |= MIX && !isfinite(v);
-                mom[k] = v;
+                slots[k & 3].scratch()[(k & ~3) + warp] = v;
             }
             nonFinite = __any_sync(FULL_MASK, nf);
-        }
-        if (__syncthreads_or(needH)) {
+            // identity padding: the last tile row's rows past nm
+            if (needH) {
+                constexpr int T = NT;
+                for (int t = 0; t < T; ++t)
+                    *reinterpret_cast<double2 *>(&sl.L[64 * tix(T - 1, t) + 2 * lane]) =
+                        make_double2(0.0, 0.0);
+                __syncwarp();
+                if (lane < 8 && 8 * (T - 1) + lane >= P.nm)
+                    sl.L[64 * tix(T - 1, T - 1) + toff(lane, lane)] = 1.0;
+            }
             __shared__ int sNeedH[RWN];
             if (lane == 0)
                 sNeedH[warp] = needH;
@@ -1289,18 +1324,16 @@ __global__ void __launch_bounds__(RWN * 32)
 #pragma unroll
             for (int w = 0; w < RWN; ++w)
                 h[w] = 0.0;
-#pragma unroll 4
+#pragma unroll 8
             for (int k = 0; k < streamLen; ++k) {
                 const GauntTerm gt = stream[k * NEWTON_THREADS + tid];
-                if (gt.col >= 0) {
-#pragma unroll
-                    for (int w = 0; w < RWN; ++w)
-                        h[w] = __dadd_rn(h[w], __dmul_rn(slots[w].scratch()[gt.col], gt.v));
-                } else {
-#pragma unroll
-                    for (int w = 0; w < RWN; ++w)
-                        h[w] = 1.0;
-                }
+                const double *m = slots[gt.col & 3].scratch() + (gt.col & ~3);
+                const double2 m01 = *reinterpret_cast<const double2 *>(m);
+                const double2 m23 = *reinterpret_cast<const double2 *>(m + 2);
+                h[0] = __dadd_rn(h[0], __dmul_rn(m01.x, gt.v));
+                h[1] = __dadd_rn(h[1], __dmul_rn(m01.y, gt.v));
+                h[2] = __dadd_rn(h[2], __dmul_rn(m23.x, gt.v));
+                h[3] = __dadd_rn(h[3], __dmul_rn(m23.y, gt.v));
                 if (gt.slot >= 0) {
 #pragma unroll
                     for (int w = 0; w < RWN; ++w) {
@@ -1319,7 +1352,7 @@ __global__ void __launch_bounds__(RWN * 32)
             L[e] = H[e];
         __syncwarp();
     }
-    if (active) {
+    if (active && !(tried && !needH)) {
     C3D_NCLK(O.stats, 0, lane);
     if constexpr (MODE == 2) {
         if (sl.s.need == NEED_PROBE) {
@@ -1347,10 +1380,14 @@ __global__ void __launch_bounds__(RWN * 32)
                 after_hessian(sl, P, O, lane, m0, e, e[NMP]);
             }
         } else {
-            after_hessian(sl, P, O, lane, m0);
+            double emin = 0.0;
+            if constexpr (GAUNT)
+                if (fused) // the symmetric pass left its bound behind the moments
+                    emin = buf[(size_t)pos * BSTR + (2 * sym_order(NT2) + 1) * (2 * sym_order(NT2) + 1)];
+            after_hessian(sl, P, O, lane, m0, nullptr, 0.0, emin);
         }
         C3D_NCLK(O.stats, 5, lane);
-    } else if (!tried && sl.s.need == NEED_TRIAL) {
+    } else if (sl.s.need == NEED_TRIAL) {
         after_trial(sl, P, O, lane, sl.s.fquad);
         C3D_NCLK(O.stats, 7, lane);
     }
