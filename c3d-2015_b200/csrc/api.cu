@@ -61,8 +61,8 @@ cudaError_t launch_sym_ansatz(const SymTables &T, int deg, long long nall, const
                               double *psi, int numSMs, cudaStream_t st);
 cudaError_t launch_sym_flux(const GridDims &g, int deg, const double *psi, const double *tab,
                             const int *idx, int r0, int r1, double theta, double *flux,
-                            const int *wrapFlag, int numSMs, cudaStream_t st);
-cudaError_t launch_psi_face_copy(const GridDims &g, int nq, double *psi, cudaStream_t st);
+                            int *errorFlag, const int *wrapFlag, int numSMs, cudaStream_t st);
+cudaError_t launch_psi_face_copy(const GridDims &g, int rows, int comp, double *psi, cudaStream_t st);
 cudaError_t launch_psi_refresh(const GridDims &g, int nq, const double *M, const double *alpha,
                                const long long *list, const unsigned int *count, double *psi,
                                int numSMs, cudaStream_t st);
@@ -225,6 +225,7 @@ struct c3d_ctx {
     int deg = 0;
     SymTables symPsi{}, symN{}, sym2{};
     double *symFlux = nullptr;
+    int psi_rows() const { return symPsi.no > 0 ? sym_rows(nq) : nq; } // rows of psi in full
     double *symBuf[3] = {nullptr, nullptr, nullptr}; // allocations of symPsi, symN, sym2
     double *gChunksC = nullptr;    // work-list engine: chunks of nm2 M2 rows + the weight row
     GauntTerm *gStream = nullptr;  // tiled assembly streams of the work-list engine
@@ -337,6 +338,9 @@ static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **b
     if (flux)
         *flux = *buf + f;
 }
+
+// Rows of psi a direction chunk takes.
+static int psi_chunk_rows(const c3d_ctx *c) { return c->qChunk >= c->nq ? c->psi_rows() : c->qChunk; }
 
 // psi no longer matches the multipliers (or may not): the next hand-off closure writes all of it.
 static void psi_invalidate(c3d_ctx *c)
@@ -479,7 +483,7 @@ c3d_status c3d_create(const c3d_params *p, const double *M, const double *w, con
     // direction chunk of the materialised ansatz: shared-memory and HBM budgets
     // (whole tiles of 32 unless one chunk covers every direction)
     long long byBudget = (long long)(c->psiBytes / ((size_t)nall * 8));
-    int qc = byBudget >= nq ? nq : (int)(byBudget / 32) * 32;
+    int qc = byBudget >= c->psi_rows() ? nq : (int)(byBudget / 32) * 32;
     if (qc < 32)
         qc = nq < 32 ? nq : 32;
     c->qChunk = qc;
@@ -680,7 +684,7 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
             (c->symN.no > 0) == (c->symPsi.no > 0)) {
             // hand the probe's ansatz to the kinetic flux when psi of every direction fits the
             // budget
-            const size_t need = (size_t)c->nq * c->g.nall() * 8;
+            const size_t need = (size_t)c->psi_rows() * c->g.nall() * 8;
             if (need <= c->psiBytes) {
                 if (!c->psiRefresh) {
                     const size_t groups = (size_t)(c->g.nall() + 7) / 8;
@@ -816,7 +820,8 @@ static cudaError_t handoff_launch(c3d_ctx *c, bool faceCopy, cudaStream_t st)
     if (e == cudaSuccess && c->psiValid)
         e = cudaMemsetAsync(c->psiValid, 1, sizeof(int), st);
     if (e == cudaSuccess && faceCopy)
-        e = launch_psi_face_copy(c->g, c->nq, c->psi, st);
+        e = c->symPsi.no > 0 ? launch_psi_face_copy(c->g, c->psi_rows() / 4, 4, c->psi, st)
+                             : launch_psi_face_copy(c->g, c->nq, 1, c->psi, st);
     return e;
 }
 
@@ -838,7 +843,7 @@ static cudaError_t flux_launch(c3d_ctx *c, const double *a, int isPn, bool ready
                                   c->psi, c->numSMs, st);
         if (e == cudaSuccess)
             e = launch_sym_flux(c->g, c->deg, c->psi, c->symFlux, c->symPsi.idx, r0, r1, c->theta,
-                                c->flux, wrapFlag, c->numSMs, st);
+                                c->flux, c->errorFlag, wrapFlag, c->numSMs, st);
     }
     return e;
 }
@@ -1493,7 +1498,7 @@ c3d_status c3d_flux_kinetic(c3d_ctx *c, int alphaIsU)
 {
     if (!c)
         return fail(C3D_ERR_INVALID, "c3d_flux_kinetic: null context");
-    const size_t need = (size_t)c->qChunk * c->g.nall() * 8;
+    const size_t need = (size_t)psi_chunk_rows(c) * c->g.nall() * 8;
     if (!c->psi || c->psiAlloc < need) {
         if (c->psi)
             cudaFree(c->psi);
@@ -1505,7 +1510,7 @@ c3d_status c3d_flux_kinetic(c3d_ctx *c, int alphaIsU)
     const double *a = alphaIsU ? c->u : c->alpha;
     int isPn = (c->solver == 0) ? 1 : 0;
     const bool ready = c->psiReady && !alphaIsU && isPn == 0 &&
-                       c->psiAlloc >= (size_t)c->nq * c->g.nall() * 8;
+                       c->psiAlloc >= (size_t)c->psi_rows() * c->g.nall() * 8;
     c->psiReady = false;
     if (!ready)
         psi_invalidate(c); // the ansatz kernel writes psi
@@ -1530,7 +1535,7 @@ c3d_status c3d_autotune(c3d_ctx *c, int *qChunk, int *runLen, double *msPerCall)
     const int nq = c->nq;
     const long long nall = c->g.nall();
     long long byBudget = (long long)(c->psiBytes / ((size_t)nall * 8));
-    int qmax = byBudget >= nq ? nq : (int)(byBudget / 32) * 32;
+    int qmax = byBudget >= c->psi_rows() ? nq : (int)(byBudget / 32) * 32;
     if (qmax < 32)
         qmax = nq < 32 ? nq : 32;
     std::vector<int> qs{qmax};
@@ -1659,7 +1664,7 @@ static c3d_status stage_prepare(c3d_ctx *c, bool *handoff)
     }
     *handoff = Rall.psi != nullptr;
     if (!*handoff) {
-        const size_t need = (size_t)c->qChunk * c->g.nall() * 8;
+        const size_t need = (size_t)psi_chunk_rows(c) * c->g.nall() * 8;
         if (!c->psi || c->psiAlloc < need) {
             if (c->psi)
                 cudaFree(c->psi);

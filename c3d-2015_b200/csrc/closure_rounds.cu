@@ -1136,19 +1136,19 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
             sym_expand<DEG>(aF, st, lane, v);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int o = SYM_BLK * b + 2 * (lane & 3) + e;
-                double *p = first.psi + (long long)(8 * o) * first.nall + gc;
+                double *p = first.psi + ((long long)(8 * (2 * b + e)) * first.nall + gc) * 4 + (lane & 3);
+                const bool w = write && 4 * (2 * b + e) < T.no; // a whole group past the end: no rows
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
                     v[e][s] = exp(v[e][s]);
-                    if (write && o < T.no)
-                        p[(long long)s * first.nall] = u0 * v[e][s];
+                    if (w)
+                        p[(long long)(4 * s) * first.nall] = u0 * v[e][s];
                 }
             }
             const double2 w = *reinterpret_cast<const double2 *>(T.w + SYM_BLK * b + 2 * (lane & 3));
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                if (SYM_BLK * b + 2 * (lane & 3) + e < T.no)
+                if (SYM_BLK * b + 4 * e + (lane & 3) < T.no)
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
                         lo = min(lo, __double2hiint(v[e][s]));

@@ -14,8 +14,11 @@
 // takes 9 n-tiles of 8 class members over nq / 8 directions instead of 7 n-tiles over nq, 6.2
 // times fewer DMMAs; the 169 extended moments of the Gaunt form 24 instead of 22 * 8.
 //
-// Directions come in blocks of 8 octant directions (BLK). psi rows of a symmetric context are in
-// octant order, row 8 o + s.
+// Directions come in blocks of 8 octant directions, position n of block b holding direction
+// 8 b + 4 (n % 2) + n / 2, so that the two columns a lane owns in a DMMA result belong to the
+// two groups of 4 consecutive directions of the block. psi of a symmetric context is
+// [group of 4 directions][reflection][cell][4 directions]: a warp's 8 cells x 4 directions are
+// 256 consecutive bytes, and a cell's 4 directions one sector, whatever the alignment of its row.
 #pragma once
 #include "c3d_common.cuh"
 
@@ -63,6 +66,9 @@ template <int DEG> struct SymCls {
 };
 
 constexpr int SYM_BLK = 8; // octant directions per block
+__host__ __device__ constexpr int sym_at(int b, int n) { return 8 * b + 4 * (n & 1) + (n >> 1); }
+// psi rows (directions, padded to whole groups) for nq directions
+__host__ __device__ constexpr int sym_rows(int nq) { return (nq + 31) / 32 * 32; }
 
 // Octant direction o (mu, xi, eta > 0) in the order of the tensor quadrature with Q nodes.
 __host__ __device__ inline int sym_direction(int Q, int o)
@@ -72,12 +78,12 @@ __host__ __device__ inline int sym_direction(int Q, int o)
 
 // Device tables of a symmetric quadrature (built by sym_build, owned by the context).
 //   expo  [block][step][lane]        B fragment of Z = A M^T: member 4 step + lane % 4 of its
-//                                    class at octant direction 8 block + lane / 4
-//   proj  [block][half][tile][lane]  B fragment of F += V M: direction 8 block + 2 (lane % 4) +
-//                                    half, member 8 tile + lane / 4 of its class
+//                                    class at position lane / 4 of the block
+//   proj  [block][half][tile][lane]  B fragment of F += V M: direction 8 block + 4 half +
+//                                    lane % 4, member 8 tile + lane / 4 of its class
 //   flux  [group of 4 directions][tile][lane], then |xi| w / dx, |eta| w / dy, |mu| w / dz and
 //                                    4 zeros of the group's directions (the kinetic flux)
-//   w     [block][8]                 weights of the octant directions (0 past the last)
+//   w     [block][position]          weights of the octant directions (0 past the last)
 //   idx   [tile][8]                  column of each class member, -1 padding
 // Degree: expo, flux and projN/idxN the basis', proj2/idx2 twice that (Gaunt form).
 struct SymTables {
@@ -134,7 +140,7 @@ __device__ __forceinline__ void sym_wht(double (&v)[8])
 }
 
 // Exponents of a block for the warp's 8 cells: lane l gets z[e][s] of cell l / 4 and octant
-// direction 2 (l % 4) + e of the block. aF: the cells' multipliers as A fragments
+// direction 4 e + l % 4 of the block. aF: the cells' multipliers as A fragments
 // [step][lane]; bE: the block's expansion fragments.
 template <int DEG>
 __device__ __forceinline__ void sym_expand(const double *aF, const double *bE, int lane,

@@ -1,7 +1,5 @@
 // The kinetic flux over an octant-symmetric quadrature (sym.cuh): the ansatz of the grid cells
-// and the limited upwind stencil with its projection (src/flux_kinetic.cpp:20-198). Both forms
-// of psi's producer (this file's ansatz kernel and the closure's probe) and its consumer use
-// octant order, row 8 o + s.
+// and the limited upwind stencil with its projection (src/flux_kinetic.cpp:20-198).
 #include "sym.cuh"
 
 namespace c3d {
@@ -13,26 +11,46 @@ __device__ __forceinline__ uint32_t saddr(const void *p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Asynchronous global -> shared copy of BYTES (8 or 16).
-template <int BYTES> __device__ __forceinline__ void copy_async(uint32_t dst, const double *src)
+__device__ __forceinline__ void bar_init(uint64_t *b, int count)
 {
-    if constexpr (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(saddr(b)), "r"(count));
 }
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait()
+__device__ __forceinline__ void bar_arrive(uint64_t *b)
 {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(saddr(b)) : "memory");
+}
+// false if the phase did not complete within the iteration limit
+__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t parity)
+{
+    for (int it = 0; it < (1 << 26); ++it) {
+        uint32_t done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done)
+                     : "r"(saddr(b)), "r"(parity)
+                     : "memory");
+        if (done)
+            return true;
+    }
+    return false;
+}
+// 16 bytes global -> shared, asynchronous
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+// arrives on b once the thread's copies so far have landed (the arrival is in b's count)
+__device__ __forceinline__ void copy_arrive(uint64_t *b)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(saddr(b)) : "memory");
 }
 
 } // namespace
 
 // ---------------------------------------------------------------- ansatz
 
-// psi[(row - r0) nall + c] = exp(alpha_c . m_row) (M_N) or alpha_c . m_row (P_N) for the rows
-// r0 <= row < r1 and either all cells (list null) or the marked cells of the *count groups of 8
+// psi (rows r0 <= row < r1, whole groups of 32 from r0 on; layout sym.cuh) = exp(alpha_c . m)
+// (M_N) or alpha_c . m (P_N) for either all cells (list null) or the marked cells of the *count groups of 8
 // consecutive cells in list (psi_groups_kernel), those whose multipliers a closure changed after
 // its probe had written their psi. A warp holds 8 cells'
 // multipliers as A fragments in shared memory and forms 64 exponents of each per block
@@ -72,12 +90,12 @@ __global__ void __launch_bounds__(128)
             sym_expand<DEG>(aF, T.expo + (size_t)b * C::STEPS * 32, lane, z);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int row = 8 * (SYM_BLK * b + 2 * (lane & 3) + e);
+                const int row = 32 * (2 * b + e); // first row of the group
                 if (c >= 0 && row >= r0 && row < r1) {
-                    double *p = psi + (long long)(row - r0) * nall + c;
+                    double *p = psi + ((long long)((row - r0) / 4) * nall + c) * 4 + (lane & 3);
 #pragma unroll
                     for (int s = 0; s < 8; ++s)
-                        p[(long long)s * nall] = isPn ? z[e][s] : exp(z[e][s]);
+                        p[(long long)(4 * s) * nall] = isPn ? z[e][s] : exp(z[e][s]);
                 }
             }
         }
@@ -120,46 +138,45 @@ __device__ __forceinline__ double sym_axis(double th2, double v2, double v1, dou
 }
 
 // Tile of a CTA: TX x 4 lines of 8 cells along z, one warp per line, staged with its halo per
-// direction as [TX + 3][7][12] doubles: x planes and y rows in upwind order (mirrored for the
-// reflections that flip the axis), z ascending from k0 - 2. The direction stride is 4 or 12
-// mod 16 doubles, so the 4 directions x 4 cells that half a warp reads at once fall into
-// distinct banks.
+// reflection and group of 4 octant directions as [TX + 3][7][12][4] doubles: x planes and y rows
+// in upwind order (mirrored for the reflections that flip the axis), z ascending from k0 - 2,
+// directions innermost (a warp reads 8 cells x 4 directions as 256 consecutive bytes).
 template <int TX> struct FluxTile {
-    static constexpr int TY = 4, TZ = 8, RY = TY + 3, RZ = TZ + 4, PX = RY * RZ;
-    static constexpr int DIR = (TX + 3) * PX;
-    static constexpr int THREADS = 32 * TX * TY;
-    static constexpr int PAIR = 8 * DIR; // a stage: 4 octant directions x the two x flips
-    static constexpr int STAGES = 4;
-    static_assert(DIR % 16 == 4 || DIR % 16 == 12, "bank pattern");
+    static constexpr int TY = 4, TZ = 8, RY = TY + 3, RZ = TZ + 4;
+    static constexpr int PZ = 4, PY = RZ * PZ, PX = RY * PY; // strides of a cell along z, y, x
+    static constexpr int SLOT = (TX + 3) * PX;
+    static constexpr int WARPS = TX * TY;           // stencil warps; then TX copy warps
+    static constexpr int COPIERS = 32 * TX, THREADS = 32 * WARPS + COPIERS;
+    // 16-byte copies of a slot: the tile's planes (4 full lines, 3 halo lines), the x halo planes
+    static constexpr int FULL = 2 * RZ, INNER = 2 * TZ, PLANE = TY * FULL + 3 * INNER;
+    static constexpr int COPIES = TX * PLANE + 3 * TY * INNER;
+    static constexpr int PER = (COPIES + COPIERS - 1) / COPIERS;
 };
 
 // flux(c) (+)= sum_q m_q (c_x fx + c_y fy + c_z fz) on the interior cells, c = cosine x weight /
-// spacing, over the rows r0 <= row < r1 of psi (whole groups of 4 octant directions unless r1
-// is the last row). Lane l of a warp owns cell l / 4 of the warp's line and, in group g, octant
-// direction 4 g + l % 4: it forms the stencil of the 8 reflections one after another (a stage
-// holds two, signs known at compile time), transforms the 8 values (sym_wht) and contracts
-// them per class on the FP64 tensor pipe, A fragments straight from registers. Stages are filled
-// by cp.async two pairs ahead, one barrier per pair. VEC: doubles per copy (2 when nz is even,
-// so that rows are 16-byte aligned).
+// spacing, over the rows r0 <= row < r1 of psi (whole groups of 4 octant directions). Lane l of
+// a warp owns cell l / 4 of the warp's line and, in group g, octant direction 4 g + l % 4: it
+// forms the stencil of the 8 reflections one after another (signs known at compile time),
+// transforms the 8 values (sym_wht) and contracts them per class on the FP64 tensor pipe, A
+// fragments straight from registers. A reflection's stage has its own ring slot, filled by
+// copy warps that run up to 8 stages ahead; warps drift against each other inside the ring (full
+// and empty barriers, no CTA barrier).
+// Issue bound: about 100 instructions per cell and direction, half of them FP64.
+// (Bulk copies, one per line of cells, took 76 clocks each: 2.6 times slower as a whole.)
 // wrapFlag (null: no): when it reads 0 the face ghosts' psi is not in place; their values are
 // read at the periodic images.
-template <int DEG, int TX, int VEC>
+template <int DEG, int TX>
 __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
     sym_flux_kernel(GridDims g, const double *__restrict__ psi, const double *__restrict__ tab,
                     const int *__restrict__ idx, int r0, int r1, double th2, int accumulate,
-                    double *__restrict__ flux, const int *wrapFlag)
+                    double *__restrict__ flux, int *errorFlag, const int *wrapFlag)
 {
     using C = SymCls<DEG>;
     using F = FluxTile<TX>;
     constexpr int TAB = C::TILES * 32 + 16; // a group's fragments and weights
-    constexpr int TABC = TAB / 2;           // 16-byte chunks
-    // copies per direction: the tile's planes (4 full rows, 3 halo rows), then the x halo planes
-    constexpr int FULL = F::RZ / VEC, INNER = F::TZ / VEC;
-    constexpr int PLANE = F::TY * FULL + 3 * INNER;
-    constexpr int PERDIR = TX * PLANE + 3 * F::TY * INNER;
-    constexpr int COPIES = (8 * PERDIR + F::THREADS - 1) / F::THREADS;
-    extern __shared__ __align__(128) double smem[]; // STAGES x PAIR, 2 x TAB
-    double *sTab = smem + F::STAGES * F::PAIR;
+    extern __shared__ __align__(128) double smem[]; // 8 x SLOT, 2 x TAB
+    double *sTab = smem + 8 * F::SLOT;
+    __shared__ uint64_t full[8], empty[8];
     const int nm = g.nm, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long nall = g.nall();
     // tiles in blocks of 4 x 4 along x and y with z inside, so that CTAs running together read
@@ -181,81 +198,82 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
         j0 = 2 + (by * B + r / ntz) * F::TY;
         k0 = 2 + (r % ntz) * F::TZ;
     }
-    const bool wrap = wrapFlag && *wrapFlag == 0;
-    // this thread's copies of a stage: destination (-1: none) and source offset from the
-    // stage's first row for either y flip, in doubles. Positions outside the grid read a cell
-    // inside it: only cells outside the grid use them.
-    int dst[COPIES];
-    uint32_t off[COPIES][2];
-#pragma unroll
-    for (int n = 0; n < COPIES; ++n) {
-        const int e = tid + n * F::THREADS;
-        const int dir = e / PERDIR; // bit 2: the x flip, bits 0-1: direction of the group
-        int f = e % PERDIR, X, Y, kc;
-        if (f < TX * PLANE) {
-            X = 2 + f / PLANE;
-            f %= PLANE;
-            if (f < F::TY * FULL) {
-                Y = 2 + f / FULL;
-                kc = (f % FULL) * VEC;
-            } else {
-                f -= F::TY * FULL;
-                Y = f / INNER;
-                Y = Y < 2 ? Y : F::TY + 2;
-                kc = 2 + (f % INNER) * VEC;
-            }
-        } else {
-            f -= TX * PLANE;
-            X = f / (F::TY * INNER);
-            X = X < 2 ? X : TX + 2;
-            f %= F::TY * INNER;
-            Y = 2 + f / INNER;
-            kc = 2 + (f % INNER) * VEC;
+    if (tid == 0) {
+        for (int s = 0; s < 8; ++s) {
+            bar_init(&full[s], F::COPIERS);
+            bar_init(&empty[s], F::WARPS);
         }
-        dst[n] = e < 8 * PERDIR ? (((dir * (TX + 3) + X) * F::RY + Y) * F::RZ + kc) * 8 : -1;
-        auto image = [&](int a, int m) { return !wrap ? a : a < 2 ? a + m : a >= m + 2 && a < m + 4 ? a - m : a; };
-        const int i = min(image(dir & 4 ? i0 + TX + 1 - X : i0 + X - 2, g.nx), g.nxg() - 1);
-        const int k = min(image(k0 - 2 + kc, g.nz), g.nzg() - VEC);
-#pragma unroll
-        for (int sy = 0; sy < 2; ++sy) {
-            const int j = min(image(sy ? j0 + F::TY + 1 - Y : j0 + Y - 2, g.ny), g.nyg() - 1);
-            off[n][sy] = (uint32_t)((8 * (dir & 3) + ((dir >> 2) & 1)) * nall + g.cell(i, j, k));
-        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    const int g0 = r0 / 32, ng = (r1 + 31) / 32 - g0;
-    const uint32_t sBase = saddr(smem);
-    // stage of group g0 + gi, reflections with y and z flips p, into ring slot p. The last
-    // group's directions past r1 read row r1 - 1's octant direction: their weights are 0.
-    auto issue = [&](int gi, int p) {
-        if (gi < ng) {
-            const int row = 32 * gi + 2 * p; // relative to r0
-            const double *src = psi + (long long)row * nall;
-            const uint32_t sb = sBase + (uint32_t)(p * F::PAIR) * 8;
-            const bool last = row + 26 > r1 - r0;
+    __syncthreads();
+    const int g0 = r0 / 32, ng = (r1 - r0 + 31) / 32;
+    if (warp >= F::WARPS) {
+        // Copy warps. A thread's copies have fixed places in a slot; their sources are the cells of
+        // the lines from k0 - 2 (halo lines: the tile's 8 cells) in upwind order for either x and
+        // y flip, at the periodic image of a wrapped ghost. Positions outside the grid read a
+        // cell inside it: only cells outside the grid use them.
+        const bool wrap = wrapFlag && *wrapFlag == 0;
+        auto image = [&](int a, int m) { return !wrap ? a : a < 2 ? a + m : a >= m + 2 && a < m + 4 ? a - m : a; };
+        uint32_t dst[F::PER], off[F::PER][2][2]; // bytes; 16-byte units from the rows' start
+        const int ct = tid - 32 * F::WARPS;
 #pragma unroll
-            for (int n = 0; n < COPIES; ++n) {
-                if (8 * PERDIR % F::THREADS != 0 && dst[n] < 0)
-                    continue;
-                uint32_t o = p & 1 ? off[n][1] : off[n][0];
-                if (last) {
-                    const int dir = (tid + n * F::THREADS) / PERDIR & 3;
-                    const int past = 4 * gi + dir - ((r1 - r0) / 8 - 1);
-                    if (past > 0)
-                        o -= (uint32_t)(8 * past * nall);
+        for (int n = 0; n < F::PER; ++n) {
+            int f = min(ct + n * F::COPIERS, F::COPIES - 1), X, Y, h;
+            if (f < TX * F::PLANE) {
+                X = 2 + f / F::PLANE;
+                f %= F::PLANE;
+                if (f < F::TY * F::FULL) {
+                    Y = 2 + f / F::FULL;
+                    h = f % F::FULL;
+                } else {
+                    f -= F::TY * F::FULL;
+                    Y = f / F::INNER;
+                    Y = Y < 2 ? Y : F::TY + 2;
+                    h = 4 + f % F::INNER;
                 }
-                copy_async<8 * VEC>(sb + (uint32_t)dst[n], src + o);
+            } else {
+                f -= TX * F::PLANE;
+                X = f / (F::TY * F::INNER);
+                X = X < 2 ? X : TX + 2;
+                f %= F::TY * F::INNER;
+                Y = 2 + f / F::INNER;
+                h = 4 + f % F::INNER;
             }
-            if (p == 0)
-                for (int e = tid; e < TABC; e += F::THREADS)
-                    copy_async<16>(saddr(sTab + (gi & 1) * TAB + 2 * e),
-                                   tab + (size_t)(g0 + gi) * TAB + 2 * e);
-        }
-        copy_commit();
-    };
-    static_assert(F::STAGES == 4, "a ring slot per pair of the group");
+            dst[n] = saddr(smem) + (uint32_t)(X * F::PX + Y * F::PY + h * 2) * 8;
+            const int k = min(image(k0 - 2 + h / 2, g.nz), g.nzg() - 1);
 #pragma unroll
-    for (int p = 0; p < F::STAGES - 1; ++p)
-        issue(0, p);
+            for (int sx = 0; sx < 2; ++sx)
+#pragma unroll
+                for (int sy = 0; sy < 2; ++sy) {
+                    const int i = min(image(sx ? i0 + TX + 1 - X : i0 + X - 2, g.nx), g.nxg() - 1);
+                    const int j = min(image(sy ? j0 + F::TY + 1 - Y : j0 + Y - 2, g.ny), g.nyg() - 1);
+                    off[n][sx][sy] = (uint32_t)(2 * g.cell(i, j, k) + (h & 1));
+                }
+        }
+        for (int gi = 0; gi < ng; ++gi) {
+            bool ok = true;
+            sym_for<8>([&](auto ss) {
+                constexpr int s = ss.value;
+                if (gi > 0)
+                    ok = bar_wait(&empty[s], (gi - 1) & 1) && ok;
+                const double *rows = psi + (long long)(8 * gi + s) * nall * 4;
+#pragma unroll
+                for (int n = 0; n < F::PER; ++n)
+                    if (F::COPIES % F::COPIERS == 0 || ct + n * F::COPIERS < F::COPIES)
+                        copy16(dst[n] + s * F::SLOT * 8, rows + 2ull * off[n][s & 1][(s >> 1) & 1]);
+                if (s == 0)
+                    for (int e = ct; e < TAB / 2; e += F::COPIERS)
+                        copy16(saddr(sTab + (gi & 1) * TAB + 2 * e), tab + (size_t)(g0 + gi) * TAB + 2 * e);
+                copy_arrive(&full[s]);
+            });
+            if (!ok) {
+                atomicExch(errorFlag, 1);
+                break;
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        return;
+    }
     const int wx = warp / F::TY, wy = warp % F::TY, z = lane >> 2, d = lane & 3;
     const int i = i0 + wx, j = j0 + wy, k = k0 + z;
     const long long myc =
@@ -268,43 +286,44 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
             const int m = idx[8 * t + 2 * d + e];
             acc[t][e] = accumulate && myc >= 0 && m >= 0 ? flux[myc * nm + m] : 0.0;
         }
-    // offsets of the lane's cell in a direction's stage for either x and y flip
-    int cellAt[2][2];
+    // the lane's cell in a slot for either x and y flip
+    const double *cellAt[2][2];
 #pragma unroll
     for (int sx = 0; sx < 2; ++sx)
 #pragma unroll
         for (int sy = 0; sy < 2; ++sy)
-            cellAt[sx][sy] = (4 * sx + d) * F::DIR + ((sx ? TX - 1 - wx : wx) + 2) * F::PX +
-                             ((sy ? F::TY - 1 - wy : wy) + 2) * F::RZ + z + 2;
-    for (int gi = 0; gi < ng; ++gi) {
+            cellAt[sx][sy] = smem + ((sx ? TX - 1 - wx : wx) + 2) * F::PX +
+                             ((sy ? F::TY - 1 - wy : wy) + 2) * F::PY + (z + 2) * F::PZ + d;
+    bool ok = true;
+    for (int gi = 0; gi < ng && ok; ++gi) {
         double S[8], cx = 0.0, cy = 0.0, cz = 0.0;
         const double *tb = sTab + (gi & 1) * TAB;
-        sym_for<4>([&](auto pp) {
-            constexpr int p = pp.value, sy = p & 1, sz = p >> 1;
-            constexpr int dz = sz ? -1 : 1;
-            copy_wait<F::STAGES - 2>(); // this thread's copies of the stage have landed
-            __syncthreads();            // everyone's, and stage (t - 1)'s readers are done
-            issue(p == 0 ? gi : gi + 1, (p + 3) & 3);
-            const double *st = smem + p * F::PAIR;
-            if (p == 0) {
+        sym_for<8>([&](auto ss) {
+            constexpr int s = ss.value, dz = (s & 4) ? -F::PZ : F::PZ;
+            ok = bar_wait(&full[s], gi & 1) && ok;
+            if (s == 0) {
                 cx = tb[C::TILES * 32 + d];
                 cy = tb[C::TILES * 32 + 4 + d];
                 cz = tb[C::TILES * 32 + 8 + d];
             }
-#pragma unroll
-            for (int sx = 0; sx < 2; ++sx) {
-                const double *q = st + cellAt[sx][sy];
-                const double v0 = q[0];
-                const double fx = sym_axis(th2, q[-2 * F::PX], q[-F::PX], v0, q[F::PX]);
-                const double fy = sym_axis(th2, q[-2 * F::RZ], q[-F::RZ], v0, q[F::RZ]);
-                const double fz = sym_axis(th2, q[-2 * dz], q[-dz], v0, q[dz]);
-                S[sx + 2 * p] = fma(fx, cx, fma(fy, cy, fz * cz));
-            }
+            const double *q = cellAt[s & 1][(s >> 1) & 1] + s * F::SLOT;
+            const double v0 = q[0];
+            const double fx = sym_axis(th2, q[-2 * F::PX], q[-F::PX], v0, q[F::PX]);
+            const double fy = sym_axis(th2, q[-2 * F::PY], q[-F::PY], v0, q[F::PY]);
+            const double fz = sym_axis(th2, q[-2 * dz], q[-dz], v0, q[dz]);
+            S[s] = fma(fx, cx, fma(fy, cy, fz * cz));
+            __syncwarp();
+            if (lane == 0)
+                bar_arrive(&empty[s]);
         });
         sym_wht(S);
         sym_contract<DEG>(S, tb, lane, acc);
     }
-    copy_wait<0>();
+    if (!ok) {
+        if (lane == 0)
+            atomicExch(errorFlag, 1);
+        return;
+    }
     if (myc < 0)
         return;
 #pragma unroll
@@ -354,45 +373,43 @@ cudaError_t launch_sym_ansatz(const SymTables &T, int deg, long long nall, const
 #undef CALL
 }
 
-template <int DEG, int TX, int VEC>
+template <int DEG, int TX>
 static cudaError_t flux_v(const GridDims &g, const double *psi, const double *tab, const int *idx,
-                          int r0, int r1, double th2, double *flux, const int *wrapFlag,
-                          cudaStream_t st)
+                          int r0, int r1, double th2, double *flux, int *errorFlag,
+                          const int *wrapFlag, cudaStream_t st)
 {
     using F = FluxTile<TX>;
-    const int smem = (F::STAGES * F::PAIR + 2 * (SymCls<DEG>::TILES * 32 + 16)) * 8;
-    auto kern = sym_flux_kernel<DEG, TX, VEC>;
+    const int smem = (8 * F::SLOT + 2 * (SymCls<DEG>::TILES * 32 + 16)) * 8;
+    auto kern = sym_flux_kernel<DEG, TX>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
     const long long tiles = (long long)((g.nx + TX - 1) / TX) * ((g.ny + F::TY - 1) / F::TY) *
                             ((g.nz + F::TZ - 1) / F::TZ);
     kern<<<(unsigned)tiles, F::THREADS, smem, st>>>(g, psi, tab, idx, r0, r1, th2, r0 > 0 ? 1 : 0,
-                                                    flux, wrapFlag);
+                                                    flux, errorFlag, wrapFlag);
     return cudaGetLastError();
 }
 
 template <int DEG>
 static cudaError_t flux_t(const GridDims &g, const double *psi, const double *tab, const int *idx,
-                          int r0, int r1, double th2, double *flux, const int *wrapFlag, int numSMs,
-                          cudaStream_t st)
+                          int r0, int r1, double th2, double *flux, int *errorFlag,
+                          const int *wrapFlag, int numSMs, cudaStream_t st)
 {
     const long long lines = (long long)((g.ny + 3) / 4) * ((g.nz + 7) / 8);
-    const bool wide = lines * ((g.nx + 3) / 4) >= 2 * numSMs;
-    if (g.nz % 2 == 0)
-        return wide ? flux_v<DEG, 4, 2>(g, psi, tab, idx, r0, r1, th2, flux, wrapFlag, st)
-                    : flux_v<DEG, 2, 2>(g, psi, tab, idx, r0, r1, th2, flux, wrapFlag, st);
-    return wide ? flux_v<DEG, 4, 1>(g, psi, tab, idx, r0, r1, th2, flux, wrapFlag, st)
-                : flux_v<DEG, 2, 1>(g, psi, tab, idx, r0, r1, th2, flux, wrapFlag, st);
+    return lines * ((g.nx + 3) / 4) >= 2 * numSMs
+               ? flux_v<DEG, 4>(g, psi, tab, idx, r0, r1, th2, flux, errorFlag, wrapFlag, st)
+               : flux_v<DEG, 2>(g, psi, tab, idx, r0, r1, th2, flux, errorFlag, wrapFlag, st);
 }
 
-// The stencil over psi's rows r0 <= row < r1 (psi points at row r0); accumulates when r0 > 0.
+// The stencil over psi's rows r0 <= row < r1 (psi points at row r0, a multiple of 32); accumulates
+// when r0 > 0.
 cudaError_t launch_sym_flux(const GridDims &g, int deg, const double *psi, const double *tab,
                             const int *idx, int r0, int r1, double theta, double *flux,
-                            const int *wrapFlag, int numSMs, cudaStream_t st)
+                            int *errorFlag, const int *wrapFlag, int numSMs, cudaStream_t st)
 {
     const double th2 = theta > 0.0 ? 2.0 * theta : 0.0;
-#define CALL(D) flux_t<D>(g, psi, tab, idx, r0, r1, th2, flux, wrapFlag, numSMs, st)
+#define CALL(D) flux_t<D>(g, psi, tab, idx, r0, r1, th2, flux, errorFlag, wrapFlag, numSMs, st)
     C3D_SYM_DEG(CALL)
 #undef CALL
 }

@@ -79,7 +79,7 @@ bool sym_build(int deg, int expoDeg, int nq, const double *M, const double *w, c
                 return false;
         }
         std::copy(m0, m0 + nm, &B[(size_t)o * nm]);
-        T.w[o] = w[q0];
+        T.w[o / 8 * 8 + 2 * (o % 4) + o / 4 % 2] = w[q0]; // position of direction o
         if (xi) {
             cx[o] = (xi[q0] * w[q0]) * rdx;
             cy[o] = (eta[q0] * w[q0]) * rdy;
@@ -95,11 +95,11 @@ bool sym_build(int deg, int expoDeg, int nq, const double *M, const double *w, c
     for (int b = 0; b < T.nb; ++b)
         for (int l = 0; l < 32; ++l) {
             for (int k = 0; k < steps; ++k)
-                T.expo[((size_t)b * steps + k) * 32 + l] = at(8 * b + l / 4, T.stepIdx[4 * k + l % 4]);
+                T.expo[((size_t)b * steps + k) * 32 + l] = at(sym_at(b, l / 4), T.stepIdx[4 * k + l % 4]);
             for (int h = 0; h < 2; ++h)
                 for (int t = 0; t < tiles; ++t)
                     T.proj[(((size_t)b * 2 + h) * tiles + t) * 32 + l] =
-                        at(8 * b + 2 * (l % 4) + h, T.idx[8 * t + l / 4]);
+                        at(8 * b + 4 * h + l % 4, T.idx[8 * t + l / 4]);
         }
     if (xi) {
         const int ng = 2 * T.nb;
