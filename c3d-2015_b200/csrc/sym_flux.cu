@@ -106,16 +106,18 @@ __global__ void __launch_bounds__(128)
 
 // Slope of the limited reconstruction at a value with differences dm (to its upwind neighbour),
 // dp (to its downwind one) and dc across both, times 4: minmod(th dp, dc / 2, th dm)
-// (src/flux_kinetic.cpp:45-61) scaled by 2, th2 = 2 th >= 0, for dm and dp of one sign (sym_same;
-// dc then has it too, and min(th |dm|, th |dp|) = th min(|dm|, |dp|)); otherwise it is 0.
+// (src/flux_kinetic.cpp:45-61) scaled by 2, th2 = 2 th >= 0, for dm and dp of one sign (dc then has it too, and min(th |dm|, th |dp|) = th min(|dm|, |dp|)); otherwise it is 0.
 __device__ __forceinline__ double sym_slope(double th2, double dm, double dp, double dc)
 {
     const double m = th2 * (fabs(dm) < fabs(dp) ? dm : dp);
     return fabs(dc) < fabs(m) ? dc : m;
 }
-__device__ __forceinline__ bool sym_same(double a, double b)
+// f += q s if a and b have one sign (a predicated FMA; as C++ it became an FMA and two selects)
+__device__ __forceinline__ void sym_add_same(double &f, double q, double s, double a, double b)
 {
-    return (__double2hiint(a) ^ __double2hiint(b)) >= 0;
+    asm("{\n .reg .pred p;\n setp.ge.s32 p, %3, 0;\n @p fma.rn.f64 %0, %1, %2, %0;\n}\n"
+        : "+d"(f)
+        : "d"(q), "d"(s), "r"(__double2hiint(a) ^ __double2hiint(b)));
 }
 
 // Limited upwind difference along one axis in upwind coordinates, v2, v1 the upwind
@@ -130,10 +132,8 @@ __device__ __forceinline__ double sym_axis(double th2, double v2, double v1, dou
     const double d2 = v1 - v2, d1 = v0 - v1, d0 = w1 - v0;
     const double s1 = sym_slope(th2, d1, d0, w1 - v1), s2 = sym_slope(th2, d2, d1, v0 - v2);
     double f = d1;
-    if (sym_same(d1, d0))
-        f = fma(0.25, s1, f);
-    if (sym_same(d2, d1))
-        f = fma(-0.25, s2, f);
+    sym_add_same(f, 0.25, s1, d1, d0);
+    sym_add_same(f, -0.25, s2, d2, d1);
     return f;
 }
 
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
     constexpr int TAB = C::TILES * 32 + 16; // a group's fragments and weights
     extern __shared__ __align__(128) double smem[]; // 8 x SLOT, 2 x TAB
     double *sTab = smem + 8 * F::SLOT;
-    __shared__ uint64_t full[8], empty[8];
+    __shared__ uint64_t full[4], empty[4]; // per pair of slots (the x flips)
     const int nm = g.nm, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long nall = g.nall();
     // tiles in blocks of 4 x 4 along x and y with z inside, so that CTAs running together read
@@ -199,9 +199,9 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
         k0 = 2 + (r % ntz) * F::TZ;
     }
     if (tid == 0) {
-        for (int s = 0; s < 8; ++s) {
-            bar_init(&full[s], F::COPIERS);
-            bar_init(&empty[s], F::WARPS);
+        for (int p = 0; p < 4; ++p) {
+            bar_init(&full[p], F::COPIERS);
+            bar_init(&empty[p], F::WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
             bool ok = true;
             sym_for<8>([&](auto ss) {
                 constexpr int s = ss.value;
-                if (gi > 0)
-                    ok = bar_wait(&empty[s], (gi - 1) & 1) && ok;
+                if (s % 2 == 0 && gi > 0 && !bar_wait(&empty[s / 2], (gi - 1) & 1))
+                    ok = false;
                 const double *rows = psi + (long long)(8 * gi + s) * nall * 4;
 #pragma unroll
                 for (int n = 0; n < F::PER; ++n)
@@ -264,7 +264,8 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
                 if (s == 0)
                     for (int e = ct; e < TAB / 2; e += F::COPIERS)
                         copy16(saddr(sTab + (gi & 1) * TAB + 2 * e), tab + (size_t)(g0 + gi) * TAB + 2 * e);
-                copy_arrive(&full[s]);
+                if (s % 2)
+                    copy_arrive(&full[s / 2]);
             });
             if (!ok) {
                 atomicExch(errorFlag, 1);
@@ -300,7 +301,8 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
         const double *tb = sTab + (gi & 1) * TAB;
         sym_for<8>([&](auto ss) {
             constexpr int s = ss.value, dz = (s & 4) ? -F::PZ : F::PZ;
-            ok = bar_wait(&full[s], gi & 1) && ok;
+            if (s % 2 == 0 && !bar_wait(&full[s / 2], gi & 1))
+                ok = false;
             if (s == 0) {
                 cx = tb[C::TILES * 32 + d];
                 cy = tb[C::TILES * 32 + 4 + d];
@@ -312,9 +314,11 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
             const double fy = sym_axis(th2, q[-2 * F::PY], q[-F::PY], v0, q[F::PY]);
             const double fz = sym_axis(th2, q[-2 * dz], q[-dz], v0, q[dz]);
             S[s] = fma(fx, cx, fma(fy, cy, fz * cz));
-            __syncwarp();
-            if (lane == 0)
-                bar_arrive(&empty[s]);
+            if (s % 2) {
+                __syncwarp();
+                if (lane == 0)
+                    bar_arrive(&empty[s / 2]);
+            }
         });
         sym_wht(S);
         sym_contract<DEG>(S, tb, lane, acc);
