@@ -321,7 +321,8 @@ static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **b
     auto add = [&](const void *src, size_t bytes) {
         const size_t at = all.size(), n = (bytes + 127) / 128 * 16; // 128-byte aligned parts
         all.resize(at + n);
-        std::memcpy(all.data() + at, src, bytes);
+        if (bytes)
+            std::memcpy(all.data() + at, src, bytes);
         return at;
     };
     const size_t e = add(H.expo.data(), H.expo.size() * 8), p = add(H.proj.data(), H.proj.size() * 8),
@@ -632,6 +633,7 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
         R.streamLen = c->gStreamLen;
         R.symN = c->symN;
         R.sym2 = c->sym2;
+        c->cp.sym = c->gaunt && c->symN.no > 0;
         R.m0 = c->m0;
         R.ncells = n;
         R.cellMap = cellMap;
@@ -741,7 +743,7 @@ static c3d_status run_closure(c3d_ctx *c, long long n, double *u, double *alpha,
             c->psiHandoffPending = true;
         return C3D_OK;
     }
-    c->cp.probe = 0; // the persistent kernels always form H
+    c->cp.probe = c->cp.sym = 0; // the persistent kernels always form H
     if (gridRecords)
         psi_invalidate(c);
     ClosureLaunch L{};

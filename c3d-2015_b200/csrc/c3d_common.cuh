@@ -78,6 +78,7 @@ struct ClosureParams {
     // in [gramLo, gramHi] (Gershgorin), bounds the condition estimate and |d| = |H^-1 g|,
     // so a cell whose visit would end converged is finalized without H (see after_probe)
     int probe;
+    int sym;           // octant-symmetric passes (sym.cuh)
     double gramLo, gramHi;
 };
 
@@ -92,8 +93,8 @@ struct __align__(16) GauntTerm {
     int slot;
 };
 
-// Threads of the work-list Newton kernel (4 cells of one warp each); the Gaunt assembly
-// streams are laid out for this many threads.
+// Threads of a CTA of the work-list Newton kernel; the Gaunt assembly streams are laid out for
+// this many threads.
 constexpr int NEWTON_THREADS = 128;
 
 // Grid with two ghost layers per face; cell (i,j,k) with k fastest (src/global.h:15).

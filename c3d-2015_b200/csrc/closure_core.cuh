@@ -88,8 +88,15 @@ __host__ __device__ constexpr int tpair(int l) { return toff(l >> 2, 2 * (l & 3)
 // tile element (r, c) at toff(r, c); lane l of the m8n8k4 DMMA accumulator layout holds the
 // pair at tpair(l). Padding rows are those of the identity. 16-byte alignment keeps
 // L of every slot in an array aligned for the double2 tile accesses.
+//
+// W lanes of a warp work on a cell: the fewest (8, 16 or 32) that cover its padded rows twice, so
+// that a warp carries 4, 2 or 1 cells and the serial parts (pivots, substitutions, sums in the
+// reference's order) are issued once for all of them. The persistent engine keeps whole warps.
+__host__ __device__ constexpr int cell_lanes(int nt) { return nt <= 2 ? 8 : nt <= 4 ? 16 : 32; }
+
 template <int NT, bool TILED = false> struct alignas(16) Slot {
     static constexpr int NMP = Cfg<NT>::NMP;
+    static constexpr int W = TILED ? cell_lanes(NT) : 32;
     static constexpr int NTILES = NT * (NT + 1) / 2;
     static constexpr int LSIZE = TILED ? 64 * NTILES : Cfg<NT>::NPK;
     static constexpr bool tiled = TILED;
@@ -129,22 +136,53 @@ __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
+// The lanes of a cell: mask, synchronisation and exchanges among them (lane arguments of the
+// functions below count from the cell's first lane).
+template <class S> __device__ __forceinline__ unsigned cell_mask()
+{
+    return S::W == 32 ? FULL_MASK : ((1u << (S::W & 31)) - 1u) << (threadIdx.x & 31 & ~(S::W - 1));
+}
+template <class S> __device__ __forceinline__ void cell_sync() { __syncwarp(cell_mask<S>()); }
+template <class S, class V> __device__ __forceinline__ V cell_shfl(V v, int src)
+{
+    return __shfl_sync(cell_mask<S>(), v, src, S::W);
+}
+template <class S> __device__ __forceinline__ bool cell_any(bool v)
+{
+    return __any_sync(cell_mask<S>(), v);
+}
+template <class S> __device__ __forceinline__ double cell_sum(double v)
+{
+#pragma unroll
+    for (int o = S::W / 2; o > 0; o >>= 1)
+        v += __shfl_xor_sync(cell_mask<S>(), v, o);
+    return v;
+}
+template <class S> __device__ __forceinline__ double cell_max(double v)
+{
+#pragma unroll
+    for (int o = S::W / 2; o > 0; o >>= 1)
+        v = fmax(v, __shfl_xor_sync(cell_mask<S>(), v, o));
+    return v;
+}
+
 // First index of the largest |x| (LAPACK idamax semantics).
-__device__ __forceinline__ int warp_iamax(double a0, double a1, int lane, int n)
+template <class S>
+__device__ __forceinline__ int cell_iamax(double a0, double a1, int lane, int n)
 {
     double best = (lane < n) ? fabs(a0) : -1.0;
     int bi = lane;
-    if (lane + 32 < n) {
+    if (lane + S::W < n) {
         double b = fabs(a1);
         if (b > best) {
             best = b;
-            bi = lane + 32;
+            bi = lane + S::W;
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(FULL_MASK, best, o);
-        int oi = __shfl_xor_sync(FULL_MASK, bi, o);
+    for (int o = S::W / 2; o > 0; o >>= 1) {
+        double ob = __shfl_xor_sync(cell_mask<S>(), best, o);
+        int oi = __shfl_xor_sync(cell_mask<S>(), bi, o);
         if (ob > best || (ob == best && oi < bi)) {
             best = ob;
             bi = oi;
@@ -278,7 +316,7 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
             rj[j] = 1.0;
             // padding columns (identity rows, zero couplings, last tile only) stay as they are
             if (8 * kb + j < n) {
-                const double ajj = __shfl_sync(FULL_MASK, v[j], j);
+                const double ajj = cell_shfl<S>(v[j], j);
                 if (!(ajj > 0.0) && info == 0)
                     info = 8 * kb + j + 1;
                 // root and reciprocal both from the pivot, so that neither waits for the other
@@ -290,13 +328,13 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
                     v[j] *= rj[j];
 #pragma unroll
                 for (int c = j + 1; c < 8; ++c) {
-                    const double lc = __shfl_sync(FULL_MASK, v[j], c);
+                    const double lc = cell_shfl<S>(v[j], c);
                     if (row >= c)
                         v[c] = fma(-v[j], lc, v[c]);
                 }
             }
         }
-        __syncwarp();
+        cell_sync<S>();
         if (lane < 8) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -309,9 +347,9 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
                 *reinterpret_cast<double2 *>(&sl.rinv[8 * kb + 2 * q]) =
                     make_double2(rj[2 * q], rj[2 * q + 1]);
         }
-        __syncwarp();
+        cell_sync<S>();
 #pragma unroll 1
-        for (int i = lane; i < 8 * (T - 1 - kb); i += 32) {
+        for (int i = lane; i < 8 * (T - 1 - kb); i += S::W) {
             double *P = A + 64 * tix(kb + 1 + (i >> 3), kb);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -331,25 +369,61 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
                 *reinterpret_cast<double2 *>(&P[toff(i & 7, 2 * q)]) =
                     make_double2(v[2 * q], v[2 * q + 1]);
         }
-        __syncwarp();
-        const int f0 = toff(lane >> 2, lane & 3), f1 = toff(lane >> 2, 4 + (lane & 3));
+        cell_sync<S>();
+        if constexpr (S::W == 32) {
+            const int f0 = toff(lane >> 2, lane & 3), f1 = toff(lane >> 2, 4 + (lane & 3));
 #pragma unroll 1
-        for (int jb = kb + 1; jb < T; ++jb) {
-            const double *Bt = A + 64 * tix(jb, kb);
-            const double b0 = Bt[f0], b1 = Bt[f1];
-            // (four tiles at a time with loads first took 126 registers instead of 96 and was
-            // 4% slower on the standalone orders, whose warps per SM it lowers)
+            for (int jb = kb + 1; jb < T; ++jb) {
+                const double *Bt = A + 64 * tix(jb, kb);
+                const double b0 = Bt[f0], b1 = Bt[f1];
+                // (four tiles at a time with loads first took 126 registers instead of 96 and was
+                // 4% slower on the standalone orders, whose warps per SM it lowers)
 #pragma unroll 2
-            for (int ib = jb; ib < T; ++ib) {
-                const double *At = A + 64 * tix(ib, kb);
-                double2 *cp = reinterpret_cast<double2 *>(&A[64 * tix(ib, jb) + tpair(lane)]);
-                double2 c = *cp;
-                dmma(c.x, c.y, -At[f0], b0);
-                dmma(c.x, c.y, -At[f1], b1);
-                *cp = c;
+                for (int ib = jb; ib < T; ++ib) {
+                    const double *At = A + 64 * tix(ib, kb);
+                    double2 *cp = reinterpret_cast<double2 *>(&A[64 * tix(ib, jb) + tpair(lane)]);
+                    double2 c = *cp;
+                    dmma(c.x, c.y, -At[f0], b0);
+                    dmma(c.x, c.y, -At[f1], b1);
+                    *cp = c;
+                }
+            }
+        } else {
+            // part of a warp per cell: row i's 8 columns of each trailing tile by FMAs
+#pragma unroll 1
+            for (int i = lane; i < 8 * (T - 1 - kb); i += S::W) {
+                const int ib = kb + 1 + (i >> 3), r = i & 7;
+                const double *P = A + 64 * tix(ib, kb);
+                double p[8];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double2 x = *reinterpret_cast<const double2 *>(&P[toff(r, 2 * q)]);
+                    p[2 * q] = x.x;
+                    p[2 * q + 1] = x.y;
+                }
+#pragma unroll 1
+                for (int jb = kb + 1; jb <= ib; ++jb) {
+                    const double *B = A + 64 * tix(jb, kb);
+                    double *C = A + 64 * tix(ib, jb);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        double2 *cp = reinterpret_cast<double2 *>(&C[toff(r, 2 * q)]);
+                        double2 c = *cp;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const double2 x = *reinterpret_cast<const double2 *>(&B[toff(2 * q, 2 * k)]);
+                            const double2 y = *reinterpret_cast<const double2 *>(&B[toff(2 * q + 1, 2 * k)]);
+                            c.x = fma(-p[2 * k], x.x, c.x);
+                            c.x = fma(-p[2 * k + 1], x.y, c.x);
+                            c.y = fma(-p[2 * k], y.x, c.y);
+                            c.y = fma(-p[2 * k + 1], y.y, c.y);
+                        }
+                        *cp = c;
+                    }
+                }
             }
         }
-        __syncwarp();
+        cell_sync<S>();
     }
     return info;
 }
@@ -385,34 +459,34 @@ __device__ void warp_apply_inverse(const S &sl, int n, int lane, double &x0, dou
     }
     const double *P = sl.L;
     for (int k = 0; k < n; ++k) {
-        double v = (k < 32) ? x0 : x1;
-        double xk = __shfl_sync(FULL_MASK, v, k & 31);
+        double v = (k < S::W) ? x0 : x1;
+        double xk = cell_shfl<S>(v, k & (S::W - 1));
         xk = exactDiv ? xk / P[S::lx(k, k)] : xk * sl.rinv[k];
-        if (lane == (k & 31)) {
-            if (k < 32)
+        if (lane == (k & (S::W - 1))) {
+            if (k < S::W)
                 x0 = xk;
             else
                 x1 = xk;
         }
         if (lane > k && lane < n)
             x0 = fma(-P[S::lx(lane, k)], xk, x0);
-        if (lane + 32 > k && lane + 32 < n)
-            x1 = fma(-P[S::lx(lane + 32, k)], xk, x1);
+        if (lane + S::W > k && lane + S::W < n)
+            x1 = fma(-P[S::lx(lane + S::W, k)], xk, x1);
     }
     for (int k = n - 1; k >= 0; --k) {
-        double v = (k < 32) ? x0 : x1;
-        double xk = __shfl_sync(FULL_MASK, v, k & 31);
+        double v = (k < S::W) ? x0 : x1;
+        double xk = cell_shfl<S>(v, k & (S::W - 1));
         xk = exactDiv ? xk / P[S::lx(k, k)] : xk * sl.rinv[k];
-        if (lane == (k & 31)) {
-            if (k < 32)
+        if (lane == (k & (S::W - 1))) {
+            if (k < S::W)
                 x0 = xk;
             else
                 x1 = xk;
         }
         if (lane < k && lane < n)
             x0 = fma(-P[S::lx(k, lane)], xk, x0);
-        if (lane + 32 < k && lane + 32 < n)
-            x1 = fma(-P[S::lx(k, lane + 32)], xk, x1);
+        if (lane + S::W < k && lane + S::W < n)
+            x1 = fma(-P[S::lx(k, lane + S::W)], xk, x1);
     }
 }
 
@@ -432,10 +506,10 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
     const int own = lane & 7;
     // the block's values and reciprocals; the lane's own row takes its value back
     auto gather = [&](int kb, double (&y)[8], double (&r)[8]) {
-        const double v = kb < 4 ? x0 : x1;
+        const double v = kb < S::W / 8 ? x0 : x1;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            y[i] = __shfl_sync(FULL_MASK, v, (8 * kb + i) & 31);
+            y[i] = cell_shfl<S>(v, (8 * kb + i) & (S::W - 1));
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double2 t = *reinterpret_cast<const double2 *>(&sl.rinv[8 * kb + 2 * q]);
@@ -448,8 +522,8 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
 #pragma unroll
         for (int i = 1; i < 8; ++i)
             v = own == i ? y[i] : v;
-        if ((lane >> 3) == (kb & 3)) {
-            if (kb < 4)
+        if ((lane >> 3) == (kb & (S::W / 8 - 1))) {
+            if (kb < S::W / 8)
                 x0 = v;
             else
                 x1 = v;
@@ -478,8 +552,8 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
                     x0 = fma(-l.y, y[2 * q + 1], x0);
                 }
             }
-            if (NMP > 32 && lane + 32 >= 8 * kb + 8 && lane + 32 < NMP) {
-                const double *Lt = A + 64 * tix((lane + 32) >> 3, kb);
+            if (NMP > S::W && lane + S::W >= 8 * kb + 8 && lane + S::W < NMP) {
+                const double *Lt = A + 64 * tix((lane + S::W) >> 3, kb);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const double2 l = *reinterpret_cast<const double2 *>(&Lt[toff(own, 2 * q)]);
@@ -508,8 +582,8 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
             for (int c = 0; c < 8; ++c)
                 x0 = fma(-Lt[toff(c, own)], y[c], x0);
         }
-        if (NMP > 32 && lane + 32 < 8 * kb) {
-            const double *Lt = A + 64 * tix(kb, (lane + 32) >> 3);
+        if (NMP > S::W && lane + S::W < 8 * kb) {
+            const double *Lt = A + 64 * tix(kb, (lane + S::W) >> 3);
 #pragma unroll
             for (int c = 0; c < 8; ++c)
                 x1 = fma(-Lt[toff(c, own)], y[c], x1);
@@ -517,10 +591,11 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
     }
 }
 
+template <class S>
 __device__ __forceinline__ double vsum_abs(double x0, double x1, int lane, int n)
 {
-    double s = (lane < n ? fabs(x0) : 0.0) + (lane + 32 < n ? fabs(x1) : 0.0);
-    return warp_sum(s);
+    double s = (lane < n ? fabs(x0) : 0.0) + (lane + S::W < n ? fabs(x1) : 0.0);
+    return cell_sum<S>(s);
 }
 
 // Hager/Higham 1-norm estimate of (L L^T)^{-1} (N. J. Higham, ACM TOMS 14 (1988)
@@ -535,24 +610,24 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm)
     warp_apply_inverse(sl, n, lane, x0, x1, false);
     double est;
     if (n == 1) {
-        est = fabs(__shfl_sync(FULL_MASK, x0, 0));
+        est = fabs(cell_shfl<S>(x0, 0));
     } else {
-        est = vsum_abs(x0, x1, lane, n);
+        est = vsum_abs<S>(x0, x1, lane, n);
         int s0 = x0 >= 0.0 ? 1 : -1, s1 = x1 >= 0.0 ? 1 : -1;
         x0 = (double)s0;
         x1 = (double)s1;
         warp_apply_inverse(sl, n, lane, x0, x1, false);
-        int j = warp_iamax(x0, x1, lane, n);
+        int j = cell_iamax<S>(x0, x1, lane, n);
         int iter = 2;
         for (;;) {
             x0 = (lane == j) ? 1.0 : 0.0;
-            x1 = (lane + 32 == j) ? 1.0 : 0.0;
+            x1 = (lane + S::W == j) ? 1.0 : 0.0;
             warp_apply_inverse(sl, n, lane, x0, x1, false);
             double estold = est;
-            est = vsum_abs(x0, x1, lane, n);
+            est = vsum_abs<S>(x0, x1, lane, n);
             bool diff = (lane < n && (x0 >= 0.0 ? 1 : -1) != s0) ||
-                        (lane + 32 < n && (x1 >= 0.0 ? 1 : -1) != s1);
-            bool same = !__any_sync(FULL_MASK, diff);
+                        (lane + S::W < n && (x1 >= 0.0 ? 1 : -1) != s1);
+            bool same = !cell_any<S>(diff);
             if (same || est <= estold)
                 break;
             s0 = x0 >= 0.0 ? 1 : -1;
@@ -561,9 +636,9 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm)
             x1 = (double)s1;
             warp_apply_inverse(sl, n, lane, x0, x1, false);
             int jlast = j;
-            j = warp_iamax(x0, x1, lane, n);
-            double xjl = __shfl_sync(FULL_MASK, jlast < 32 ? x0 : x1, jlast & 31);
-            double xj = fabs(__shfl_sync(FULL_MASK, j < 32 ? x0 : x1, j & 31));
+            j = cell_iamax<S>(x0, x1, lane, n);
+            double xjl = cell_shfl<S>(jlast < S::W ? x0 : x1, jlast & (S::W - 1));
+            double xj = fabs(cell_shfl<S>(j < S::W ? x0 : x1, j & (S::W - 1)));
             if (xjl != xj && iter < 5) {
                 ++iter;
                 continue;
@@ -571,9 +646,9 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm)
             break;
         }
         x0 = ((lane & 1) ? -1.0 : 1.0) * (1.0 + (double)lane / (double)(n - 1));
-        x1 = (((lane + 32) & 1) ? -1.0 : 1.0) * (1.0 + (double)(lane + 32) / (double)(n - 1));
+        x1 = (((lane + S::W) & 1) ? -1.0 : 1.0) * (1.0 + (double)(lane + S::W) / (double)(n - 1));
         warp_apply_inverse(sl, n, lane, x0, x1, false);
-        double temp = 2.0 * (vsum_abs(x0, x1, lane, n) / (double)(3 * n));
+        double temp = 2.0 * (vsum_abs<S>(x0, x1, lane, n) / (double)(3 * n));
         if (temp > est)
             est = temp;
     }
@@ -583,14 +658,15 @@ __device__ double warp_condest(const S &sl, int n, int lane, double anorm)
     return 1.0 / rcond;
 }
 
-__device__ __forceinline__ double warp_nrm2(const double *v, int n, int lane)
+template <class S>
+__device__ __forceinline__ double cell_nrm2(const double *v, int n, int lane)
 {
     double s = 0.0;
     if (lane < n)
         s = v[lane] * v[lane];
-    if (lane + 32 < n)
-        s = fma(v[lane + 32], v[lane + 32], s);
-    return sqrt(warp_sum(s));
+    if (lane + S::W < n)
+        s = fma(v[lane + S::W], v[lane + S::W], s);
+    return sqrt(cell_sum<S>(s));
 }
 
 // ---------------------------------------------------------------- Newton state machine
@@ -610,10 +686,10 @@ __device__ void finalize(S &sl, const ClosureParams &P, const Outputs &O, int la
 {
     const int nm = P.nm;
     long long c = sl.s.cell;
-    __syncwarp();
+    cell_sync<S>();
     if (sl.s.status != CELL_NONPOSITIVE_U0) {
         // postProcess: rescale (src/opt/optBatch.cpp:334-344, src/opt/opt.cpp:352-354)
-        for (int i = lane; i < nm; i += 32) {
+        for (int i = lane; i < nm; i += S::W) {
             O.u[c * nm + i] = sl.u[i] * sl.s.u0;
             double a = sl.alpha[i];
             if (i == 0)
@@ -647,7 +723,7 @@ __device__ void finalize(S &sl, const ClosureParams &P, const Outputs &O, int la
         sl.s.need = NEED_NONE;
         sl.s.cell = -1;
     }
-    __syncwarp();
+    cell_sync<S>();
 }
 
 // Regularise (src/opt/opt.cpp:251-279). Returns false if the ladder is exhausted.
@@ -655,18 +731,18 @@ template <class S>
 __device__ bool regularize(S &sl, const ClosureParams &P, int lane)
 {
     const int nm = P.nm;
-    __syncwarp();
+    cell_sync<S>();
     if (sl.s.regIndex >= P.nreg - 1)
         return false;
     int ri = sl.s.regIndex + 1;
     double r = P.reg[ri];
-    for (int i = lane; i < nm; i += 32)
+    for (int i = lane; i < nm; i += S::W)
         sl.u[i] = (i == 0) ? 1.0 : sl.uOrig[i] * (1.0 - r);
-    __syncwarp();
-    double rt = P.batched ? P.tol : warp_nrm2(sl.u, nm, lane) * P.tol;
-    for (int i = lane; i < nm; i += 32)
+    cell_sync<S>();
+    double rt = P.batched ? P.tol : cell_nrm2<S>(sl.u, nm, lane) * P.tol;
+    for (int i = lane; i < nm; i += S::W)
         sl.alpha[i] = sl.alpha0[i];
-    __syncwarp();
+    cell_sync<S>();
     if (lane == 0) {
         sl.s.regIndex = ri;
         sl.s.r = r;
@@ -677,7 +753,7 @@ __device__ bool regularize(S &sl, const ClosureParams &P, int lane)
         if (!P.batched && ri == P.nreg - 1)
             sl.s.maxIter = 10 * sl.s.maxIter;
     }
-    __syncwarp();
+    cell_sync<S>();
     return true;
 }
 
@@ -688,19 +764,19 @@ template <class S>
 __device__ void begin_iteration(S &sl, const ClosureParams &P, const Outputs &O, int lane)
 {
     for (;;) {
-        __syncwarp();
+        cell_sync<S>();
         int maxIterEff = sl.s.maxIter;
         if (P.batched && sl.s.regIndex == P.nreg - 1)
             maxIterEff = 10 * P.maxIter;
         int iter = sl.s.iter + 1, total = sl.s.totalIter + 1;
         long long passes = sl.s.passes + 1;
-        __syncwarp();
+        cell_sync<S>();
         if (lane == 0) {
             sl.s.iter = iter;
             sl.s.totalIter = total;
             sl.s.passes = passes;
         }
-        __syncwarp();
+        cell_sync<S>();
         if (passes > P.passBudget) {
             if (lane == 0)
                 sl.s.status = CELL_PASS_BUDGET;
@@ -718,7 +794,7 @@ __device__ void begin_iteration(S &sl, const ClosureParams &P, const Outputs &O,
         }
         if (lane == 0)
             sl.s.need = (P.probe && total == 1) ? NEED_PROBE : NEED_H;
-        __syncwarp();
+        cell_sync<S>();
         return;
     }
 }
@@ -731,7 +807,7 @@ __device__ void load_cell(S &sl, const ClosureParams &P, const Outputs &O, long 
     constexpr int NMP = S::NMP;
     double u0 = O.u[c * nm];
     double alphaScale = log(u0) * 2.0 * sqrt(M_PI);
-    for (int i = lane; i < NMP; i += 32) {
+    for (int i = lane; i < NMP; i += S::W) {
         double ui = 0.0, ai = 0.0;
         if (i < nm) {
             ui = O.u[c * nm + i] / u0;
@@ -746,8 +822,8 @@ __device__ void load_cell(S &sl, const ClosureParams &P, const Outputs &O, long 
         sl.g[i] = 0.0;
         sl.d[i] = 0.0;
     }
-    __syncwarp();
-    double rt = P.batched ? P.tol : warp_nrm2(sl.u, nm, lane) * P.tol;
+    cell_sync<S>();
+    double rt = P.batched ? P.tol : cell_nrm2<S>(sl.u, nm, lane) * P.tol;
     if (lane == 0) {
         sl.s.cell = c;
         sl.s.passes = 0;
@@ -769,7 +845,7 @@ __device__ void load_cell(S &sl, const ClosureParams &P, const Outputs &O, long 
         sl.s.cshift = 0;
         sl.s.hprec = 0;
     }
-    __syncwarp();
+    cell_sync<S>();
     if (u0 <= 0) {
         if (lane == 0)
             sl.s.status = CELL_NONPOSITIVE_U0;
@@ -788,22 +864,22 @@ __device__ void next_trial(S &sl, const ClosureParams &P, const Outputs &O, int 
 {
     const int nm = P.nm;
     double t = sl.s.t;
-    __syncwarp();
+    cell_sync<S>();
     if (t * sl.s.maxFactor > EPS_HALF) {
-        for (int i = lane; i < nm; i += 32)
+        for (int i = lane; i < nm; i += S::W)
             sl.alpha[i] = __dadd_rn(sl.alphaOld[i], __dmul_rn(t, sl.d[i]));
-        __syncwarp();
+        cell_sync<S>();
         if (lane == 0) {
             sl.s.need = NEED_TRIAL;
             if (O.stats)
                 atomicAdd(&O.stats[STAT_TRIALS], 1ull);
         }
-        __syncwarp();
+        cell_sync<S>();
     } else {
         // backtracked all the way (src/opt/linesearch.cpp:76-78)
-        for (int i = lane; i < nm; i += 32)
+        for (int i = lane; i < nm; i += S::W)
             sl.alpha[i] = sl.alphaOld[i];
-        __syncwarp();
+        cell_sync<S>();
         // mixed precision: a direction from a reduced-precision Hessian is not the reference's
         // Newton direction; the iteration is redone from alphaOld with FP64 moments instead of
         // regularising
@@ -816,7 +892,7 @@ __device__ void next_trial(S &sl, const ClosureParams &P, const Outputs &O, int 
                     atomicAdd(&O.stats[STAT_ESCALATED], 1ull);
             }
         }
-        __syncwarp();
+        cell_sync<S>();
         begin_iteration(sl, P, O, lane);
     }
 }
@@ -826,7 +902,7 @@ __device__ void next_trial(S &sl, const ClosureParams &P, const Outputs &O, int 
 template <class S>
 __device__ void escalate_fp64(S &sl, const Outputs &O, int lane)
 {
-    __syncwarp();
+    cell_sync<S>();
     if (lane == 0) {
         sl.s.fp64 = 1;
         sl.s.passes += 1;
@@ -834,7 +910,7 @@ __device__ void escalate_fp64(S &sl, const Outputs &O, int lane)
         if (O.stats)
             atomicAdd(&O.stats[STAT_ESCALATED], 1ull);
     }
-    __syncwarp();
+    cell_sync<S>();
 }
 
 // gext (mixed precision): the FP64 moments <m_i e^{alpha.m}> and fqext = <e^{alpha.m}> of
@@ -848,11 +924,11 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     const int nm = P.nm;
     C3D_NCLK_DECL
     // g_i = H_i0 / m_0 - u_i ; f = H_00 / m_0^2 - alpha.u  (src/opt/fobj.cpp:121-129)
-    for (int i = lane; i < nm; i += 32)
+    for (int i = lane; i < nm; i += S::W)
         sl.g[i] = gext ? __dsub_rn(gext[i], sl.u[i]) : sl.L[S::lx(i, 0)] / m0 - sl.u[i];
-    __syncwarp();
+    cell_sync<S>();
     if (gext && P.mixPolish > 0.0) {
-        const double e0 = warp_nrm2(sl.g, nm, lane);
+        const double e0 = cell_nrm2<S>(sl.g, nm, lane);
         if (e0 > sl.s.rtol && e0 <= P.mixPolish * sl.s.rtol) {
             escalate_fp64(sl, O, lane);
             return;
@@ -864,10 +940,10 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
         for (int i = 0; i < nm; ++i)
             f = __dsub_rn(f, __dmul_rn(sl.alpha[i], sl.u[i]));
     }
-    f = __shfl_sync(FULL_MASK, f, 0);
+    f = cell_shfl<S>(f, 0);
     // 1-norm: max row sum of |H| (src/utils.cpp:35-49)
     double rs = 0.0, gmin = 1.0 / 0.0;
-    for (int i = lane; i < nm; i += 32) {
+    for (int i = lane; i < nm; i += S::W) {
         double s = 0.0;
         if constexpr (S::tiled) {
             // row i = the row segments of tiles (ib, jb <= ib) and the column segments of
@@ -896,8 +972,8 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
         rs = fmax(rs, s);
         gmin = fmin(gmin, 2.0 * sl.L[S::lx(i, i)] - s); // Gershgorin: H_ii - sum_{j!=i} |H_ij|
     }
-    double norm1 = warp_max(rs);
-    gmin = -warp_max(-gmin);
+    double norm1 = cell_max<S>(rs);
+    gmin = -cell_max<S>(-gmin);
     // All eigenvalues of H are >= gmin, so when gmin > 0, ||H^-1||_1 <= sqrt(n)/gmin and the
     // 1-norm condition number is at most norm1 sqrt(n)/gmin. The Hager estimate can only be
     // smaller, so if this bound is below condHMax/2 the reference's test `condest > condHMax`
@@ -911,7 +987,7 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     bool condSure = gmin > 0.0 && norm1 * sqrt((double)nm) / gmin <= 0.5 * P.condHMax;
     if (lane == 0) // the condition record: the bound, or the estimate below
         sl.s.cnd = condSure ? norm1 * sqrt((double)nm) / gmin : 0.0;
-    __syncwarp();
+    cell_sync<S>();
     C3D_NCLK(O.stats, 1, lane);
     int info = warp_cholesky(sl, nm, lane);
     C3D_NCLK(O.stats, 2, lane);
@@ -919,13 +995,13 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     if (info == 0) {
         // reciprocal pivots (the tiled factorisation leaves them in rinv)
         if constexpr (!S::tiled)
-            for (int i = lane; i < nm; i += 32)
+            for (int i = lane; i < nm; i += S::W)
                 sl.rinv[i] = 1.0 / sl.L[S::lx(i, i)];
-        __syncwarp();
+        cell_sync<S>();
         if (!condSure)
             cond = warp_condest(sl, nm, lane, norm1);
     }
-    __syncwarp();
+    cell_sync<S>();
     C3D_NCLK(O.stats, 3, lane);
 
     if (lane == 0 && (info != 0 || !condSure))
@@ -937,20 +1013,20 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     }
     if (sl.s.totalIter == 1 && bad) {
         // isotropic restart (src/opt/opt.cpp:236-247)
-        double rt = P.batched ? P.tol : warp_nrm2(sl.u, nm, lane) * P.tol;
-        for (int i = lane; i < nm; i += 32) {
+        double rt = P.batched ? P.tol : cell_nrm2<S>(sl.u, nm, lane) * P.tol;
+        for (int i = lane; i < nm; i += S::W) {
             double a = (i == 0) ? 2.0 * sqrt(M_PI) * log(0.5 / sqrt(M_PI)) : 0.0;
             sl.alpha0[i] = a;
             sl.alpha[i] = a;
         }
-        __syncwarp();
+        cell_sync<S>();
         if (lane == 0) {
             sl.s.rtol = rt;
             sl.s.iter = 0;
             sl.s.iterGamma = 0;
             sl.s.t = 1.0;
         }
-        __syncwarp();
+        cell_sync<S>();
         begin_iteration(sl, P, O, lane);
         return;
     }
@@ -969,16 +1045,16 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
     }
     // d = -H^{-1} g
     double x0 = lane < nm ? sl.g[lane] : 0.0;
-    double x1 = lane + 32 < nm ? sl.g[lane + 32] : 0.0;
+    double x1 = lane + S::W < nm ? sl.g[lane + S::W] : 0.0;
     warp_apply_inverse(sl, nm, lane, x0, x1, true);
     if (lane < nm)
         sl.d[lane] = -x0;
-    if (lane + 32 < nm)
-        sl.d[lane + 32] = -x1;
-    __syncwarp();
+    if (lane + S::W < nm)
+        sl.d[lane + S::W] = -x1;
+    cell_sync<S>();
     C3D_NCLK(O.stats, 4, lane);
-    double err = warp_nrm2(sl.g, nm, lane);
-    double d1 = vsum_abs(x0, x1, lane, nm);
+    double err = cell_nrm2<S>(sl.g, nm, lane);
+    double d1 = vsum_abs<S>(x0, x1, lane, nm);
     int pnOrder = (int)floor(sqrt((double)nm)) + 1;
     double minf = sqrt((2 * pnOrder + 1) / (2 * M_PI));
     double gamma = exp(2.0 * d1 * minf);
@@ -987,20 +1063,20 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
         sl.s.err = err;
         sl.s.gamma = gamma;
     }
-    __syncwarp();
+    cell_sync<S>();
     if (err <= tolEff && gamma <= P.tolGamma) {
         finalize(sl, P, O, lane);
         return;
     }
     // line search set-up (src/opt/linesearch.cpp:41-54)
     double mf = 0.0;
-    for (int i = lane; i < nm; i += 32) {
+    for (int i = lane; i < nm; i += S::W) {
         sl.alphaOld[i] = sl.alpha[i];
         mf = fmax(mf, fabs(sl.d[i]) / (fabs(sl.alpha[i]) + 1e-100));
     }
-    mf = warp_max(mf);
+    mf = cell_max<S>(mf);
     double gd = 0.0;
-    __syncwarp();
+    cell_sync<S>();
     if (lane == 0) {
         for (int i = 0; i < nm; ++i)
             gd = __dadd_rn(gd, __dmul_rn(sl.g[i], sl.d[i]));
@@ -1011,7 +1087,7 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
         sl.s.gd = gd;
         sl.s.t = 1.0;
     }
-    __syncwarp();
+    cell_sync<S>();
     next_trial(sl, P, O, lane);
 }
 
@@ -1035,7 +1111,7 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
 {
     const int nm = P.nm;
     constexpr int NMP = S::NMP;
-    for (int i = lane; i < nm; i += 32) {
+    for (int i = lane; i < nm; i += S::W) {
         double gi;
         if (g0) {
             double h = 0.0;
@@ -1050,8 +1126,8 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
         }
         sl.g[i] = gi;
     }
-    __syncwarp();
-    const double err = warp_nrm2(sl.g, nm, lane);
+    cell_sync<S>();
+    const double err = cell_nrm2<S>(sl.g, nm, lane);
     const double emin = pm[NMP + 1], emax = pm[NMP + 2];
     int maxIterEff = sl.s.maxIter;
     if (P.batched && sl.s.regIndex == P.nreg - 1)
@@ -1067,7 +1143,7 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
         gexp = 2.0 * minf * sqrt((double)nm) * err / lam;
         ok = k1 <= 0.25 * P.condHMax && gexp <= 0.5 * log(P.tolGamma);
     }
-    __syncwarp();
+    cell_sync<S>();
     if (ok) {
         if (lane == 0) {
             sl.s.err = err;
@@ -1076,7 +1152,7 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
             if (O.stats)
                 atomicAdd(&O.stats[STAT_CERTIFIED], 1ull);
         }
-        __syncwarp();
+        cell_sync<S>();
         finalize(sl, P, O, lane);
         return;
     }
@@ -1089,7 +1165,7 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
         if (P.mixed && P.mixPolish > 0.0 && err > sl.s.rtol && err <= P.mixPolish * sl.s.rtol)
             sl.s.fp64 = 1;
     }
-    __syncwarp();
+    cell_sync<S>();
 }
 
 template <class S>
@@ -1103,17 +1179,17 @@ __device__ void after_trial(S &sl, const ClosureParams &P, const Outputs &O, int
         for (int i = 0; i < nm; ++i)
             fnew = __dsub_rn(fnew, __dmul_rn(sl.alpha[i], sl.u[i]));
     }
-    fnew = __shfl_sync(FULL_MASK, fnew, 0);
+    fnew = cell_shfl<S>(fnew, 0);
     double t = sl.s.t;
     bool accept = fnew <= __dadd_rn(sl.s.f, __dmul_rn(__dmul_rn(1e-3, t), sl.s.gd));
-    __syncwarp();
+    cell_sync<S>();
     if (accept) {
         begin_iteration(sl, P, O, lane);
         return;
     }
     if (lane == 0)
         sl.s.t = 0.5 * t;
-    __syncwarp();
+    cell_sync<S>();
     next_trial(sl, P, O, lane);
 }
 

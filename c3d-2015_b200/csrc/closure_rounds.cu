@@ -39,12 +39,14 @@ template <int NT> struct CellState {
 
 namespace {
 
+template <int W>
 __device__ __forceinline__ void copy_scalars(SlotScalars &dst, const SlotScalars &src, int lane)
 {
-    static_assert(sizeof(SlotScalars) % 8 == 0 && sizeof(SlotScalars) <= 256, "one word per lane");
-    if (lane < (int)sizeof(SlotScalars) / 8)
-        reinterpret_cast<unsigned long long *>(&dst)[lane] =
-            reinterpret_cast<const unsigned long long *>(&src)[lane];
+    static_assert(sizeof(SlotScalars) % 8 == 0, "whole words");
+#pragma unroll
+    for (int i = lane; i < (int)sizeof(SlotScalars) / 8; i += W)
+        reinterpret_cast<unsigned long long *>(&dst)[i] =
+            reinterpret_cast<const unsigned long long *>(&src)[i];
 }
 
 // lineSearch = false skips d and alphaOld, which a Hessian visit recomputes before use.
@@ -52,7 +54,7 @@ template <int NT, class S>
 __device__ void state_to_slot(const CellState<NT> &st, S &sl, int lane, bool lineSearch = true)
 {
     constexpr int NMP = Cfg<NT>::NMP;
-    for (int i = lane; i < NMP; i += 32) {
+    for (int i = lane; i < NMP; i += S::W) {
         sl.u[i] = st.u[i];
         sl.alpha[i] = st.alpha[i];
         sl.alpha0[i] = st.alpha0[i];
@@ -62,16 +64,16 @@ __device__ void state_to_slot(const CellState<NT> &st, S &sl, int lane, bool lin
             sl.alphaOld[i] = st.alphaOld[i];
         }
     }
-    copy_scalars(sl.s, st.s, lane);
-    __syncwarp();
+    copy_scalars<S::W>(sl.s, st.s, lane);
+    cell_sync<S>();
 }
 
 template <int NT, class S>
 __device__ void slot_to_state(const S &sl, CellState<NT> &st, int lane)
 {
     constexpr int NMP = Cfg<NT>::NMP;
-    __syncwarp();
-    for (int i = lane; i < NMP; i += 32) {
+    cell_sync<S>();
+    for (int i = lane; i < NMP; i += S::W) {
         st.u[i] = sl.u[i];
         st.alpha[i] = sl.alpha[i];
         st.alpha0[i] = sl.alpha0[i];
@@ -79,13 +81,23 @@ __device__ void slot_to_state(const S &sl, CellState<NT> &st, int lane)
         st.d[i] = sl.d[i];
         st.alphaOld[i] = sl.alphaOld[i];
     }
-    copy_scalars(st.s, sl.s, lane);
+    copy_scalars<S::W>(st.s, sl.s, lane);
 }
 
 // The work lists of one round: 0 trials and FP64 Hessian passes, 1 BF16 Hessian passes,
 // 2 3xTF32 Hessian passes (lists 1 and 2: mixed-precision closure only), 3 first visits
-// through the probe pass (convergence certificate).
+// through the probe pass (convergence certificate) or, with an octant-symmetric quadrature (whose
+// probe visits never enter a list), trials and FP64 Hessian passes in the reference's order.
 constexpr int NLISTS = 4;
+
+// 2-norm of a cell's multipliers beyond alpha_0 from which the passes of a symmetric quadrature
+// keep the reference's order over the full basis. Such cells sit at the realizability boundary
+// (exponents to -1600, condition numbers to 1e9, steps of 1e-3 along directions of 1e6, a few
+// directions carrying the moments), where the rounding of the basis and of the sums decides at
+// which multipliers inside the stopping tolerance the iteration ends: on M_6 pulses with the
+// symmetric passes they ended 1e-8 to 1e-7 from the oracle's, in its order 5e-10 to 5e-9.
+// Standalone vectors with components of unit variance reach 8 (N = 7).
+constexpr double REF_NORM = 32.0;
 struct Lists {
     int *list[NLISTS];
     unsigned int *count[NLISTS];
@@ -94,13 +106,13 @@ struct Lists {
 // The list of a cell's next pass. Mixed precision: the Hessian's moments in BF16 when the
 // last condition estimate is <= condBf16, in 3xTF32 up to condMixMax or when there is no
 // estimate yet, else (and after mixIterMax iterations at one regularisation level, or once a
-// reduced-precision factorisation failed) in FP64.
-template <class S> __device__ int route_list(const S &sl, const ClosureParams &P)
+// reduced-precision factorisation failed) in FP64; far: the multipliers exceed REF_NORM.
+template <class S> __device__ int route_list(const S &sl, const ClosureParams &P, bool far)
 {
     if (sl.s.need == NEED_PROBE)
         return 3;
     if (sl.s.need != NEED_H || !P.mixed || sl.s.fp64 || sl.s.iter > P.mixIterMax)
-        return 0;
+        return far ? 3 : 0;
     const double c = sl.s.cnd;
     if (c < 0.0)
         return 2;
@@ -108,7 +120,7 @@ template <class S> __device__ int route_list(const S &sl, const ClosureParams &P
         return 1;
     if (c <= P.condMixMax)
         return 2;
-    return 0;
+    return far ? 3 : 0;
 }
 
 // Appends cell c to its list when it still needs a pass.
@@ -116,9 +128,17 @@ template <class S>
 __device__ void append_if_needed(const S &sl, const ClosureParams &P, long long c, int lane,
                                  const Lists &out)
 {
+    bool far = false;
+    if (P.sym) {
+        cell_sync<S>();
+        double a2 = 0.0;
+        for (int i = lane; i < P.nm; i += S::W)
+            a2 = i > 0 ? fma(sl.alpha[i], sl.alpha[i], a2) : a2;
+        far = !(cell_sum<S>(a2) <= REF_NORM * REF_NORM);
+    }
     if (lane == 0 && sl.s.need != NEED_NONE) {
         // selects, not an indexed parameter array (which would be copied to local memory)
-        const int l = route_list(sl, P);
+        const int l = route_list(sl, P, far);
         unsigned int *cnt = l == 0   ? out.count[0]
                             : l == 1 ? out.count[1]
                             : l == 2 ? out.count[2]
@@ -132,7 +152,8 @@ __device__ void append_if_needed(const S &sl, const ClosureParams &P, long long 
 } // namespace
 
 constexpr int RW = 8;  // warps (cells) per CTA of the init and pass kernels
-constexpr int RWN = 4; // warps (cells) per CTA of the Newton kernel
+// cells per CTA of the Newton kernel (NEWTON_THREADS threads, cell_lanes of them per cell)
+__host__ __device__ constexpr int newton_cells(int nt) { return NEWTON_THREADS / cell_lanes(nt); }
 
 // Entries a round kernel works on: n, or with nDev (the list's device counter, as the
 // graph-resident round loop launches them) the smaller of n and *nDev.
@@ -146,7 +167,7 @@ template <int NT> using TSlot = Slot<NT, true>;
 // Per-warp state of a first visit after the probe pass: the vectors and scalars of Slot
 // without the factor (the probe's Newton kernel forms no Hessian).
 template <int NT> struct alignas(16) ProbeSlot {
-    static constexpr int NMP = Cfg<NT>::NMP;
+    static constexpr int NMP = Cfg<NT>::NMP, W = cell_lanes(NT);
     double u[NMP], alpha[NMP], alpha0[NMP], uOrig[NMP], g[NMP], d[NMP], alphaOld[NMP];
     double pm[NMP + 8]; // the cell's probe entry, loaded before the cell's state
     SlotScalars s;
@@ -1195,7 +1216,7 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
     }
 }
 
-// Newton logic for the listed cells: one warp per cell, RWN cells per CTA, state staged
+// Newton logic for the listed cells: cell_lanes(NT) lanes per cell, state staged
 // in shared memory with H in the tiled layout (TSlot).
 // MODE 0: FP64 Hessians and trials. MODE 1: the list of a mixed-precision pass (entries of
 // mix_entry_doubles): H from the reduced-precision moments, g and f from the pass's FP64
@@ -1205,11 +1226,10 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
 // 1 BF16, 2 3xTF32, 3 probe).
 // GAUNT: the CTA assembles H_ij = sum_k beta_ijk mom_k (i >= j, the CSR terms of beta in
 // the order of src/opt/fobj.cpp:81-99, laid out per tile slot by c3d_set_gaunt) for its
-// cells that need a Hessian in one sweep over the tile slots, so that each term is read once
-// for RWN cells. The cells' moments sit in the slots' g..rinv vectors, which a Hessian visit
+// cells that need a Hessian in one sweep over the tile slots per four cells. The cells' moments sit in the slots' g..rinv vectors, which a Hessian visit
 // recomputes afterwards. Otherwise the pass wrote H in tiles to hBuf.
 template <int NT, int NT2, bool GAUNT, int MODE>
-__global__ void __launch_bounds__(RWN * 32)
+__global__ void __launch_bounds__(NEWTON_THREADS)
     rounds_newton_kernel(ClosureParams P, double m0, const int *__restrict__ list, int n,
                          const unsigned int *nDev, CellState<NT> *state,
                          const double *__restrict__ buf,
@@ -1217,8 +1237,9 @@ __global__ void __launch_bounds__(RWN * 32)
                          Outputs Og, Lists out, int level, const GauntTerm *__restrict__ g0,
                          int g0n, FirstRound first, bool fused)
 {
+    constexpr int W = cell_lanes(NT), CELLS = newton_cells(NT);
     n = round_entries(n, nDev);
-    if (blockIdx.x * RWN >= n)
+    if (blockIdx.x * CELLS >= n)
         return;
     constexpr bool MIX = MODE == 1;
     constexpr int NM2P = 8 * NT2;
@@ -1230,30 +1251,30 @@ __global__ void __launch_bounds__(RWN * 32)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using SlotT = NewtonSlot<NT, MODE>;
     SlotT *slots = reinterpret_cast<SlotT *>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & (W - 1), ci = tid / W; // ci: the CTA's cell
     // the CTA's closure counters, added to the context's once at the end (one global atomic
     // per counter and CTA instead of several per finished cell)
     __shared__ unsigned long long sStat[STAT_COUNT];
-    for (int q = tid; q < STAT_COUNT; q += RWN * 32)
+    for (int q = tid; q < STAT_COUNT; q += NEWTON_THREADS)
         sStat[q] = 0;
     __syncthreads();
     Outputs O = Og;
     if (Og.stats)
         O.stats = sStat;
-    const int pos = blockIdx.x * RWN + warp;
+    const int pos = blockIdx.x * CELLS + ci;
     const bool active = pos < n;
     const long long cell = active ? (list ? list[pos] : first.off + pos) : -1;
     bool needH = MODE != 2 && active && state[cell].s.need == NEED_H;
-    SlotT &sl = slots[warp];
+    SlotT &sl = slots[ci];
     // probe visits: the probe entry's loads go out before the cell's state is read, so the
     // two global round trips overlap
-    constexpr int PMR = (BSTR + 31) / 32;
+    constexpr int PMR = (BSTR + W - 1) / W;
     double pmr[PMR];
     if constexpr (MODE == 2)
         if (active)
 #pragma unroll
             for (int r = 0; r < PMR; ++r)
-                pmr[r] = lane + 32 * r < BSTR ? buf[(size_t)pos * BSTR + lane + 32 * r] : 0.0;
+                pmr[r] = lane + W * r < BSTR ? buf[(size_t)pos * BSTR + lane + W * r] : 0.0;
     C3D_NCLK_DECL
     long long gcell = -1; // probe visits: the grid cell, for the ansatz hand-off's marks
     if (MODE == 2 && active && first.mark)
@@ -1289,57 +1310,58 @@ __global__ void __launch_bounds__(RWN * 32)
     if constexpr (MODE == 2) {
     } else if (GAUNT) {
         if (__syncthreads_or(needH)) {
-            // The CTA's moments, cells innermost, so that a term's loads for all cells are two
-            // 16-byte accesses: moment k of cell w at offset 4 (k / 4) + w of slot k % 4's scratch
-            // (g, d, alphaOld, rinv: NM2P <= 4 NMP doubles). Slots whose cell needs no Hessian
-            // hold nothing in theirs any more.
-            static_assert(RWN == 4, "moment layout");
+            // The moments of each four cells, cells innermost, so that a term's loads for them are
+            // two 16-byte accesses: moment k of cell w of the four at offset 4 (k / 4) + w of slot
+            // k % 4's scratch (g, d, alphaOld, rinv: NM2P <= 4 NMP doubles). Slots whose cell
+            // needs no Hessian hold nothing in theirs any more.
+            static_assert(CELLS % 4 == 0, "moment layout");
             bool nf = false;
-            for (int k = lane; k < NM2P; k += 32) {
+            for (int k = lane; k < NM2P; k += W) {
                 const double v = needH ? buf[(size_t)pos * BSTR + k] : 0.0;
                 nf |= MIX && !isfinite(v);
-                slots[k & 3].scratch()[(k & ~3) + warp] = v;
+                slots[(ci & ~3) + (k & 3)].scratch()[(k & ~3) + (ci & 3)] = v;
             }
-            nonFinite = __any_sync(FULL_MASK, nf);
+            nonFinite = cell_any<SlotT>(nf);
             // identity padding: the last tile row's rows past nm
             if (needH) {
                 constexpr int T = NT;
-                for (int t = 0; t < T; ++t)
-                    *reinterpret_cast<double2 *>(&sl.L[64 * tix(T - 1, t) + 2 * lane]) =
+                for (int e = lane; e < 32 * T; e += W)
+                    *reinterpret_cast<double2 *>(&sl.L[64 * tix(T - 1, 0) + 2 * e]) =
                         make_double2(0.0, 0.0);
-                __syncwarp();
+                cell_sync<SlotT>();
                 if (lane < 8 && 8 * (T - 1) + lane >= P.nm)
                     sl.L[64 * tix(T - 1, T - 1) + toff(lane, lane)] = 1.0;
             }
-            __shared__ int sNeedH[RWN];
+            __shared__ int sNeedH[CELLS];
             if (lane == 0)
-                sNeedH[warp] = needH;
+                sNeedH[ci] = needH;
             __syncthreads();
-            bool hw[RWN];
+#pragma unroll 1
+            for (int c4 = 0; c4 < CELLS; c4 += 4) {
+                bool hw[4], any = false;
 #pragma unroll
-            for (int w = 0; w < RWN; ++w)
-                hw[w] = sNeedH[w] != 0;
-            static_assert(RWN * 32 == NEWTON_THREADS, "stream layout");
-            double h[RWN];
-#pragma unroll
-            for (int w = 0; w < RWN; ++w)
-                h[w] = 0.0;
+                for (int w = 0; w < 4; ++w)
+                    any |= hw[w] = sNeedH[c4 + w] != 0;
+                if (!any)
+                    continue;
+                double h[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 8
-            for (int k = 0; k < streamLen; ++k) {
-                const GauntTerm gt = stream[k * NEWTON_THREADS + tid];
-                const double *m = slots[gt.col & 3].scratch() + (gt.col & ~3);
-                const double2 m01 = *reinterpret_cast<const double2 *>(m);
-                const double2 m23 = *reinterpret_cast<const double2 *>(m + 2);
-                h[0] = __dadd_rn(h[0], __dmul_rn(m01.x, gt.v));
-                h[1] = __dadd_rn(h[1], __dmul_rn(m01.y, gt.v));
-                h[2] = __dadd_rn(h[2], __dmul_rn(m23.x, gt.v));
-                h[3] = __dadd_rn(h[3], __dmul_rn(m23.y, gt.v));
-                if (gt.slot >= 0) {
+                for (int k = 0; k < streamLen; ++k) {
+                    const GauntTerm gt = stream[k * NEWTON_THREADS + tid];
+                    const double *m = slots[c4 + (gt.col & 3)].scratch() + (gt.col & ~3);
+                    const double2 m01 = *reinterpret_cast<const double2 *>(m);
+                    const double2 m23 = *reinterpret_cast<const double2 *>(m + 2);
+                    h[0] = __dadd_rn(h[0], __dmul_rn(m01.x, gt.v));
+                    h[1] = __dadd_rn(h[1], __dmul_rn(m01.y, gt.v));
+                    h[2] = __dadd_rn(h[2], __dmul_rn(m23.x, gt.v));
+                    h[3] = __dadd_rn(h[3], __dmul_rn(m23.y, gt.v));
+                    if (gt.slot >= 0) {
 #pragma unroll
-                    for (int w = 0; w < RWN; ++w) {
-                        if (hw[w])
-                            slots[w].L[gt.slot] = h[w];
-                        h[w] = 0.0;
+                        for (int w = 0; w < 4; ++w) {
+                            if (hw[w])
+                                slots[c4 + w].L[gt.slot] = h[w];
+                            h[w] = 0.0;
+                        }
                     }
                 }
             }
@@ -1348,9 +1370,9 @@ __global__ void __launch_bounds__(RWN * 32)
     } else if (needH) {
         const double2 *H = reinterpret_cast<const double2 *>(buf + (size_t)pos * LS);
         double2 *L = reinterpret_cast<double2 *>(sl.L);
-        for (int e = lane; e < LS / 2; e += 32)
+        for (int e = lane; e < LS / 2; e += W)
             L[e] = H[e];
-        __syncwarp();
+        cell_sync<SlotT>();
     }
     if (active && !(tried && !needH)) {
     C3D_NCLK(O.stats, 0, lane);
@@ -1358,9 +1380,9 @@ __global__ void __launch_bounds__(RWN * 32)
         if (sl.s.need == NEED_PROBE) {
 #pragma unroll
             for (int r = 0; r < PMR; ++r)
-                if (lane + 32 * r < BSTR)
-                    sl.pm[lane + 32 * r] = pmr[r];
-            __syncwarp();
+                if (lane + W * r < BSTR)
+                    sl.pm[lane + W * r] = pmr[r];
+            cell_sync<SlotT>();
             after_probe(sl, P, O, lane, m0, sl.pm, g0, g0n);
         }
     } else if (needH) {
@@ -1405,7 +1427,7 @@ __global__ void __launch_bounds__(RWN * 32)
     }
     __syncthreads();
     if (Og.stats)
-        for (int q = tid; q < STAT_COUNT; q += RWN * 32) {
+        for (int q = tid; q < STAT_COUNT; q += NEWTON_THREADS) {
             const unsigned long long v = sStat[q];
             if (v == 0)
                 continue;
@@ -1669,13 +1691,13 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                              (int)slotSmem);
     if (e != cudaSuccess)
         return e;
-    size_t newtonSmem = RWN * sizeof(TSlot<NT>);
+    size_t newtonSmem = newton_cells(NT) * sizeof(TSlot<NT>);
     e = cudaFuncSetAttribute(rounds_newton_kernel<NT, NT2, GAUNT, 0>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)newtonSmem);
     if (e != cudaSuccess)
         return e;
     const bool probe = GAUNT && P.probe;
-    const size_t probeSmem = RWN * sizeof(ProbeSlot<NT>);
+    const size_t probeSmem = newton_cells(NT) * sizeof(ProbeSlot<NT>);
     size_t passSmem, mixSmem[3] = {0, 0, 0};
     // octant-symmetric quadrature: the passes of sym.cuh
     const bool sym = GAUNT && R.symN.no > 0;
@@ -1746,13 +1768,24 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
     // the lists the graph's rounds can fill: FP64 Hessian passes and, when the mixed closure
     // routes any visit to reduced precision, its BF16 and 3xTF32 ones (probe passes happen in
     // round 0 only: no later visit is a first visit)
-    const unsigned int usedLists = 1u | (mixed && P.mixIterMax > 0 ? 6u : 0u);
+    const unsigned int usedLists = 1u | (mixed && P.mixIterMax > 0 ? 6u : 0u) | (sym ? 8u : 0u);
 
     // pass + Newton kernels of list l: entries la[0 .. nb) (with nDev, at most *nDev of them),
     // the cells still in need appended to out
     auto launch_list = [&](int l, const int *la, int nb, const unsigned int *nDev, const Lists &out,
                            cudaStream_t s) {
-        if (l == 3) {
+        if (l == 3 && sym) {
+            // the reference's order for cells far out
+            if constexpr (GAUNT) {
+                rounds_pass_gaunt_kernel<NT, NT2>
+                    <<<(unsigned)((nb + RWP - 1) / RWP), RW * 32, passSmem, s>>>(
+                        P, R.chunks, R.nm2, la, nb, nDev, state, R.buf, R.errorFlag);
+                rounds_newton_kernel<NT, NT2, GAUNT, 0>
+                    <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS,
+                       newtonSmem, s>>>(P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O,
+                                        out, 0, nullptr, 0, FirstRound{}, false);
+            }
+        } else if (l == 3) {
             // probe passes of first visits (Gaunt form only)
             if constexpr (GAUNT) {
                 const unsigned grid = (unsigned)((nb + MXC - 1) / MXC);
@@ -1765,7 +1798,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                         P, R.mixF64, nullptr, la, nb, nDev, state, R.buf, R.errorFlag,
                         FirstRound{});
                 rounds_newton_kernel<NT, NT2, GAUNT, 2>
-                    <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, probeSmem, s>>>(
+                    <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS, probeSmem, s>>>(
                         P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, l,
                         mixed ? nullptr : R.g0, R.g0n, FirstRound{}, false);
             }
@@ -1782,7 +1815,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                         P, R.mixF64, R.mixA[1], la, nb, nDev, state, R.buf, R.errorFlag,
                         FirstRound{});
                 rounds_newton_kernel<NT, NT2, GAUNT, 1>
-                    <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, newtonSmem, s>>>(
+                    <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS, newtonSmem, s>>>(
                         P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, l,
                         nullptr, 0, FirstRound{}, false);
             }
@@ -1802,7 +1835,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                     <<<(unsigned)((nb + RW - 1) / RW), RW * 32, passSmem, s>>>(
                         P, R.chunks, la, nb, nDev, state, R.buf, R.errorFlag);
             rounds_newton_kernel<NT, NT2, GAUNT, 0>
-                <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, newtonSmem, s>>>(
+                <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS, newtonSmem, s>>>(
                     P, m0, la, nb, nDev, state, R.buf, R.gstream, R.streamLen, O, out, 0, nullptr,
                     0, FirstRound{}, sym);
         }
@@ -1836,7 +1869,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                             P, R.mixF64, nullptr, nullptr, nb, nullptr, state, R.buf, R.errorFlag,
                             fr);
                     rounds_newton_kernel<NT, NT2, GAUNT, 2>
-                        <<<(unsigned)((nb + RWN - 1) / RWN), RWN * 32, probeSmem, s>>>(
+                        <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS, probeSmem, s>>>(
                             P, m0, nullptr, nb, nullptr, state, R.buf, R.gstream, R.streamLen, O,
                             A, 3, mixed ? nullptr : R.g0, R.g0n, fr, false);
                     *R.launches += 2;
