@@ -283,6 +283,19 @@ __device__ int warp_cholesky_packed(S &sl, int n, int lane)
     return 0;
 }
 
+// l = sqrt(a) and r = 1 / sqrt(a): the root by one correction of a r (within an ulp), off the
+// chain of pivots, which waits for r alone.
+__device__ __forceinline__ void root(double a, double &l, double &r)
+{
+    r = rsqrt(a);
+    if (a > 1e-280 && a < 1e280) {
+        l = a * r;
+        l = fma(fma(-l, l, a), 0.5 * r, l);
+    } else {
+        l = sqrt(a); // zero, negative, not finite, or a square that underflows
+    }
+}
+
 // Blocked Cholesky of the tiled lower triangle (Slot<NT, true>); returns LAPACK info.
 // Per tile column kb: lane l holds row l % 8 of the diagonal tile (the four octets repeat each
 // other) and the 8 columns are factored with shuffles inside the tile; then each lane solves
@@ -319,9 +332,8 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
                 const double ajj = cell_shfl<S>(v[j], j);
                 if (!(ajj > 0.0) && info == 0)
                     info = 8 * kb + j + 1;
-                // root and reciprocal both from the pivot, so that neither waits for the other
-                const double ljj = sqrt(ajj);
-                rj[j] = rsqrt(ajj);
+                double ljj;
+                root(ajj, ljj, rj[j]);
                 if (row == j)
                     v[j] = ljj;
                 else if (row > j)
@@ -535,11 +547,15 @@ __device__ __forceinline__ void warp_apply_inverse_tiled(const S &sl, int lane, 
         double y[8], r[8];
         gather(kb, y, r);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            y[i] *= r[i];
+        for (int k = 0; k < 8; ++k) {
 #pragma unroll
-            for (int k = i + 1; k < 8; ++k)
-                y[k] = fma(-D[toff(k, i)], y[i], y[k]);
+            for (int q = 0; 2 * q < k; ++q) {
+                const double2 l = *reinterpret_cast<const double2 *>(&D[toff(k, 2 * q)]);
+                y[k] = fma(-l.x, y[2 * q], y[k]);
+                if (2 * q + 1 < k)
+                    y[k] = fma(-l.y, y[2 * q + 1], y[k]);
+            }
+            y[k] *= r[k];
         }
         scatter(kb, y);
         if (kb + 1 < T) {
@@ -913,13 +929,32 @@ __device__ void escalate_fp64(S &sl, const Outputs &O, int lane)
     cell_sync<S>();
 }
 
+// f0 - sum_i a_i b_i (SUB) or f0 + sum_i a_i b_i over i < n in ascending order, unfused as the
+// reference's loops: the products by the cell's lanes, through rinv (free outside
+// the substitutions), the sum by its first lane. Returned to all lanes.
+template <bool SUB, class S>
+__device__ __forceinline__ double serial_dot(S &sl, double f0, const double *a, const double *b,
+                                             int n, int lane)
+{
+    for (int i = lane; i < n; i += S::W)
+        sl.rinv[i] = __dmul_rn(a[i], b[i]);
+    cell_sync<S>();
+    if (lane == 0)
+#pragma unroll 4
+        for (int i = 0; i < n; ++i)
+            f0 = SUB ? __dsub_rn(f0, sl.rinv[i]) : __dadd_rn(f0, sl.rinv[i]);
+    f0 = cell_shfl<S>(f0, 0);
+    cell_sync<S>();
+    return f0;
+}
+
 // gext (mixed precision): the FP64 moments <m_i e^{alpha.m}> and fqext = <e^{alpha.m}> of
 // the pass, from which g and f are formed instead of from row 0 of the reduced-precision H.
-// emin: a lower bound of e^{alpha.m} over the quadrature (0: none).
+// emin, emax: bounds of e^{alpha.m} over the quadrature (0: none).
 template <class S>
 __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, int lane,
                               double m0, const double *gext = nullptr, double fqext = 0.0,
-                              double emin = 0.0)
+                              double emin = 0.0, double emax = 0.0)
 {
     const int nm = P.nm;
     C3D_NCLK_DECL
@@ -934,59 +969,56 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
             return;
         }
     }
-    double f = 0.0;
-    if (lane == 0) {
-        f = gext ? fqext : sl.L[0] / (m0 * m0);
-        for (int i = 0; i < nm; ++i)
-            f = __dsub_rn(f, __dmul_rn(sl.alpha[i], sl.u[i]));
-    }
-    f = cell_shfl<S>(f, 0);
-    // 1-norm: max row sum of |H| (src/utils.cpp:35-49)
-    double rs = 0.0, gmin = 1.0 / 0.0;
-    for (int i = lane; i < nm; i += S::W) {
-        double s = 0.0;
-        if constexpr (S::tiled) {
-            // row i = the row segments of tiles (ib, jb <= ib) and the column segments of
-            // tiles (ib' > ib, ib); padding entries are 0
-            const int ib = i >> 3, r = i & 7;
-            for (int jb = 0; jb < ib; ++jb) {
-                const double *Lt = sl.L + 64 * tix(ib, jb);
+    const double f = serial_dot<true>(sl, gext ? fqext : sl.L[0] / (m0 * m0), sl.alpha, sl.u, nm, lane);
+    // emin G <= H <= emax G bounds the 1-norm condition number by nm kappa_2 (after_probe); when
+    // that settles the test `condest > condHMax` -- with room for rounding -- neither norms nor
+    // estimate are needed. The mixed closure routes by the record, so it takes the estimate.
+    double norm1 = 0.0, record = nm * (emax * P.gramHi) / (0.5 * emin * P.gramLo);
+    bool condSure = !P.mixed && emin > 0.0 && P.gramLo > 0.0 && record <= 1e12 &&
+                    record <= 0.25 * P.condHMax;
+    if (!condSure) {
+        // 1-norm: max row sum of |H| (src/utils.cpp:35-49)
+        double rs = 0.0, gmin = 1.0 / 0.0;
+        for (int i = lane; i < nm; i += S::W) {
+            double s = 0.0;
+            if constexpr (S::tiled) {
+                // row i = the row segments of tiles (ib, jb <= ib) and the column segments of
+                // tiles (ib' > ib, ib); padding entries are 0
+                const int ib = i >> 3, r = i & 7;
+                for (int jb = 0; jb < ib; ++jb) {
+                    const double *Lt = sl.L + 64 * tix(ib, jb);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        s += fabs(Lt[toff(r, c)]);
+                }
+                const double *D = sl.L + 64 * tix(ib, ib);
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
-                    s += fabs(Lt[toff(r, c)]);
-            }
-            const double *D = sl.L + 64 * tix(ib, ib);
+                    s += fabs(c <= r ? D[toff(r, c)] : D[toff(c, r)]);
+                for (int ib2 = ib + 1; ib2 < S::nt; ++ib2) {
+                    const double *Lt = sl.L + 64 * tix(ib2, ib);
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-                s += fabs(c <= r ? D[toff(r, c)] : D[toff(c, r)]);
-            for (int ib2 = ib + 1; ib2 < S::nt; ++ib2) {
-                const double *Lt = sl.L + 64 * tix(ib2, ib);
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    s += fabs(Lt[toff(c, r)]);
+                    for (int c = 0; c < 8; ++c)
+                        s += fabs(Lt[toff(c, r)]);
+                }
+            } else {
+                for (int j = 0; j < nm; ++j)
+                    s += fabs(j <= i ? sl.L[S::lx(i, j)] : sl.L[S::lx(j, i)]);
             }
-        } else {
-            for (int j = 0; j < nm; ++j)
-                s += fabs(j <= i ? sl.L[S::lx(i, j)] : sl.L[S::lx(j, i)]);
+            rs = fmax(rs, s);
+            gmin = fmin(gmin, 2.0 * sl.L[S::lx(i, i)] - s); // Gershgorin: H_ii - sum_{j!=i} |H_ij|
         }
-        rs = fmax(rs, s);
-        gmin = fmin(gmin, 2.0 * sl.L[S::lx(i, i)] - s); // Gershgorin: H_ii - sum_{j!=i} |H_ij|
+        norm1 = cell_max<S>(rs);
+        gmin = -cell_max<S>(-gmin);
+        // All eigenvalues of H are >= gmin, so when gmin > 0, ||H^-1||_1 <= sqrt(n)/gmin and the
+        // 1-norm condition number is at most norm1 sqrt(n)/gmin. The Hager estimate can only be
+        // smaller, so if this bound is below condHMax/2 the reference's test is false whatever the
+        // estimate; the estimate is then skipped.
+        record = norm1 * sqrt((double)nm) / gmin;
+        condSure = gmin > 0.0 && record <= 0.5 * P.condHMax;
     }
-    double norm1 = cell_max<S>(rs);
-    gmin = -cell_max<S>(-gmin);
-    // All eigenvalues of H are >= gmin, so when gmin > 0, ||H^-1||_1 <= sqrt(n)/gmin and the
-    // 1-norm condition number is at most norm1 sqrt(n)/gmin. The Hager estimate can only be
-    // smaller, so if this bound is below condHMax/2 the reference's test `condest > condHMax`
-    // is false whatever the estimate; the estimate is then skipped.
-    // H >= e_min G bounds the smallest eigenvalue too (after_probe), halved for rounding, which
-    // must be far below it. The mixed closure routes by the record, so there only the Gershgorin
-    // bound replaces the estimate.
-    const double lam = 0.5 * emin * P.gramLo;
-    if (!P.mixed && lam > 1e-12 * norm1)
-        gmin = fmax(gmin, lam);
-    bool condSure = gmin > 0.0 && norm1 * sqrt((double)nm) / gmin <= 0.5 * P.condHMax;
     if (lane == 0) // the condition record: the bound, or the estimate below
-        sl.s.cnd = condSure ? norm1 * sqrt((double)nm) / gmin : 0.0;
+        sl.s.cnd = condSure ? record : 0.0;
     cell_sync<S>();
     C3D_NCLK(O.stats, 1, lane);
     int info = warp_cholesky(sl, nm, lane);
@@ -1075,11 +1107,9 @@ __device__ void after_hessian(S &sl, const ClosureParams &P, const Outputs &O, i
         mf = fmax(mf, fabs(sl.d[i]) / (fabs(sl.alpha[i]) + 1e-100));
     }
     mf = cell_max<S>(mf);
-    double gd = 0.0;
     cell_sync<S>();
+    const double gd = serial_dot<false>(sl, 0.0, sl.g, sl.d, nm, lane);
     if (lane == 0) {
-        for (int i = 0; i < nm; ++i)
-            gd = __dadd_rn(gd, __dmul_rn(sl.g[i], sl.d[i]));
         if (err <= tolEff)
             sl.s.iterGamma += 1;
         sl.s.f = f;
@@ -1173,13 +1203,7 @@ __device__ void after_trial(S &sl, const ClosureParams &P, const Outputs &O, int
                             double fquad)
 {
     const int nm = P.nm;
-    double fnew = 0.0;
-    if (lane == 0) {
-        fnew = fquad;
-        for (int i = 0; i < nm; ++i)
-            fnew = __dsub_rn(fnew, __dmul_rn(sl.alpha[i], sl.u[i]));
-    }
-    fnew = cell_shfl<S>(fnew, 0);
+    const double fnew = serial_dot<true>(sl, fquad, sl.alpha, sl.u, nm, lane);
     double t = sl.s.t;
     bool accept = fnew <= __dadd_rn(sl.s.f, __dmul_rn(__dmul_rn(1e-3, t), sl.s.gd));
     cell_sync<S>();

@@ -987,8 +987,8 @@ __device__ __forceinline__ bool trial_fused(const ClosureParams &P, int fp64, in
 }
 
 // Hessian and trial pass over the listed cells (the FP64 list): the nm2 extended moments of
-// cells that need them into momBuf (stride 8 NT2), followed by a lower bound of e^{alpha.m} (the
-// smallest high word), and f's sum of trial cells into their state.
+// cells that need them into momBuf (stride 8 NT2), followed by bounds of e^{alpha.m} (the extreme
+// high words, rounded outwards), and f's sum of trial cells into their state.
 template <int NT, int NT2>
 __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
     sym_pass_kernel(ClosureParams P, SymTables T, const int *__restrict__ list, int n,
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
     for (int t = 0; t < E::TILES; ++t)
         acc[t][0] = acc[t][1] = 0.0;
     double f = 0.0;
-    int lo = 0x7fffffff;
+    int lo = 0x7fffffff, hi = 0;
     __syncthreads();
     for (int b = 0; b < T.nb; ++b) {
         const double *st = stage + (b % SYM_STAGES) * G::DOUBLES;
@@ -1048,8 +1048,9 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
                     const double ez = exp(v[e][s]);
-                    // (directions past the last have exponent 0: they only lower the bound)
+                    // (directions past the last have exponent 0: they only widen the bounds)
                     lo = min(lo, __double2hiint(ez));
+                    hi = max(hi, __double2hiint(ez));
                     v[e][s] = (e == 0 ? w.x : w.y) * ez;
                 }
                 sym_wht(v[e]);
@@ -1066,13 +1067,18 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
         if (tid == 0 && b + SYM_STAGES < T.nb)
             sym_stage_load<DEG, PD>(T, b + SYM_STAGES, stage, full);
     }
-    lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, 1));
-    lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, 2));
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, o));
+        hi = max(hi, __shfl_xor_sync(FULL_MASK, hi, o));
+    }
     if (wantH) {
         double *o = momBuf + (size_t)pos * (8 * NT2);
-        static_assert((PD + 1) * (PD + 1) < 8 * NT2, "room for the bound");
-        if ((lane & 3) == 0)
+        static_assert((PD + 1) * (PD + 1) + 2 <= 8 * NT2, "room for the bounds");
+        if ((lane & 3) == 0) {
             o[(PD + 1) * (PD + 1)] = __hiloint2double(lo, 0);
+            o[(PD + 1) * (PD + 1) + 1] = __hiloint2double(hi, -1);
+        }
 #pragma unroll
         for (int t = 0; t < E::TILES; ++t)
 #pragma unroll
@@ -1402,11 +1408,15 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
                 after_hessian(sl, P, O, lane, m0, e, e[NMP]);
             }
         } else {
-            double emin = 0.0;
+            double emin = 0.0, emax = 0.0;
             if constexpr (GAUNT)
-                if (fused) // the symmetric pass left its bound behind the moments
-                    emin = buf[(size_t)pos * BSTR + (2 * sym_order(NT2) + 1) * (2 * sym_order(NT2) + 1)];
-            after_hessian(sl, P, O, lane, m0, nullptr, 0.0, emin);
+                if (fused) { // the symmetric pass left its bounds behind the moments
+                    const double *e = buf + (size_t)pos * BSTR +
+                                      (2 * sym_order(NT2) + 1) * (2 * sym_order(NT2) + 1);
+                    emin = e[0];
+                    emax = e[1];
+                }
+            after_hessian(sl, P, O, lane, m0, nullptr, 0.0, emin, emax);
         }
         C3D_NCLK(O.stats, 5, lane);
     } else if (sl.s.need == NEED_TRIAL) {
