@@ -1018,8 +1018,11 @@ static c3d_status build_certificate(c3d_ctx *c, int nm2, const double *M2,
     const int nm = c->g.nm, nq = c->nq;
     int g0n = 1;
     bool valid = true;
+    bool diagonal = true; // H_i0 = m_0 mom_i, as the harmonics' own tables give it
     for (int i = 0; i < nm; ++i) {
         g0n = std::max(g0n, rowPtr[i + 1] - rowPtr[i]);
+        diagonal = diagonal && rowPtr[i + 1] - rowPtr[i] == 1 && colInd[rowPtr[i]] == i &&
+                   std::fabs(val[rowPtr[i]] - c->m0) <= 1e-12 * std::fabs(c->m0);
         for (int k = rowPtr[i]; k < rowPtr[i + 1]; ++k)
             valid = valid && colInd[k] >= 0 && colInd[k] < nm;
     }
@@ -1054,6 +1057,8 @@ static c3d_status build_certificate(c3d_ctx *c, int nm2, const double *M2,
     c->g0 = d;
     c->g0n = g0n;
     c->g0Valid = valid;
+    if (!diagonal) // the symmetric probe decides the certificate from its own moments
+        c->symN = c->sym2 = SymTables{};
     c->cp.gramLo = lo;
     c->cp.gramHi = hi;
     return C3D_OK;

@@ -534,6 +534,10 @@ struct FirstRound {
     // face ghosts' (gnx, gny, gnz: the interior sizes that tell them)
     const int *psiValid;
     int gnx, gny, gnz;
+    // symmetric quadrature: the probe pass finishes certified cells itself and lists the others'
+    // positions here for the Newton kernel (null: every cell)
+    int *todo;
+    unsigned int *todoCount;
 };
 [[maybe_unused]] constexpr int PSTR = 17; // row stride (cells) of the probe's psi tile
 [[maybe_unused]] constexpr int PRS = 3;   // stages of the mixed probe's psi read ring (chunks k .. k + 2)
@@ -947,6 +951,7 @@ __global__ void __launch_bounds__(RW * 32, KIND == 1 ? 1 : KIND == 2 ? 3 : 2)
 constexpr int SYM_STAGES = 3;
 [[maybe_unused]] constexpr int SYM_PASS_WARPS = 4;
 [[maybe_unused]] constexpr int SYM_PROBE_WARPS = 8;
+[[maybe_unused]] constexpr unsigned PROBE_GRID = 148 * 16; // CTAs that walk a probe's list
 
 // Degree of the basis of rounds_t<NT, NT2, true>.
 __host__ __device__ constexpr int sym_order(int nt2)
@@ -1097,12 +1102,15 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
 // Probe pass of a closure's first round (FirstRound; see rounds_pass_mixed_kernel for the
 // hand-off's psi and the certificate's entry): first-order moments, f's sum and bounds of
 // e^{alpha.m} per cell. It always forms e^{alpha.m}: reading psi / u_0 back instead was no faster
-// (11.9 against 10.8 ms per M_6 128^3 closure). e_min and e_max come from the high words of the values (rounded outwards by 2^-20: the
+// (11.9 against 10.8 ms per M_6 128^3 closure). A lane holds the gradient of a quarter of its
+// cell's moments at the end, so the certificate is decided here (as after_probe decides it)
+// and a certified cell finished -- no probe entry, no Newton visit (3.2 of 13.6 ms per closure
+// there); the rest is listed for the Newton kernel. e_min and e_max come from the high words of the values (rounded outwards by 2^-20: the
 // certificate keeps factors of 2 and 4 in hand).
 template <int NT, int NT2>
 __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
     sym_probe_kernel(ClosureParams P, SymTables T, int n, double *__restrict__ out, int *errorFlag,
-                     FirstRound first)
+                     Outputs O, FirstRound first)
 {
     constexpr int WARPS = SYM_PROBE_WARPS, DEG = sym_order(NT2), NMP = 8 * NT;
     using C = SymCls<DEG>;
@@ -1140,6 +1148,10 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
         }
     }
     const bool any = __any_sync(FULL_MASK, gc >= 0);
+    // the moments are read at the end: their lines come to L2 meanwhile
+    if (gc >= 0)
+        for (int i = 16 * (lane & 3); i < nm; i += 64)
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(first.u + gc * nm + i));
 #pragma unroll
     for (int k = 0; k < C::STEPS; ++k) {
         const int m = T.stepIdx[4 * k + (lane & 3)];
@@ -1204,21 +1216,96 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
         lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, o));
         hi = max(hi, __shfl_xor_sync(FULL_MASK, hi, o));
     }
-    if (gc < 0)
-        return;
-    double *o = out + (size_t)pos * probe_entry_doubles(NMP);
+    // gradient of the scaled cell (H_i0 / m_0 - u_i = <m_i e^{alpha.m}> - u_i) and its stopping test
+    __shared__ unsigned int sCertified;
+    if (tid == 0)
+        sCertified = 0;
+    __syncthreads();
+    double g2 = 0.0, u2 = 0.0, us[C::TILES][2];
+    const double inv = 1.0 / u0;
 #pragma unroll
     for (int t = 0; t < C::TILES; ++t)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int m = T.idx[8 * t + 2 * (lane & 3) + e];
-            if (m >= 0)
-                o[m] = acc[t][e];
+            us[t][e] = gc >= 0 && m >= 0 ? first.u[gc * nm + m] : 0.0;
         }
-    if ((lane & 3) == 0) {
-        o[NMP] = f;
-        o[NMP + 1] = __hiloint2double(lo, 0);
-        o[NMP + 2] = __hiloint2double(hi, -1);
+#pragma unroll
+    for (int t = 0; t < C::TILES; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            // (padding: 0 - 0, its projection fragments are 0)
+            const double ui = us[t][e] * inv, gi = acc[t][e] - ui;
+            g2 = fma(gi, gi, g2);
+            u2 = fma(ui, ui, u2);
+        }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        g2 += __shfl_xor_sync(FULL_MASK, g2, o);
+        u2 += __shfl_xor_sync(FULL_MASK, u2, o);
+    }
+    const double err = sqrt(g2), emin = __hiloint2double(lo, 0), emax = __hiloint2double(hi, -1);
+    const double rtol = P.batched ? P.tol : sqrt(u2) * P.tol;
+    const int maxIter = P.batched && P.nreg == 1 ? 10 * P.maxIter : P.maxIter;
+    const double lam = 0.5 * emin * P.gramLo, k1 = nm * (emax * P.gramHi) / lam;
+    const double minf = sqrt((2 * (DEG + 2) + 1) / (2 * M_PI));
+    const double gexp = 2.0 * minf * (DEG + 1) * err / lam;
+    const bool done = gc >= 0 && u0 > 0.0 && err <= rtol && maxIter > 1 && P.passBudget >= 1 &&
+                      P.tolGamma > 1.0 && emin > 0.0 && emax < 1.0 / 0.0 && P.gramLo > 0.0 &&
+                      k1 <= 0.25 * P.condHMax && gexp <= 0.5 * log(P.tolGamma);
+    // one list position per cell that goes on, claimed per warp
+    const unsigned goes = __ballot_sync(FULL_MASK, gc >= 0 && !done && (lane & 3) == 0);
+    unsigned at = 0;
+    if (lane == 0 && goes)
+        at = atomicAdd(first.todoCount, (unsigned)__popc(goes));
+    at = __shfl_sync(FULL_MASK, at, 0) + __popc(goes & ((1u << lane) - 1u));
+    if (done) {
+        // finalize (closure_core.cuh) of a cell converged in its first iteration
+#pragma unroll
+        for (int t = 0; t < C::TILES; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int m = T.idx[8 * t + 2 * (lane & 3) + e];
+                if (m >= 0)
+                    O.u[gc * nm + m] = us[t][e] / u0 * u0;
+            }
+        if ((lane & 3) == 0) {
+            O.alpha[gc * nm] = first.alpha[gc * nm] - ascale + ascale;
+            if (O.iters) O.iters[gc] = 1;
+            if (O.iterGamma) O.iterGamma[gc] = 0;
+            if (O.regIdx) O.regIdx[gc] = 0;
+            if (O.status) O.status[gc] = CELL_OK;
+            if (O.gamma) O.gamma[gc] = exp(gexp);
+            if (O.normG) O.normG[gc] = err;
+            if (O.cond) O.cond[gc] = (float)k1;
+            atomicAdd(&sCertified, 1u);
+        }
+    } else if (gc >= 0) {
+        double *o = out + (size_t)pos * probe_entry_doubles(NMP);
+#pragma unroll
+        for (int t = 0; t < C::TILES; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int m = T.idx[8 * t + 2 * (lane & 3) + e];
+                if (m >= 0)
+                    o[m] = acc[t][e];
+            }
+        if ((lane & 3) == 0) {
+            o[NMP] = f;
+            o[NMP + 1] = emin;
+            o[NMP + 2] = emax;
+            first.todo[at] = pos;
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && O.stats && sCertified) {
+        const unsigned long long c = sCertified;
+        atomicAdd(&O.stats[STAT_CELLS], c);
+        atomicAdd(&O.stats[STAT_ITERS], c);
+        atomicMax(&O.stats[STAT_MAX_ITER], 1ull);
+        atomicAdd(&O.stats[STAT_REG_HIST], c);
+        atomicAdd(&O.stats[STAT_ITER_HIST + 1], c);
+        atomicAdd(&O.stats[STAT_CERTIFIED], c);
     }
 }
 
@@ -1244,7 +1331,7 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
                          int g0n, FirstRound first, bool fused)
 {
     constexpr int W = cell_lanes(NT), CELLS = newton_cells(NT);
-    n = round_entries(n, nDev);
+    n = round_entries(n, MODE == 2 && first.todo ? first.todoCount : nDev);
     if (blockIdx.x * CELLS >= n)
         return;
     constexpr bool MIX = MODE == 1;
@@ -1267,8 +1354,11 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
     Outputs O = Og;
     if (Og.stats)
         O.stats = sStat;
-    const int pos = blockIdx.x * CELLS + ci;
-    const bool active = pos < n;
+    // (a probe's list is walked by a grid smaller than the worst case)
+    int blk = blockIdx.x;
+    do {
+    const bool active = blk * CELLS + ci < n;
+    const int pos = MODE == 2 && active && first.todo ? first.todo[blk * CELLS + ci] : blk * CELLS + ci;
     const long long cell = active ? (list ? list[pos] : first.off + pos) : -1;
     bool needH = MODE != 2 && active && state[cell].s.need == NEED_H;
     SlotT &sl = slots[ci];
@@ -1436,6 +1526,7 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
     C3D_NCLK(O.stats, 6, lane);
     }
     __syncthreads();
+    } while (MODE == 2 && (blk += gridDim.x) * CELLS < n);
     if (Og.stats)
         for (int q = tid; q < STAT_COUNT; q += NEWTON_THREADS) {
             const unsigned long long v = sStat[q];
@@ -1710,7 +1801,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
     const size_t probeSmem = newton_cells(NT) * sizeof(ProbeSlot<NT>);
     size_t passSmem, mixSmem[3] = {0, 0, 0};
     // octant-symmetric quadrature: the passes of sym.cuh
-    const bool sym = GAUNT && R.symN.no > 0;
+    const bool sym = GAUNT && P.sym;
     constexpr int DEG = sym_order(NT2);
     constexpr size_t symPassSmem = sym_smem<DEG, 2 * DEG, SYM_PASS_WARPS>(),
                      symProbeSmem = sym_smem<DEG, DEG, SYM_PROBE_WARPS>();
@@ -1854,7 +1945,8 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
 
     // round 0: set-up of every cell (with the certificate: set-up and probe pass in one round)
     auto round0 = [&](cudaStream_t s) -> cudaError_t {
-        cudaError_t e0 = cudaMemsetAsync(A.count[0], 0, NLISTS * sizeof(unsigned int), s);
+        // the lists' counters, the round counter and the probe's list
+        cudaError_t e0 = cudaMemsetAsync(R.counts, 0, (2 * NLISTS + 2) * sizeof(unsigned int), s);
         if (e0 != cudaSuccess)
             return e0;
         if (probe) {
@@ -1863,13 +1955,16 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                     const int nb = (int)((R.ncells - off) < R.batch ? (R.ncells - off) : R.batch);
                     const FirstRound fr{off,       R.cellMap,      R.u,      R.alpha,
                                         R.psi,     R.psiNall,      R.mark,
-                                        R.psiValid, R.gnx,         R.gny,    R.gnz};
+                                        R.psiValid, R.gnx,         R.gny,    R.gnz,
+                                        sym ? B.list[3] : nullptr, sym ? R.counts + 2 * NLISTS + 1 : nullptr};
                     const unsigned grid = (unsigned)((nb + MXC - 1) / MXC);
                     constexpr int per = 8 * SYM_PROBE_WARPS;
                     const unsigned gridS = (unsigned)((nb + per - 1) / per);
+                    if (sym && off > 0 && (e0 = cudaMemsetAsync(fr.todoCount, 0, sizeof(unsigned int), s)) != cudaSuccess)
+                        return e0;
                     if (sym)
                         sym_probe_kernel<NT, NT2><<<gridS, SYM_PROBE_WARPS * 32, symProbeSmem, s>>>(
-                            P, R.symN, nb, R.buf, R.errorFlag, fr);
+                            P, R.symN, nb, R.buf, R.errorFlag, O, fr);
                     else if (mixed)
                         rounds_pass_mixed_kernel<NT, NT2, 2, true><<<grid, RW * 32, mixSmem[2], s>>>(
                             P, R.mixF64, nullptr, nullptr, nb, nullptr, state, R.buf, R.errorFlag,
@@ -1878,8 +1973,9 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                         rounds_pass_mixed_kernel<NT, NT2, 2, false><<<grid, RW * 32, mixSmem[2], s>>>(
                             P, R.mixF64, nullptr, nullptr, nb, nullptr, state, R.buf, R.errorFlag,
                             fr);
+                    const unsigned gridN = (unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT));
                     rounds_newton_kernel<NT, NT2, GAUNT, 2>
-                        <<<(unsigned)((nb + newton_cells(NT) - 1) / newton_cells(NT)), NEWTON_THREADS, probeSmem, s>>>(
+                        <<<sym && gridN > PROBE_GRID ? PROBE_GRID : gridN, NEWTON_THREADS, probeSmem, s>>>(
                             P, m0, nullptr, nb, nullptr, state, R.buf, R.gstream, R.streamLen, O,
                             A, 3, mixed ? nullptr : R.g0, R.g0n, fr, false);
                     *R.launches += 2;
@@ -1908,8 +2004,6 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
                 if ((usedLists >> l) & 1u)
                     ec = cudaGraphConditionalHandleCreate(&th[hr].h[l], top, NTIER,
                                                           cudaGraphCondAssignDefault);
-        if (ec == cudaSuccess)
-            ec = cudaMemsetAsync(R.counts + 2 * NLISTS, 0, sizeof(unsigned int), cs[0]);
         const long long launches0 = *R.launches;
         if (ec == cudaSuccess)
             ec = round0(cs[0]);
