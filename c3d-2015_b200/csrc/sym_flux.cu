@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
     constexpr int TAB = C::TILES * 32 + 16; // a group's fragments and weights
     extern __shared__ __align__(128) double smem[]; // 8 x SLOT, 2 x TAB
     double *sTab = smem + 8 * F::SLOT;
-    __shared__ uint64_t full[4], empty[4]; // per pair of slots (the x flips)
+    __shared__ uint64_t full[8], empty[8];
     const int nm = g.nm, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long nall = g.nall();
     // tiles in blocks of 4 x 4 along x and y with z inside, so that CTAs running together read
@@ -199,9 +199,9 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
         k0 = 2 + (r % ntz) * F::TZ;
     }
     if (tid == 0) {
-        for (int p = 0; p < 4; ++p) {
-            bar_init(&full[p], F::COPIERS);
-            bar_init(&empty[p], F::WARPS);
+        for (int s = 0; s < 8; ++s) {
+            bar_init(&full[s], F::COPIERS);
+            bar_init(&empty[s], F::WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
             bool ok = true;
             sym_for<8>([&](auto ss) {
                 constexpr int s = ss.value;
-                if (s % 2 == 0 && gi > 0 && !bar_wait(&empty[s / 2], (gi - 1) & 1))
+                if (gi > 0 && !bar_wait(&empty[s], (gi - 1) & 1))
                     ok = false;
                 const double *rows = psi + (long long)(8 * gi + s) * nall * 4;
 #pragma unroll
@@ -264,8 +264,7 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
                 if (s == 0)
                     for (int e = ct; e < TAB / 2; e += F::COPIERS)
                         copy16(saddr(sTab + (gi & 1) * TAB + 2 * e), tab + (size_t)(g0 + gi) * TAB + 2 * e);
-                if (s % 2)
-                    copy_arrive(&full[s / 2]);
+                copy_arrive(&full[s]);
             });
             if (!ok) {
                 atomicExch(errorFlag, 1);
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
         const double *tb = sTab + (gi & 1) * TAB;
         sym_for<8>([&](auto ss) {
             constexpr int s = ss.value, dz = (s & 4) ? -F::PZ : F::PZ;
-            if (s % 2 == 0 && !bar_wait(&full[s / 2], gi & 1))
+            if (!bar_wait(&full[s], gi & 1))
                 ok = false;
             if (s == 0) {
                 cx = tb[C::TILES * 32 + d];
@@ -314,11 +313,9 @@ __global__ void __launch_bounds__(FluxTile<TX>::THREADS, TX == 4 ? 1 : 2)
             const double fy = sym_axis(th2, q[-2 * F::PY], q[-F::PY], v0, q[F::PY]);
             const double fz = sym_axis(th2, q[-2 * dz], q[-dz], v0, q[dz]);
             S[s] = fma(fx, cx, fma(fy, cy, fz * cz));
-            if (s % 2) {
-                __syncwarp();
-                if (lane == 0)
-                    bar_arrive(&empty[s / 2]);
-            }
+            __syncwarp();
+            if (lane == 0)
+                bar_arrive(&empty[s]);
         });
         sym_wht(S);
         sym_contract<DEG>(S, tb, lane, acc);
