@@ -309,35 +309,44 @@ static void free_ctx(c3d_ctx *c)
     delete c;
 }
 
-// Uploads the tables of a symmetric quadrature into one allocation, *buf (null: a failed
-// allocation; the previous one is freed).
-static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **buf)
+// Uploads the tables of a symmetric quadrature (and of another basis over it) into one
+// allocation, *buf (null: a failed allocation; the previous one is freed).
+static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **buf,
+                       const SymHost *H2 = nullptr, SymTables *T2 = nullptr)
 {
     if (*buf)
         cudaFree(*buf);
     *buf = nullptr;
-    T = SymTables{};
     std::vector<double> all;
-    auto add = [&](const void *src, size_t bytes) {
-        const size_t at = all.size(), n = (bytes + 127) / 128 * 16; // 128-byte aligned parts
-        all.resize(at + n);
-        if (bytes)
-            std::memcpy(all.data() + at, src, bytes);
-        return at;
-    };
-    const size_t e = add(H.expo.data(), H.expo.size() * 8), p = add(H.proj.data(), H.proj.size() * 8),
-                 w = add(H.w.data(), H.w.size() * 8), s = add(H.stepIdx.data(), H.stepIdx.size() * 4),
-                 i = add(H.idx.data(), H.idx.size() * 4), f = add(H.flux.data(), H.flux.size() * 8);
+    size_t at[2][6];
+    for (int k = 0; k < (H2 ? 2 : 1); ++k) {
+        const SymHost &S = k ? *H2 : H;
+        const void *src[6] = {S.expo.data(), S.proj.data(), S.w.data(),
+                              S.stepIdx.data(), S.idx.data(), S.flux.data()};
+        const size_t bytes[6] = {S.expo.size() * 8, S.proj.size() * 8, S.w.size() * 8,
+                                 S.stepIdx.size() * 4, S.idx.size() * 4, S.flux.size() * 8};
+        for (int i = 0; i < 6; ++i) {
+            at[k][i] = all.size();
+            all.resize(all.size() + (bytes[i] + 127) / 128 * 16); // 128-byte aligned parts
+            if (bytes[i])
+                std::memcpy(all.data() + at[k][i], src[i], bytes[i]);
+        }
+    }
     if (cudaMalloc(buf, all.size() * 8) != cudaSuccess) {
         cudaGetLastError();
         *buf = nullptr;
         return;
     }
     cudaMemcpy(*buf, all.data(), all.size() * 8, cudaMemcpyHostToDevice);
-    T = SymTables{H.no,     H.nb,     *buf + e, *buf + p,
-                  *buf + w, (const int *)(*buf + s), (const int *)(*buf + i)};
+    auto tables = [&](const SymHost &S, const size_t *a) {
+        return SymTables{S.no, S.nb, *buf + a[0], *buf + a[1], *buf + a[2],
+                         (const int *)(*buf + a[3]), (const int *)(*buf + a[4])};
+    };
+    T = tables(H, at[0]);
+    if (T2)
+        *T2 = tables(*H2, at[1]);
     if (flux)
-        *flux = *buf + f;
+        *flux = *buf + at[0][5];
 }
 
 // Rows of psi a direction chunk takes.
@@ -1214,12 +1223,9 @@ c3d_status c3d_set_gaunt(c3d_ctx *c, int nm2, const double *M2, const int *rowPt
     if (c->symPsi.no > 0 &&
         sym_build(c->deg, c->deg, nq, M1.data(), wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h1) &&
         sym_build(2 * c->deg, c->deg, nq, M2, wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h2)) {
-        sym_upload(h1, c->symN, nullptr, &c->symBuf[1]);
-        sym_upload(h2, c->sym2, nullptr, &c->symBuf[2]);
-        if (!c->symBuf[1] || !c->symBuf[2]) {
-            c->symN = c->sym2 = SymTables{};
+        sym_upload(h1, c->symN, nullptr, &c->symBuf[1], &h2, &c->sym2);
+        if (!c->symBuf[1])
             return fail(C3D_ERR_OOM, "c3d_set_gaunt: device allocation failed");
-        }
     }
     return build_certificate(c, nm2, M2, wh, rowPtr, colInd, val);
 }

@@ -1600,16 +1600,26 @@ template <int NT, int KIND, bool ZD> static size_t mixed_pass_smem(const Closure
 // A closure is one CUDA graph: round 0 (set-up, or the certificate's probe round) then a
 // conditional WHILE node whose body runs two rounds (lists A -> B, then B -> A) and sets the
 // loop condition on the device, so no round waits for the host. Within a round, each list's
-// pass and Newton kernels sit in a SWITCH node whose branch -- one of four launch sizes
+// pass and Newton kernels sit in a SWITCH node whose branch -- one of up to four launch sizes
 // (up to 512, 8192, 65536 and `cap` entries) or none for an empty list -- a control kernel
 // picks from the list's device counter; entries past `cap` are carried to the next round's
 // list. The kernels read their entry count from the counter (round_entries).
 
+// A list whose launches are all below a size has no branch above it (a graph's build takes
+// about 25 us per kernel node, most of a new state's first step: M_2 16^3, 8000 cells, has 2
+// branches per list), and the rare list of cells in the reference's order has 8192 and cap only.
 constexpr int NTIER = 4;
-__host__ __device__ inline long long tier_entries(int t, long long cap)
+__host__ __device__ inline long long tier_entries(int t, long long cap, bool rare)
 {
-    const long long t0 = t == 0 ? 512 : t == 1 ? 8192 : 65536;
+    const long long t0 = rare ? (t == 0 ? 8192 : cap) : t == 0 ? 512 : t == 1 ? 8192 : 65536;
     return t < 3 && t0 < cap ? t0 : cap;
+}
+__host__ __device__ inline int tier_count(long long cap, bool rare)
+{
+    int n = 1;
+    while (tier_entries(n - 1, cap, rare) < cap)
+        ++n;
+    return n;
 }
 
 struct TierHandles {
@@ -1618,9 +1628,10 @@ struct TierHandles {
 
 #if C3D_ROUNDS_PART != 0
 // Picks each used list's launch size (SWITCH branch; NTIER = none) from its counter (bit l of
-// mask marks list l as used) and clears the counters of the lists the round fills.
+// mask marks list l as used, of rare as a rare one) and clears the counters of the lists the
+// round fills.
 static __global__ void rounds_tier_kernel(const Lists in, Lists out, TierHandles th, unsigned int mask,
-                                   long long cap, unsigned long long *launches)
+                                   unsigned int rare, long long cap, unsigned long long *launches)
 {
     if (threadIdx.x != 0)
         return;
@@ -1631,12 +1642,14 @@ static __global__ void rounds_tier_kernel(const Lists in, Lists out, TierHandles
         if (!((mask >> l) & 1u))
             continue;
         const long long c = (long long)*in.count[l];
+        const bool ra = (rare >> l) & 1u;
+        const int last = tier_count(cap, ra) - 1;
         int t = NTIER;
-        for (int k = NTIER - 1; k >= 0; --k)
-            if (c > 0 && c <= tier_entries(k, cap))
+        for (int k = last; k >= 0; --k)
+            if (c > 0 && c <= tier_entries(k, cap, ra))
                 t = k;
         if (c > cap)
-            t = NTIER - 1;
+            t = last;
         cudaGraphSetConditional(th.h[l], (unsigned int)t);
         l2 += t < NTIER ? 2 : 0;
     }
@@ -1870,6 +1883,7 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
     // routes any visit to reduced precision, its BF16 and 3xTF32 ones (probe passes happen in
     // round 0 only: no later visit is a first visit)
     const unsigned int usedLists = 1u | (mixed && P.mixIterMax > 0 ? 6u : 0u) | (sym ? 8u : 0u);
+    const unsigned int rareLists = sym ? 8u : 0u;
 
     // pass + Newton kernels of list l: entries la[0 .. nb) (with nDev, at most *nDev of them),
     // the cells still in need appended to out
@@ -2018,18 +2032,21 @@ template <int NT, int NT2, bool GAUNT> cudaError_t rounds_t(const RoundsLaunch &
             return ec;
         for (int hr = 0; hr < 2 && ec == cudaSuccess; ++hr) {
             const Lists &X = hr == 0 ? A : B, &Y = hr == 0 ? B : A;
-            rounds_tier_kernel<<<1, 32, 0, cs[1]>>>(X, Y, th[hr], usedLists, cap, R.launchDev);
+            rounds_tier_kernel<<<1, 32, 0, cs[1]>>>(X, Y, th[hr], usedLists, rareLists, cap,
+                                                  R.launchDev);
             ec = cudaGetLastError();
             for (int l = 0; l < NLISTS && ec == cudaSuccess; ++l) {
                 if (!((usedLists >> l) & 1u))
                     continue;
+                const bool rare = (rareLists >> l) & 1u;
+                const int nt = tier_count(cap, rare);
                 cudaGraph_t *tiers = nullptr;
-                ec = capture_conditional(cs[1], th[hr].h[l], cudaGraphCondTypeSwitch, NTIER, &tiers);
-                for (int t = 0; t < NTIER && ec == cudaSuccess; ++t) {
+                ec = capture_conditional(cs[1], th[hr].h[l], cudaGraphCondTypeSwitch, nt, &tiers);
+                for (int t = 0; t < nt && ec == cudaSuccess; ++t) {
                     ec = cudaStreamBeginCaptureToGraph(cs[2], tiers[t], nullptr, nullptr, 0,
                                                        cudaStreamCaptureModeRelaxed);
                     if (ec == cudaSuccess) {
-                        cudaError_t el = launch_list(l, X.list[l], (int)tier_entries(t, cap),
+                        cudaError_t el = launch_list(l, X.list[l], (int)tier_entries(t, cap, rare),
                                                      X.count[l], Y, cs[2]);
                         cudaGraph_t body = nullptr;
                         ec = cudaStreamEndCapture(cs[2], &body);
