@@ -4,6 +4,7 @@
 // condition estimate and substitutions, and the per-cell Newton state machine of
 // src/opt/optBatch.cpp:143-344 / src/opt/opt.cpp:139-355 (see closure_fp64.cu).
 #pragma once
+#include <type_traits>
 #include "c3d_common.cuh"
 
 #include <cfloat>
@@ -101,19 +102,27 @@ template <int NT, bool TILED = false> struct alignas(16) Slot {
     static constexpr int LSIZE = TILED ? 64 * NTILES : Cfg<NT>::NPK;
     static constexpr bool tiled = TILED;
     static constexpr int nt = NT;
+    // alpha0 and uOrig are read by a new regularisation level only. Small orders (several cells
+    // per warp) leave them in the cell's global state: two of the six vectors a visit would
+    // load and store, and for N = 4 a fourth CTA per SM (54.7 KB each; Newton kernel of M_4
+    // 64^3 9.75 -> 7.98 ms, of M_3 visits 2.5% faster). From N = 5 on neither limits, and the slot
+    // keeps them (visits were 2% slower without).
+    static constexpr bool KEEP = !TILED || W == 32;
+    using Kept = typename std::conditional<KEEP, double[NMP], double *>::type;
     // A tiled slot is 48 bytes more than a multiple of 128: the assembly of H gathers moments at
-    // 32-byte places of four slots, and a multiple of 32 left it half the banks (shared data pipe
-    // 75% busy; Newton kernel of M_4 64^3 9.89 -> 9.76 ms, of M_5 visits 4% faster).
-    static constexpr int PAD = TILED ? 2 : 0;
-    double u[NMP], alpha[NMP], alpha0[NMP], uOrig[NMP], g[NMP], d[NMP], alphaOld[NMP], rinv[NMP];
+    // 32-byte places of four slots, and a multiple of 32 left it half the banks, with the shared
+    // data pipe 75% busy (M_5 visits 4% faster).
+    static constexpr int PAD = TILED && KEEP ? 2 : 0;
+    double u[NMP], alpha[NMP], g[NMP], d[NMP], alphaOld[NMP], rinv[NMP];
     double L[LSIZE + PAD];
+    Kept alpha0, uOrig;
     SlotScalars s;
     // g, d, alphaOld and rinv as one array of 4 NMP doubles (scratch between Hessian visits),
     // addressed through the slot object so that it may span the four vectors
     __device__ __forceinline__ double *scratch()
     {
         return reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(this) +
-                                          4 * NMP * sizeof(double));
+                                          2 * NMP * sizeof(double));
     }
     // offset of element (i, j), i >= j
     __device__ static __forceinline__ int lx(int i, int j)

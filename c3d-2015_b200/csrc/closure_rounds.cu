@@ -49,16 +49,27 @@ __device__ __forceinline__ void copy_scalars(SlotScalars &dst, const SlotScalars
             reinterpret_cast<const unsigned long long *>(&src)[i];
 }
 
+// Whether a slot leaves alpha0 and uOrig in the cell's state.
+template <class S> constexpr bool keeps_in_state = std::is_pointer<decltype(S::alpha0)>::value;
+
 // lineSearch = false skips d and alphaOld, which a Hessian visit recomputes before use.
 template <int NT, class S>
-__device__ void state_to_slot(const CellState<NT> &st, S &sl, int lane, bool lineSearch = true)
+__device__ void state_to_slot(CellState<NT> &st, S &sl, int lane, bool lineSearch = true)
 {
     constexpr int NMP = Cfg<NT>::NMP;
+    if constexpr (keeps_in_state<S>) {
+        if (lane == 0) {
+            sl.alpha0 = st.alpha0;
+            sl.uOrig = st.uOrig;
+        }
+    }
     for (int i = lane; i < NMP; i += S::W) {
         sl.u[i] = st.u[i];
         sl.alpha[i] = st.alpha[i];
-        sl.alpha0[i] = st.alpha0[i];
-        sl.uOrig[i] = st.uOrig[i];
+        if constexpr (!keeps_in_state<S>) {
+            sl.alpha0[i] = st.alpha0[i];
+            sl.uOrig[i] = st.uOrig[i];
+        }
         if (lineSearch) {
             sl.d[i] = st.d[i];
             sl.alphaOld[i] = st.alphaOld[i];
@@ -76,8 +87,10 @@ __device__ void slot_to_state(const S &sl, CellState<NT> &st, int lane)
     for (int i = lane; i < NMP; i += S::W) {
         st.u[i] = sl.u[i];
         st.alpha[i] = sl.alpha[i];
-        st.alpha0[i] = sl.alpha0[i];
-        st.uOrig[i] = sl.uOrig[i];
+        if constexpr (!keeps_in_state<S>) {
+            st.alpha0[i] = sl.alpha0[i];
+            st.uOrig[i] = sl.uOrig[i];
+        }
         st.d[i] = sl.d[i];
         st.alphaOld[i] = sl.alphaOld[i];
     }
