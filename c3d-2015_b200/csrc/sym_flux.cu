@@ -106,7 +106,10 @@ __global__ void __launch_bounds__(128)
 
 // Slope of the limited reconstruction at a value with differences dm (to its upwind neighbour),
 // dp (to its downwind one) and dc across both, times 4: minmod(th dp, dc / 2, th dm)
-// (src/flux_kinetic.cpp:45-61) scaled by 2, th2 = 2 th >= 0, for dm and dp of one sign (dc then has it too, and min(th |dm|, th |dp|) = th min(|dm|, |dp|)); otherwise it is 0.
+// (src/flux_kinetic.cpp:45-61) scaled by 2, th2 = 2 th >= 0, for dm and dp of one sign (dc then
+// has it too, and min(th |dm|, th |dp|) = th min(|dm|, |dp|)); otherwise it is 0. (The selects as
+// predicated FP64 operations: 24 instructions fewer per cell and direction, 7% slower, since 12
+// more go to the FP64 pipe.)
 __device__ __forceinline__ double sym_slope(double th2, double dm, double dp, double dc)
 {
     const double m = th2 * (fabs(dm) < fabs(dp) ? dm : dp);
@@ -161,8 +164,12 @@ template <int TX> struct FluxTile {
 // fragments straight from registers. A reflection's stage has its own ring slot, filled by
 // copy warps that run up to 8 stages ahead; warps drift against each other inside the ring (full
 // and empty barriers, no CTA barrier).
-// Issue bound: about 100 instructions per cell and direction, half of them FP64.
-// (Bulk copies, one per line of cells, took 76 clocks each: 2.6 times slower as a whole.)
+// Bound by the FP64 pipe's latency and issue: 137 warp instructions per 32 (cell, direction)
+// pairs, 44 of them FP64; 0.6 instructions per clock and scheduler, FP64 pipe 39%, ALU 51%, DRAM
+// 30%. M_6 64^3: 2.61 ms per call, 128^3: 20.6 ms (5.2 and 40.2 ms with all directions as one run
+// each and no symmetry); M_4 64^3 1.31 ms, M_3 37 x 45 x 51 0.31 ms.
+// (Bulk copies, one per line of cells, took 76 clocks each: 2.6 times slower as a whole. One
+// barrier per pair of reflections spilled: N <= 5 1 to 6% slower, N = 6 1% faster.)
 // wrapFlag (null: no): when it reads 0 the face ghosts' psi is not in place; their values are
 // read at the periodic images.
 template <int DEG, int TX>
@@ -397,8 +404,16 @@ static cudaError_t flux_t(const GridDims &g, const double *psi, const double *ta
                           int r0, int r1, double th2, double *flux, int *errorFlag,
                           const int *wrapFlag, int numSMs, cudaStream_t st)
 {
+    // Tiles of 4 x planes: one CTA of 640 threads per SM, so whole waves of numSMs tiles. Tiles of
+    // 2: two CTAs per SM, more halo (5 / 2 of psi against 7 / 4), measured in waves of the former
+    // as 0.75 for up to a tile per SM, then 0.54 per tile and SM and a tail of 0.3, 1.06 at least.
+    // M_6, 20 x 20 directions, 4 against 2 planes: 16^3 98 and 73 us, 24^3 99 and 106, 28^3 197
+    // and 172, 32^3 198 and 210, 40^3 389 and 370, 64^3 1358 and 1443 (M_2, M_4 in proportion).
     const long long lines = (long long)((g.ny + 3) / 4) * ((g.nz + 7) / 8);
-    return lines * ((g.nx + 3) / 4) >= 2 * numSMs
+    const double x = (double)(lines * ((g.nx + 1) / 2)) / numSMs;
+    const double two = x <= 1.0 ? 0.75 : fmax(1.06, 0.54 * x + 0.3);
+    const long long four = (lines * ((g.nx + 3) / 4) + numSMs - 1) / numSMs;
+    return four <= two
                ? flux_v<DEG, 4>(g, psi, tab, idx, r0, r1, th2, flux, errorFlag, wrapFlag, st)
                : flux_v<DEG, 2>(g, psi, tab, idx, r0, r1, th2, flux, errorFlag, wrapFlag, st);
 }

@@ -65,6 +65,14 @@ def test_flux_matches_general_kernels(N, Q, n, chunk, theta, pn):
     assert _rel(f[0], f[1]) < 1e-13
 
 
+@pytest.mark.parametrize("N,Q,n", [(0, 4, (20, 20, 24)), (2, 10, (18, 22, 26)), (4, 12, (35, 34, 36)),
+                                   (6, 14, (21, 24, 17)), (7, 16, (17, 19, 25))])
+def test_flux_on_wider_tiles(N, Q, n):
+    """Grids whose stencil takes tiles of 4 x planes (a wave of them or more on 148 SMs), their last
+    tiles ragged along x, y and z."""
+    test_flux_matches_general_kernels(N, Q, n, 0, 2.0, 0)
+
+
 @pytest.mark.parametrize("N,Q,n", [(1, 8, (8, 6, 5)), (2, 10, (12, 9, 8)), (3, 14, (10, 12, 11)),
                                    (4, 14, (8, 8, 16)), (5, 16, (9, 8, 10)), (6, 18, (8, 8, 8)),
                                    (7, 20, (6, 6, 6))])
