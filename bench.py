@@ -920,14 +920,14 @@ def b200_arm(args):
                   "tcgen05 beside it (lowp_tflops)" if precision == 1
                   else "fp64 (DMMA m8n8k4 + DFMA)"),
             achieved=achieved, peak=peak, unit="TFLOP/s", frac=achieved / peak if peak else None,
-            traffic=(profile_traffic("closure_rounds_m6_64")
+            traffic=(profile_traffic("sym_kernels_m6_64")
                      if args.engine == "rounds" and args.hessian == "gaunt" else None),
-            traffic_source="profiles/closure_rounds_m6_64.txt: one closure's DRAM bytes at 64^3 "
+            traffic_source="profiles/sym_kernels_m6_64.txt: the probe pass's DRAM bytes at 64^3 "
                            "(ncu) scaled by solved cells to 128^3",
             peak_source="in-run cuBLAS DGEMM 8192^3 via torch (FP64 is not in "
                         "MEASURED_PEAKS.json)",
-            kernel=(("closure work-list rounds: rounds_pass_mixed_kernel<7,22,2> (first-visit "
-                     "probe) + rounds_pass_gaunt_kernel<7,22> + rounds_newton_kernel"
+            kernel=(("closure work-list rounds: sym_probe_kernel<7,22> (first visits) + "
+                     "sym_pass_kernel<7,22> + rounds_newton_kernel"
                      if args.hessian == "gaunt" else
                      "closure work-list rounds: rounds_pass_direct_kernel<7> + "
                      "rounds_newton_kernel") if args.engine == "rounds" else
@@ -940,9 +940,9 @@ def b200_arm(args):
         if low is not None:
             closure_roofline["lowp_tflops"] = low / max(1, closure_launches) / per_launch_s / 1e12
             closure_roofline["kernel"] = (
-                "closure work-list rounds: rounds_pass_mixed_kernel<7,22,2> (first-visit probe), "
-                "<7,22,0|1> (tcgen05 Hessian moments), rounds_pass_gaunt_kernel<7,22> (trials, "
-                "FP64 Hessians) + rounds_newton_kernel")
+                "closure work-list rounds: sym_probe_kernel<7,22> (first visits), "
+                "rounds_pass_mixed_kernel<7,22,0|1> (tcgen05 Hessian moments), "
+                "sym_pass_kernel<7,22> (trials, FP64 Hessians) + rounds_newton_kernel")
         compare = None
         if other is not None:
             fp, mx = (other, head) if precision == 1 else (head, other)
@@ -971,7 +971,7 @@ def b200_arm(args):
                               f"{args.steps} timed steps from the same start state, mixed vs "
                               "the FP64 drop-in (all cells incl. ghosts); the FP64 drop-in "
                               "matches the C oracle to 1e-12 (tests)")
-        # the dominant kernel: the kinetic flux's stencil + projection (kinetic_staged_kernel),
+        # the dominant kernel: the kinetic flux's stencil + projection (sym_flux_kernel),
         # one launch per flux call when the closure handed its ansatz over (psi of all
         # directions within the 32 GiB budget). Algorithmic work per (cell, direction):
         # 2 nm FLOPs of projection + 60 of the three axes' limited upwind differences; bytes:
@@ -983,17 +983,17 @@ def b200_arm(args):
         stencil_flops = float((2 * nm + 60) * nq) * cells
         stencil_bytes = 8.0 * ((cells + face_ghosts) * nq + cells * nm)
         achieved_k = stencil_flops / (flux_ms * 1e-3) / 1e12
-        traffic_k = profile_traffic("kinetic_staged_m6_64", "dram_bytes_per_launch:")
+        traffic_k = profile_traffic("sym_kernels_m6_64", "dram_bytes_per_launch:")
         if traffic_k is not None:
             traffic_k *= cells / 64 ** 3  # ncu capture at 64^3, scaled by (cell, direction) pairs
         roofline = dict(
             bound="tensor", pipe="fp64 (DMMA m8n8k4 projection + DFMA/ALU limiter)",
-            kernel="kinetic_staged_kernel<7> (kinetic flux: MUSCL stencil + projection)",
+            kernel="sym_flux_kernel<6,4> (kinetic flux: MUSCL stencil + projection)",
             achieved=achieved_k, peak=peak, unit="TFLOP/s",
             frac=achieved_k / peak if peak else None,
             traffic=traffic_k,
-            traffic_source="profiles/kinetic_staged_m6_64.txt: dram__bytes_read.sum + "
-                           "dram__bytes_write.sum of one launch at 64^3 (ncu), scaled by "
+            traffic_source="profiles/sym_kernels_m6_64.txt: DRAM rate x time of one launch at "
+                           "64^3 (ncu), scaled by "
                            "(cell, direction) pairs to this grid",
             peak_source="in-run cuBLAS DGEMM 8192^3 via torch (FP64 is not in "
                         "MEASURED_PEAKS.json)",

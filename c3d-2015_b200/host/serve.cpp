@@ -33,9 +33,10 @@ long long footprint(const c3d_host::Config &c)
     const long long nmp = 8 * ((nm + 7) / 8);
     const long long nq = 2LL * c.quadOrder * c.quadOrder;
     const long long psiCap = (32LL << 30) / 8 / (nall > 0 ? nall : 1);
-    const long long psiDirs = nq < psiCap ? nq : psiCap;
+    const long long psiRows = (nq + 31) / 32 * 32; // whole groups of 4 octant directions
+    const long long psiDirs = psiRows < psiCap ? psiRows : psiCap;
     long long b = 4 * nall * nm * 8 + 2 * nall * 8 + 5 * nall * 4 + 2 * nall * 8;
-    b += psiDirs * nall * 8 + nall * 4;
+    b += psiDirs * nall * 8 + nall * 4; // the marks and groups of the hand-off: 2 bytes a cell
     if (c.solver == "mn") {
         const long long batch = nall < (1LL << 20) ? nall : (1LL << 20);
         const long long nm2 = (2LL * c.momentOrder + 1) * (2 * c.momentOrder + 1);

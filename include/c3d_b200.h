@@ -95,7 +95,8 @@ typedef struct {
     int nreg;                  /* regularisation ladder (reference: 5 values) */
     double reg[16];
     size_t psiBytes;           /* budget for the materialised ansatz (0 = default, 32 GiB);
-                                  the closure's ansatz hand-off needs nq * nall * 8 bytes */
+                                  the closure's ansatz hand-off needs nq * nall * 8 bytes, nq
+                                  rounded up to a multiple of 32 */
     int mnReproject;           /* 1: after each grid closure set u = <m e^{alpha.m}> with u_0
                                   kept (the robustness note of the reference's readme.txt);
                                   deck key MN_REPROJECT; no counterpart in the reference code */
@@ -225,7 +226,7 @@ c3d_status c3d_gaunt_build(int nm, int nm2, int nq, const double *M2, double thr
                            double *val, long long *nnz);
 
 /* Closure engine: 0 (default) runs rounds over a device work list -- a pass kernel for
- * the quadrature sums of every listed cell, then a Newton kernel with one warp per cell,
+ * the quadrature sums of every listed cell, then a Newton kernel with 8 to 32 lanes per cell,
  * re-listing cells that need another pass (the reference's Optimization::opt stacks,
  * src/opt/optBatch.cpp:350-472); 1 runs one persistent kernel whose warps pull cells
  * from a device counter. Both run the reference's per-cell algorithm; they differ in the
@@ -270,7 +271,8 @@ c3d_status c3d_set_certificate(c3d_ctx *ctx, int on);
  * and the balanced splits into up to 3 more chunks) and z run length per CTA of the staged
  * kernel (64, and 32 where nz is a multiple of 32), then keeps the fastest for later calls.
  * The flux buffer is overwritten; u and alpha are not touched. Outputs may be NULL
- * (runLen 0: min(64, nz)). */
+ * (runLen 0: min(64, nz); without effect on even tensor quadratures in their own order,
+ * whose stencil takes its tiles by the grid's size). */
 c3d_status c3d_autotune(c3d_ctx *ctx, int *qChunk, int *runLen, double *msPerCall);
 
 /* The work-list closure as one CUDA graph (engine 0; on by default; no counterpart in the
@@ -289,7 +291,7 @@ c3d_status c3d_set_graphs(c3d_ctx *ctx, int on);
 /* Ansatz hand-off from the closure to the kinetic flux (on by default; no counterpart in the
  * reference). A grid closure with the convergence certificate evaluates e^{alpha.m_q} of
  * every cell and direction in its probe pass; with this on, that pass also stores them as the
- * flux's ansatz psi (one buffer of nq * nall doubles, within the params' psiBytes budget),
+ * flux's ansatz psi (one buffer within the params' psiBytes budget, see there),
  * face ghosts copy their images' values and the few cells whose multipliers change after the
  * probe are recomputed at the end of the closure, and the next c3d_flux_kinetic runs the
  * limited stencil and projection alone instead of forming psi again. The flux equals the
@@ -305,7 +307,8 @@ c3d_status c3d_set_ansatz_handoff(c3d_ctx *ctx, int on);
  * 2^40), after which the cell ends with status 3 and c3d_sync reports C3D_ERR_CLOSURE, and at
  * most batch list entries per pass and Newton launch (default 2^20; the pass output buffer
  * holds that many; longer lists run in several launches, or carry over between the graph's
- * rounds). Values <= 0 restore the defaults. */
+ * rounds). An accepted line-search trial and the next Hessian share a round on even tensor
+ * quadratures. Values <= 0 restore the defaults. */
 c3d_status c3d_set_limits(c3d_ctx *ctx, long long maxRounds, long long passBudget,
                           long long batch);
 
