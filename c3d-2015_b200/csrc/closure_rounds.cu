@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(RW * 32, KIND == 1 ? 1 : KIND == 2 ? 3 : 2)
 
 constexpr int SYM_STAGES = 3;
 [[maybe_unused]] constexpr int SYM_PASS_WARPS = 4;
-[[maybe_unused]] constexpr int SYM_PROBE_WARPS = 8;
+[[maybe_unused]] constexpr int SYM_PROBE_WARPS = 4; // (8 and 2 CTAs per SM: 2 to 5% slower for N <= 6)
 [[maybe_unused]] constexpr unsigned PROBE_GRID = 148 * 16; // CTAs that walk a probe's list
 
 // Degree of the basis of rounds_t<NT, NT2, true>.
@@ -1006,7 +1006,10 @@ __device__ __forceinline__ bool trial_fused(const ClosureParams &P, int fp64, in
 
 // Hessian and trial pass over the listed cells (the FP64 list): the nm2 extended moments of
 // cells that need them into momBuf (stride 8 NT2), followed by bounds of e^{alpha.m} (the extreme
-// high words, rounded outwards), and f's sum of trial cells into their state.
+// high words, rounded outwards), and f's sum of trial cells into their state. FP64 pipe bound: 24
+// class tiles over nq / 8 directions for the 169 moments of M_6 against 22 over nq. M_4 64^3:
+// 2.7 ms per two steps (17.4 with all directions), M_5 visits 1.1 ns each. 8 warps per CTA: 1 to 15%
+// slower; one CTA more per SM (fewer registers) 3 to 30%.
 template <int NT, int NT2>
 __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
     sym_pass_kernel(ClosureParams P, SymTables T, const int *__restrict__ list, int n,
@@ -1118,10 +1121,12 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
 // (11.9 against 10.8 ms per M_6 128^3 closure). A lane holds the gradient of a quarter of its
 // cell's moments at the end, so the certificate is decided here (as after_probe decides it)
 // and a certified cell finished -- no probe entry, no Newton visit (3.2 of 13.6 ms per closure
-// there); the rest is listed for the Newton kernel. e_min and e_max come from the high words of the values (rounded outwards by 2^-20: the
-// certificate keeps factors of 2 and 4 in hand).
+// there); the rest is listed for the Newton kernel. e_min and e_max come from the high words of
+// the values (rounded outwards by 2^-20: the certificate keeps factors of 2 and 4 in hand).
+// Bound by the FP64 pipe (vector 39% + DMMA 28% busy) and the latency of its chains. M_6 64^3:
+// 1.44 ms per closure (6.8 with all directions), M_4 0.73.
 template <int NT, int NT2>
-__global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 2)
+__global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
     sym_probe_kernel(ClosureParams P, SymTables T, int n, double *__restrict__ out, int *errorFlag,
                      Outputs O, FirstRound first)
 {
