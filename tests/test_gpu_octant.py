@@ -149,3 +149,41 @@ def test_cells_at_the_realizability_boundary(N, Q, n):
     assert not res[0][2].any() and not res[1][2].any()
     assert _rel(res[0][0], res[1][0]) < 1e-6
     assert _rel(res[0][1], res[1][1]) < 1e-6
+
+
+@pytest.mark.parametrize("N", [3, 4, 5])
+def test_regularised_cells_match_persistent_engine(N):
+    """Cells far from isotropy under a condition limit of 200: isotropic restarts and several
+    ladder levels, which read a cell's start and original vectors again -- orders up to 4 from its
+    global state, N = 5 and the persistent engine from the slot. Both engines take the same
+    decisions (no ties at tolerance 1e-6: the condition estimates agree to 1e-12); rounding
+    amplified by condition numbers up to 200 over some ten iterations stays below 1e-9."""
+    n, Q = (9, 8, 7), 2 * (N + 3)
+    T = c3d.quadrature(N, Q, with_m2=True)
+    nm, nq = T["nm"], T["nq"]
+    _, row, col, val = c3d.gaunt_build(nm, T["nm2"], nq, T["M2"])
+    nall = (n[0] + 4) * (n[1] + 4) * (n[2] + 4)
+    M = T["M"].reshape(nq, nm)
+    rng = np.random.default_rng([11, N])
+    a = rng.standard_normal((nall, nm)) * rng.uniform(0.2, 1.5, (nall, 1))
+    a[:, 0] = 0.0
+    u = (np.exp(a @ M.T) * T["w"]) @ M
+    start = np.zeros_like(a)
+    start[:, 0] = 2 * np.sqrt(np.pi) * np.log(u[:, 0] / (2 * np.sqrt(np.pi)))
+    res = []
+    for engine in (0, 1):
+        x = c3d.Context(nx=n[0], ny=n[1], nz=n[2], nm=nm, nq=nq, dx=1.0, dy=1.0, dz=1.0, M=T["M"],
+                        w=T["w"], xi=T["xi"], eta=T["eta"], mu=T["mu"], tol=1e-6, cond_h_max=200.0,
+                        ladder=(0.0, 1e-2, 1e-1, 0.5, 0.9, 0.99))
+        x.set_gaunt(T["nm2"], T["M2"], row, col, val)
+        x.set_engine(engine)
+        x.set_state(u=u.ravel(), alpha=start.ravel(), sig_t=np.ones(nall), sig_s=np.ones(nall))
+        x.closure()
+        x.sync()
+        res.append(x.get_state() + (x.records(),))
+        x.close()
+    (u0, a0, r0), (u1, a1, r1) = res
+    assert len(set(r0["regIndex"])) >= 3 and (r0["regIndex"] > 0).sum() > 20
+    for k in ("iters", "regIndex", "status"):
+        assert np.array_equal(r0[k], r1[k]), k
+    assert _rel(u0, u1) < 1e-9 and _rel(a0, a1) < 1e-9
