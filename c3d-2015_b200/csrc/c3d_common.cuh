@@ -97,6 +97,14 @@ struct __align__(16) GauntTerm {
 // this many threads.
 constexpr int NEWTON_THREADS = 128;
 
+#ifdef __CUDACC__
+// Orders the thread's accesses of shared memory before bulk copies that a thread issues past the
+// next barrier of the CTA. Bulk copies write through the async proxy, which a barrier alone does
+// not order after reads: a load that a warp issued before the barrier may still be queued behind
+// other loads of the SM when the copy into its place lands.
+__device__ __forceinline__ void refill_fence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+#endif
+
 // Grid with two ghost layers per face; cell (i,j,k) with k fastest (src/global.h:15).
 struct GridDims {
     int nx, ny, nz; // interior cells

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(W * 32, 1)
                     }
                 }
             }
+            refill_fence();
             __syncthreads();
             if (tid == 0 && k + STAGES < nchunks) {
                 mbar_expect_tx(&full[s], chunkBytes);
@@ -316,6 +317,7 @@ __global__ void __launch_bounds__(W * 32, 1)
                     }
                 }
             }
+            refill_fence();
             __syncthreads();
             if (tid == 0 && k + GSTAGES < nchunks) {
                 mbar_expect_tx(&full[s], chunkBytes);
@@ -444,6 +446,7 @@ __global__ void __launch_bounds__(W * 32, 1)
                 for (int J = 0; J <= I; ++J)
                     dmma(acc[I * (I + 1) / 2 + J][0], acc[I * (I + 1) / 2 + J][1], a[I], m[J]);
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && k + STAGES < nchunks) {
             mbar_expect_tx(&full[s], chunkBytes);
@@ -550,6 +553,7 @@ __global__ void __launch_bounds__(256, 1)
                          ch[(nm + 8 * j + (lane >> 2)) * QCP + 4 * g + (lane & 3)]);
             }
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && k + GSTAGES < nchunks) {
             mbar_expect_tx(&full[s], chunkBytes);

@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(RW * 32, 2)
                 }
             }
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && k + GSTAGES < nchunks) {
             mbar_expect_tx(&full[s], chunkBytes);
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(RW * 32, 1)
                 }
             }
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && k + ST < nchunks) {
             mbar_expect_tx(&full[s], chunkBytes);
@@ -858,6 +860,7 @@ __global__ void __launch_bounds__(RW * 32, KIND == 1 ? 1 : KIND == 2 ? 3 : 2)
                 dmma(acc[1][0], acc[1][1], a, b1);
             }
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && k + GSTAGES < nchunks) {
             // the MMAs of chunk k have read stage s and B buffer s
@@ -1080,6 +1083,7 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
                     sym_contract<PD>(v[e], st + G::EXPO + e * (E::TILES * 32), lane, acc);
             }
         }
+        refill_fence();
         if (__syncthreads_or(!ok)) {
             if (tid == 0)
                 atomicExch(errorFlag, 1);
@@ -1219,6 +1223,7 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
                 sym_contract<DEG>(v[e], st + G::EXPO + e * (C::TILES * 32), lane, acc);
             }
         }
+        refill_fence();
         if (__syncthreads_or(!ok)) {
             if (tid == 0)
                 atomicExch(errorFlag, 1);

@@ -393,6 +393,7 @@ __global__ void __launch_bounds__(256)
                     psi[(long long)(ql + 1) * nall + c] = isPn ? z1 : exp(z1);
             }
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && t + FLUX_STAGES < nt)
             fbar_load(sB[s], mfA + (size_t)(t0 + t + FLUX_STAGES) * TILE, TILE * 8, &bar[s]);
@@ -511,6 +512,7 @@ __global__ void __launch_bounds__(256)
             for (int j = 0; j < NT; ++j)
                 dmma_g(acc[j][0], acc[j][1], a, B[(kk * NT + j) * 32 + lane]);
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && t + FLUX_STAGES < nt)
             fbar_load(sB[s], mfP + (size_t)(t0 + t + FLUX_STAGES) * TILE, TILE * 8, &bar[s]);
@@ -765,6 +767,7 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
             for (int jj = 0; jj < NT; ++jj)
                 dmma_g(acc[jj][0], acc[jj][1], afr[h], B[(h * NT + jj) * 32 + lane]);
+        refill_fence();
         if (__syncthreads_or(!ok)) {
             if (tid == 0)
                 atomicExch(errorFlag, 1);
@@ -1063,6 +1066,7 @@ __global__ void __launch_bounds__(256)
             for (int j = 0; j < NT; ++j)
                 dmma_g(acc[j][0], acc[j][1], av, sP[st][(kk * NT + j) * 32 + lane]);
         }
+        refill_fence();
         __syncthreads();
         if (tid == 0 && t + FLUX_STAGES < nt)
             fbar_load2(sA[st], mfA + (size_t)(t + FLUX_STAGES) * TA, TA * 8, sP[st],
