@@ -1211,8 +1211,10 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
     cell_sync<S>();
 }
 
+// Returns whether the trial was accepted: the iteration that then begins (unless it regularises)
+// is at the trial's multipliers. A rejected last trial may begin one too, at the old ones.
 template <class S>
-__device__ void after_trial(S &sl, const ClosureParams &P, const Outputs &O, int lane,
+__device__ bool after_trial(S &sl, const ClosureParams &P, const Outputs &O, int lane,
                             double fquad)
 {
     const int nm = P.nm;
@@ -1222,12 +1224,13 @@ __device__ void after_trial(S &sl, const ClosureParams &P, const Outputs &O, int
     cell_sync<S>();
     if (accept) {
         begin_iteration(sl, P, O, lane);
-        return;
+        return true;
     }
     if (lane == 0)
         sl.s.t = 0.5 * t;
     cell_sync<S>();
     next_trial(sl, P, O, lane);
+    return false;
 }
 
 } // namespace

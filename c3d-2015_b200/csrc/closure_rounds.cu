@@ -1425,8 +1425,8 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
             tried = true;
             const bool moments = fused && trial_fused(P, sl.s.fp64, sl.s.iter, sl.s.cnd);
             const int reg = sl.s.regIndex;
-            after_trial(sl, P, O, lane, sl.s.fquad);
-            needH = moments && sl.s.need == NEED_H && sl.s.regIndex == reg;
+            const bool accepted = after_trial(sl, P, O, lane, sl.s.fquad);
+            needH = accepted && moments && sl.s.need == NEED_H && sl.s.regIndex == reg;
             if (!needH) {
                 // on to another pass (or finished): stored before the assembly takes the scratch
                 if (sl.s.need != NEED_NONE)
