@@ -868,7 +868,7 @@ static c3d_status finish_handoff(c3d_ctx *c, bool faceCopy)
         return C3D_OK;
     c->psiHandoffPending = false;
     C3D_CUDA(handoff_launch(c, faceCopy, c->stream));
-    c->launches += faceCopy ? 2 : 1;
+    c->launches += faceCopy ? 3 : 2; // groups, refresh (, face ghosts)
     c->psiReady = true;
     return C3D_OK;
 }
