@@ -296,19 +296,6 @@ __device__ int warp_cholesky_packed(S &sl, int n, int lane)
     return 0;
 }
 
-// l = sqrt(a) and r = 1 / sqrt(a): the root by one correction of a r (within an ulp), off the
-// chain of pivots, which waits for r alone.
-__device__ __forceinline__ void root(double a, double &l, double &r)
-{
-    r = rsqrt(a);
-    if (a > 1e-280 && a < 1e280) {
-        l = a * r;
-        l = fma(fma(-l, l, a), 0.5 * r, l);
-    } else {
-        l = sqrt(a); // zero, negative, not finite, or a square that underflows
-    }
-}
-
 // Blocked Cholesky of the tiled lower triangle (Slot<NT, true>); returns LAPACK info.
 // Per tile column kb: lane l holds row l % 8 of the diagonal tile (the four octets repeat each
 // other) and the 8 columns are factored with shuffles inside the tile; then each lane solves
@@ -316,8 +303,9 @@ __device__ __forceinline__ void root(double a, double &l, double &r)
 // tiles (ib, jb), kb < jb <= ib, receive -L(ib,kb) L(jb,kb)^T as two m8n8k4 DMMAs each (lane l
 // holds L[l/4][4s + l%4] for k-step s, which is the A fragment of L(ib,kb) and the B fragment
 // of L(jb,kb)^T). Every element sees the operations of the column-by-column form in its order.
-// The chain of pivots (square root and reciprocal) bounds it; the loop over tile columns stays
-// rolled so that the code fits the instruction cache.
+// Nothing reads the factor's diagonal: the solves take the reciprocal pivots 1 / L_jj (sl.rinv),
+// and the diagonal's places keep the pivots L_jj^2. The chain of pivots (reciprocal square roots)
+// bounds it; the loop over tile columns stays rolled so that the code fits the instruction cache.
 template <class S>
 __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
 {
@@ -345,11 +333,8 @@ __device__ int warp_cholesky_tiled(S &sl, int n, int lane)
                 const double ajj = cell_shfl<S>(v[j], j);
                 if (!(ajj > 0.0) && info == 0)
                     info = 8 * kb + j + 1;
-                double ljj;
-                root(ajj, ljj, rj[j]);
-                if (row == j)
-                    v[j] = ljj;
-                else if (row > j)
+                rj[j] = rsqrt(ajj);
+                if (row > j)
                     v[j] *= rj[j];
 #pragma unroll
                 for (int c = j + 1; c < 8; ++c) {
