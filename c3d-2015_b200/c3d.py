@@ -49,7 +49,7 @@ HEADER_SYMBOLS = [
     "c3d_set_certificate", "c3d_autotune", "c3d_closure_vectors_noalloc_check",
     "c3d_set_limits", "c3d_set_ansatz_handoff", "c3d_set_graphs", "c3d_group_create",
     "c3d_group_closure_vectors", "c3d_group_step", "c3d_group_destroy", "c3d_stage_part",
-    "c3d_gaunt_build",
+    "c3d_gaunt_build", "c3d_octant_info",
 ]
 
 
@@ -170,6 +170,7 @@ def lib():
         L.c3d_server_destroy.argtypes = [vp]
         L.c3d_solver_output_timings.argtypes = [vp, ctypes.c_char_p]
         L.c3d_solver_output_opt_stats.argtypes = [vp, ctypes.c_char_p]
+        L.c3d_octant_info.argtypes = [vp, _ip, _ip, ctypes.POINTER(ctypes.c_longlong)]
         L.c3d_timing_events.argtypes = [vp, _ip, _dp, ctypes.c_int]
         L.c3d_closure_records_fp.argtypes = [vp, _dp, _dp]
         L.c3d_line_stats_enable.argtypes = [vp, ctypes.c_int]
@@ -333,6 +334,14 @@ class Context:
         s = ClosureStats()
         check(lib().c3d_closure_stats_get(self.h, ctypes.byref(s)), "stats")
         return s
+
+    def octant_info(self):
+        """(flux, closure, visits): whether the kinetic flux and the closure run on the octant
+        kernels, and the closure's visits over the full basis since the last reset."""
+        f, c, v = ctypes.c_int(), ctypes.c_int(), ctypes.c_longlong()
+        check(lib().c3d_octant_info(self.h, ctypes.byref(f), ctypes.byref(c), ctypes.byref(v)),
+              "c3d_octant_info")
+        return bool(f.value), bool(c.value), v.value
 
     def reset_stats(self):
         check(lib().c3d_closure_stats_reset(self.h), "stats reset")

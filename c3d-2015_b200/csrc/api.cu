@@ -2266,6 +2266,23 @@ c3d_status c3d_closure_stats_get(c3d_ctx *c, c3d_closure_stats *st)
     return C3D_OK;
 }
 
+c3d_status c3d_octant_info(c3d_ctx *c, int *flux, int *closure, long long *visits)
+{
+    if (!c)
+        return fail(C3D_ERR_INVALID, "c3d_octant_info: null context");
+    if (flux)
+        *flux = c->symPsi.no > 0;
+    if (closure)
+        *closure = c->engine == 0 && c->gaunt && c->symN.no > 0;
+    if (visits) {
+        unsigned long long h = 0;
+        C3D_CUDA(cudaStreamSynchronize(c->stream));
+        C3D_CUDA(cudaMemcpy(&h, c->stats + STAT_FULL_ORDER, sizeof(h), cudaMemcpyDeviceToHost));
+        *visits = (long long)h;
+    }
+    return C3D_OK;
+}
+
 c3d_status c3d_closure_stats_reset(c3d_ctx *c)
 {
     if (!c)

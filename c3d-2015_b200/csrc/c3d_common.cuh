@@ -44,7 +44,8 @@ enum StatSlot : int {
     STAT_ITER_HIST = 32, // 64 bins (last: >= 63)
     STAT_CLK_NEWTON = 96, // 8 slots, builds with C3D_NEWTON_CLOCKS only: SM clocks of the
                           // work-list Newton kernel's phases (c3d_closure_stats.clkNewton)
-    STAT_COUNT = 104,
+    STAT_FULL_ORDER = 104, // symmetric closure: visits whose pass ran over the full basis
+    STAT_COUNT = 105,
 };
 
 // Closure options (the MN_* deck keys, src/init.cpp:252-258).

@@ -107,9 +107,11 @@ constexpr int NLISTS = 4;
 // keep the reference's order over the full basis. Such cells sit at the realizability boundary
 // (exponents to -1600, condition numbers to 1e9, steps of 1e-3 along directions of 1e6, a few
 // directions carrying the moments), where the rounding of the basis and of the sums decides at
-// which multipliers inside the stopping tolerance the iteration ends: on M_6 pulses with the
-// symmetric passes they ended 1e-8 to 1e-7 from the oracle's, in its order 5e-10 to 5e-9.
-// Standalone vectors with components of unit variance reach 8 (N = 7).
+// which multipliers inside the stopping tolerance the iteration ends: over three steps of M_6
+// pulses on 20^3, 24^3, 26^3 and 28^3 the farthest cell ended 9.4e-8, 1.0e-8, 8.9e-9 and 7.2e-8
+// from the oracle's with the symmetric passes, 1.6e-9, 1.1e-9, 4.3e-9 and 1.7e-8 in its order; on
+// 32^3, where no norm passes 25, 1.0e-10 and 3.7e-11. Standalone vectors with components of unit
+// variance reach 8 (N = 7).
 constexpr double REF_NORM = 32.0;
 struct Lists {
     int *list[NLISTS];
@@ -1505,6 +1507,9 @@ __global__ void __launch_bounds__(NEWTON_THREADS)
             L[e] = H[e];
         cell_sync<SlotT>();
     }
+    // (not fused, symmetric closure: the list of cells far out)
+    if (MODE == 0 && GAUNT && P.sym && !fused && active && lane == 0 && O.stats)
+        atomicAdd(&O.stats[STAT_FULL_ORDER], 1ull);
     if (active && !(tried && !needH)) {
     C3D_NCLK(O.stats, 0, lane);
     if constexpr (MODE == 2) {

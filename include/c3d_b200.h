@@ -201,6 +201,16 @@ c3d_status c3d_closure_records(c3d_ctx *ctx, int *iters, int *iterGamma, int *re
 c3d_status c3d_closure_stats_get(c3d_ctx *ctx, c3d_closure_stats *st);
 c3d_status c3d_closure_stats_reset(c3d_ctx *ctx);
 
+/* The kernels in use (any pointer may be NULL; synchronises when visits is asked for). An even
+ * tensor quadrature in its own order has an octant symmetry that the kinetic flux (*flux 1) and
+ * the work-list closure in the Gaunt form (*closure 1) use; any other set of directions, basis
+ * or beta table (as of a quadrature with fewer than 2N + 1 nodes) takes the general kernels
+ * (0), slower by up to five times. *visits: Hessian and
+ * trial visits of the symmetric closure since creation or the last c3d_closure_stats_reset whose
+ * passes ran over all directions in the reference's order (cells near the realizability boundary,
+ * whose results rounding decides). */
+c3d_status c3d_octant_info(c3d_ctx *ctx, int *flux, int *closure, long long *visits);
+
 /* Switches the closure to the Gaunt form of the Hessian (MN_USE_GAUNT_COEF true,
  * src/opt/fobj.cpp:58-95): extended moments over the harmonics of degree <= 2N, then
  * H_ij = sum_k beta_ijk mom_k in CSR order. M2[nq*nm2] and the CSR table
