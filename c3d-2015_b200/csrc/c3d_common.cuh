@@ -81,6 +81,7 @@ struct ClosureParams {
     int probe;
     int sym;           // octant-symmetric passes (sym.cuh)
     double gramLo, gramHi;
+    double certSlack;  // symmetric passes: |g| of the probe may differ by this from a full visit's
 };
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

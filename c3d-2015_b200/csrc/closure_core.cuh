@@ -1160,7 +1160,9 @@ __device__ void after_probe(S &sl, const ClosureParams &P, const Outputs &O, int
     int maxIterEff = sl.s.maxIter;
     if (P.batched && sl.s.regIndex == P.nreg - 1)
         maxIterEff = 10 * P.maxIter;
-    bool ok = err <= sl.s.rtol && sl.s.iter < maxIterEff && sl.s.t != 0.0 && P.tolGamma > 1.0 &&
+    // (symmetric passes: the full visit's sums may round otherwise, within certSlack; a cell that
+    // close to the tolerance is left to the full visit)
+    bool ok = err + (P.sym ? P.certSlack : 0.0) <= sl.s.rtol && sl.s.iter < maxIterEff && sl.s.t != 0.0 && P.tolGamma > 1.0 &&
               emin > 0.0 && emax < 1.0 / 0.0 && P.gramLo > 0.0;
     double k1 = 0.0, gexp = 0.0;
     if (ok) {

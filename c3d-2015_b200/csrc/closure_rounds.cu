@@ -1241,7 +1241,8 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
         lo = min(lo, __shfl_xor_sync(FULL_MASK, lo, o));
         hi = max(hi, __shfl_xor_sync(FULL_MASK, hi, o));
     }
-    // gradient of the scaled cell (H_i0 / m_0 - u_i = <m_i e^{alpha.m}> - u_i) and its stopping test
+    // gradient of the scaled cell (H_i0 / m_0 - u_i = <m_i e^{alpha.m}> - u_i) and its stopping test,
+    // short of the tolerance by what the roundings of the full visit's form may differ by
     __shared__ unsigned int sCertified;
     if (tid == 0)
         sCertified = 0;
@@ -1275,7 +1276,7 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
     const double lam = 0.5 * emin * P.gramLo, k1 = nm * (emax * P.gramHi) / lam;
     const double minf = sqrt((2 * (DEG + 2) + 1) / (2 * M_PI));
     const double gexp = 2.0 * minf * (DEG + 1) * err / lam;
-    const bool done = gc >= 0 && u0 > 0.0 && err <= rtol && maxIter > 1 && P.passBudget >= 1 &&
+    const bool done = gc >= 0 && u0 > 0.0 && err + P.certSlack <= rtol && maxIter > 1 && P.passBudget >= 1 &&
                       P.tolGamma > 1.0 && emin > 0.0 && emax < 1.0 / 0.0 && P.gramLo > 0.0 &&
                       k1 <= 0.25 * P.condHMax && gexp <= 0.5 * log(P.tolGamma);
     // one list position per cell that goes on, claimed per warp

@@ -269,8 +269,9 @@ c3d_status c3d_set_precision(c3d_ctx *ctx, int mode, double condBf16, double con
  * exponents, e^{alpha.m}, the first-order moments and the extreme values e_min, e_max of
  * e^{alpha.m} over the quadrature -- instead of the Hessian pass. Since H >= e_min G with G the
  * quadrature's Gram matrix, |H^-1 g| and the condition estimate are bounded without H; a cell
- * whose gradient passes the stopping test with these bounds inside the test's thresholds (by
- * factors of 2 and 4) ends exactly as the full iteration would end it -- same multipliers,
+ * whose gradient passes the stopping test (on the octant kernels by 1e-11, above what another
+ * order of the sums moves it; tolerances below that are left to the full visit) with these
+ * bounds inside the test's thresholds (by factors of 2 and 4) ends exactly as the full iteration would end it -- same multipliers,
  * moments, counts and status -- and is finalized without forming or factoring H; its gamma
  * record is then the bound. Other cells continue with the Hessian pass of the same
  * iteration. Off while the x-line statistics log (which records gamma) is enabled. */
