@@ -310,8 +310,8 @@ static void free_ctx(c3d_ctx *c)
 }
 
 // Uploads the tables of a symmetric quadrature (and of another basis over it) into one
-// allocation, *buf (null: a failed allocation; the previous one is freed).
-static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **buf,
+// allocation, *buf (the previous one is freed). The caller waits for the copy (null stream).
+static cudaError_t sym_upload(const SymHost &H, SymTables &T, double **flux, double **buf,
                        const SymHost *H2 = nullptr, SymTables *T2 = nullptr)
 {
     if (*buf)
@@ -332,12 +332,16 @@ static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **b
                 std::memcpy(all.data() + at[k][i], src[i], bytes[i]);
         }
     }
-    if (cudaMalloc(buf, all.size() * 8) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(buf, all.size() * 8);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(*buf, all.data(), all.size() * 8, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
         cudaGetLastError();
+        if (*buf)
+            cudaFree(*buf);
         *buf = nullptr;
-        return;
+        return e;
     }
-    cudaMemcpy(*buf, all.data(), all.size() * 8, cudaMemcpyHostToDevice);
     auto tables = [&](const SymHost &S, const size_t *a) {
         return SymTables{S.no, S.nb, *buf + a[0], *buf + a[1], *buf + a[2],
                          (const int *)(*buf + a[3]), (const int *)(*buf + a[4])};
@@ -347,6 +351,7 @@ static void sym_upload(const SymHost &H, SymTables &T, double **flux, double **b
         *T2 = tables(*H2, at[1]);
     if (flux)
         *flux = *buf + at[0][5];
+    return cudaSuccess;
 }
 
 // Rows of psi a direction chunk takes.
@@ -453,7 +458,7 @@ c3d_status c3d_create(const c3d_params *p, const double *M, const double *w, con
     SymHost sh;
     if (ok && sym_build(c->deg, c->deg, nq, M, w, xi, eta, mu, 1.0 / p->dx, 1.0 / p->dy,
                         1.0 / p->dz, sh))
-        sym_upload(sh, c->symPsi, &c->symFlux, &c->symBuf[0]), ok = c->symBuf[0] != nullptr;
+        ok = sym_upload(sh, c->symPsi, &c->symFlux, &c->symBuf[0]) == cudaSuccess;
     if (ok && pnOps)
         ok = alloc((void **)&c->pnops, (size_t)6 * nm * nm * 8);
     if (!ok) {
@@ -684,7 +689,7 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
                 c->roundsGraph = rounds_graph_new();
             if (!c->launchDev) {
                 C3D_CUDA(cudaMalloc(&c->launchDev, sizeof(unsigned long long)));
-                C3D_CUDA(cudaMemset(c->launchDev, 0, sizeof(unsigned long long)));
+                C3D_CUDA(cudaMemsetAsync(c->launchDev, 0, sizeof(unsigned long long), c->stream));
             }
             R.graphs = c->roundsGraph;
             R.launchDev = c->launchDev;
@@ -704,7 +709,7 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
                     C3D_CUDA(cudaMalloc(&c->psiRefresh, groups * sizeof(long long)));
                     C3D_CUDA(cudaMalloc(&c->psiRefreshCount, sizeof(unsigned int)));
                     C3D_CUDA(cudaMalloc(&c->psiValid, sizeof(int)));
-                    C3D_CUDA(cudaMemset(c->psiValid, 0, sizeof(int)));
+                    C3D_CUDA(cudaMemsetAsync(c->psiValid, 0, sizeof(int), c->stream));
                 }
                 if (!c->psi || c->psiAlloc < need) {
                     if (c->psi)
@@ -713,7 +718,7 @@ static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha
                     c->psiAlloc = 0;
                     C3D_CUDA(cudaMalloc(&c->psi, need));
                     c->psiAlloc = need;
-                    C3D_CUDA(cudaMemset(c->psiValid, 0, sizeof(int)));
+                    C3D_CUDA(cudaMemsetAsync(c->psiValid, 0, sizeof(int), c->stream));
                 }
                 R.psi = c->psi;
                 R.psiNall = c->g.nall();
@@ -895,8 +900,8 @@ static c3d_status ensure_cellmap(c3d_ctx *c)
                 cudaGetLastError();
                 return fail(C3D_ERR_OOM, "c3d_closure: device allocation failed");
             }
-            C3D_CUDA(cudaMemcpy(c->cellMap, map.data(), map.size() * sizeof(int),
-                                cudaMemcpyHostToDevice));
+            C3D_CUDA(cudaMemcpyAsync(c->cellMap, map.data(), map.size() * sizeof(int),
+                                     cudaMemcpyHostToDevice, c->stream));
             c->cellMapCount = (long long)map.size();
         }
     }
@@ -1230,11 +1235,16 @@ c3d_status c3d_set_gaunt(c3d_ctx *c, int nm2, const double *M2, const int *rowPt
     if (c->symPsi.no > 0 &&
         sym_build(c->deg, c->deg, nq, M1.data(), wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h1) &&
         sym_build(2 * c->deg, c->deg, nq, M2, wh.data(), nullptr, nullptr, nullptr, 0, 0, 0, h2)) {
-        sym_upload(h1, c->symN, nullptr, &c->symBuf[1], &h2, &c->sym2);
-        if (!c->symBuf[1])
+        const cudaError_t e = sym_upload(h1, c->symN, nullptr, &c->symBuf[1], &h2, &c->sym2);
+        if (e == cudaErrorMemoryAllocation)
             return fail(C3D_ERR_OOM, "c3d_set_gaunt: device allocation failed");
+        C3D_CUDA(e);
     }
-    return build_certificate(c, nm2, M2, wh, rowPtr, colInd, val);
+    s = build_certificate(c, nm2, M2, wh, rowPtr, colInd, val);
+    // a copy from pageable memory returns once it is staged, and the context's stream does not wait
+    // for the null stream
+    C3D_CUDA(cudaStreamSynchronize(nullptr));
+    return s;
 }
 
 c3d_status c3d_set_precision(c3d_ctx *c, int mode, double condBf16, double condMixedMax,
@@ -1680,7 +1690,7 @@ static c3d_status stage_prepare(c3d_ctx *c, bool *handoff)
         return s;
     if (!c->launchDev) {
         C3D_CUDA(cudaMalloc(&c->launchDev, sizeof(unsigned long long)));
-        C3D_CUDA(cudaMemset(c->launchDev, 0, sizeof(unsigned long long)));
+        C3D_CUDA(cudaMemsetAsync(c->launchDev, 0, sizeof(unsigned long long), c->stream));
     }
     *handoff = Rall.psi != nullptr;
     if (!*handoff) {
@@ -2041,8 +2051,8 @@ static c3d_status ensure_xsplit(c3d_ctx *c)
             cudaGetLastError();
             return fail(C3D_ERR_OOM, "c3d_stage_part: device allocation failed");
         }
-        C3D_CUDA(cudaMemcpy(c->xSplit[w], part[w].data(), part[w].size() * sizeof(int),
-                            cudaMemcpyHostToDevice));
+        C3D_CUDA(cudaMemcpyAsync(c->xSplit[w], part[w].data(), part[w].size() * sizeof(int),
+                                 cudaMemcpyHostToDevice, c->stream));
         c->xSplitCount[w] = (long long)part[w].size();
     }
     return C3D_OK;
