@@ -357,6 +357,13 @@ static cudaError_t sym_upload(const SymHost &H, SymTables &T, double **flux, dou
 // Rows of psi a direction chunk takes.
 static int psi_chunk_rows(const c3d_ctx *c) { return c->qChunk >= c->nq ? c->psi_rows() : c->qChunk; }
 
+// Whether grid closures may copy face ghosts from their images: not where the caller fills the x
+// ghosts, nor on an axis of one cell, whose outer ghost layer lags its image by one exchange.
+static bool mirror_used(const c3d_ctx *c)
+{
+    return c->mirror && !c->xHaloExternal && c->g.nx > 1 && c->g.ny > 1 && c->g.nz > 1;
+}
+
 // psi no longer matches the multipliers (or may not): the next hand-off closure writes all of it.
 static void psi_invalidate(c3d_ctx *c)
 {
@@ -910,7 +917,7 @@ static c3d_status ensure_cellmap(c3d_ctx *c)
 
 static c3d_status closure_grid(c3d_ctx *c)
 {
-    if (c->engine == 0 && c->mirror && !c->xHaloExternal) {
+    if (c->engine == 0 && mirror_used(c)) {
         // Face ghosts hold copies of their periodic images (src/comm.cpp:281-323); when their
         // multipliers (the warm starts) are bitwise those of the images too, the per-cell
         // solve of the reference gives them the images' results, so they are copied after
@@ -1678,7 +1685,7 @@ static bool stage_graphs_usable(const c3d_ctx *c)
 // *handoff: whether the closure hands its ansatz to the flux.
 static c3d_status stage_prepare(c3d_ctx *c, bool *handoff)
 {
-    if (c->mirror && !c->xHaloExternal) {
+    if (mirror_used(c)) {
         c3d_status sm = ensure_cellmap(c);
         if (sm != C3D_OK)
             return sm;
@@ -1718,7 +1725,7 @@ static std::vector<unsigned char> stage_key(const c3d_ctx *c, int stage, double 
         const unsigned char *b = reinterpret_cast<const unsigned char *>(&v);
         key.insert(key.end(), b, b + sizeof(v));
     };
-    const bool mirrorPath = c->mirror && !c->xHaloExternal;
+    const bool mirrorPath = mirror_used(c);
     skey(stage);
     skey(dt);
     skey(c->cp);
@@ -1748,7 +1755,7 @@ static std::vector<unsigned char> stage_key(const c3d_ctx *c, int stage, double 
 static cudaError_t stage_capture(c3d_ctx *c, int stage, double dt, bool handoff, cudaGraph_t top,
                                  cudaStream_t *cs, long long *launches)
 {
-    const bool mirrorPath = c->mirror && !c->xHaloExternal;
+    const bool mirrorPath = mirror_used(c);
     // mirrored closure with the hand-off and the staged stencil: the face ghosts' psi is not
     // copied; the stencil reads their periodic images (the mirror flag tells it, on the device,
     // which closure body ran)

@@ -24,9 +24,23 @@ namespace c3d {
 
 // ---------------------------------------------------------------- ghost fill
 
+// For the ghost cell f of an axis of one cell, where a layer's image may be a ghost itself: the
+// faces per layer, and the layer (0, 1 low outer and inner, 2, 3 high inner and outer). 0 else.
+__device__ __forceinline__ long long one_cell_axis(const GridDims &g, long long f, int &layer)
+{
+    const long long px = (long long)g.ny * g.nz, py = (long long)g.nx * g.nz, pz = (long long)g.nx * g.ny;
+    const long long per = f < 4 * px ? px : f < 4 * (px + py) ? py : pz;
+    const int n = f < 4 * px ? g.nx : f < 4 * (px + py) ? g.ny : g.nz;
+    if (n > 1)
+        return 0;
+    f -= f < 4 * px ? 0 : f < 4 * (px + py) ? 4 * px : 4 * (px + py);
+    layer = (int)(f / per);
+    return per;
+}
+
 // Two periodic ghost layers per face over interior ranges of the other two axes
-// (no edges or corners). The three face groups read only interior cells, so
-// they run as one launch. f0 > 0 skips the first f0 faces: f0 = 4 ny nz leaves the x faces to
+// (no edges or corners). The three face groups read only interior cells (but for an axis of one
+// cell, whose layers one warp copies in order), so they run as one launch. f0 > 0 skips the first f0 faces: f0 = 4 ny nz leaves the x faces to
 // the caller (x-slab decomposition, whose x ghosts come from the neighbouring slabs). One warp
 // per ghost cell: the cell indices cost several 64-bit divisions.
 __global__ void ghost_fill_kernel(GridDims g, double *__restrict__ u, long long f0)
@@ -37,8 +51,27 @@ __global__ void ghost_fill_kernel(GridDims g, double *__restrict__ u, long long 
          f += warps) {
         long long dst, src;
         ghost_pair(g, f, dst, src);
-        for (int m = lane; m < nm; m += 32)
-            u[dst * nm + m] = u[src * nm + m];
+        int layer;
+        const long long per = one_cell_axis(g, f, layer);
+        if (per == 0) {
+            for (int m = lane; m < nm; m += 32)
+                u[dst * nm + m] = u[src * nm + m];
+        } else if (layer == 0) {
+            // low layers, in the reference's order: the outer one takes the inner one's old values
+            long long dst1, src1;
+            ghost_pair(g, f + per, dst1, src1);
+            for (int m = lane; m < nm; m += 32) {
+                u[dst * nm + m] = u[src * nm + m];
+                u[dst1 * nm + m] = u[src1 * nm + m];
+            }
+        } else if (layer >= 2) {
+            // high layers: both end with the cell's values
+            long long near;
+            if (layer == 3)
+                ghost_pair(g, f - per, near, src);
+            for (int m = lane; m < nm; m += 32)
+                u[dst * nm + m] = u[src * nm + m];
+        }
     }
 }
 
