@@ -231,10 +231,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
 }
 
 // Returns false if the phase did not complete within the iteration limit.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int limit = 1 << 26)
 {
     uint32_t addr = smem_u32(bar);
-    for (int it = 0; it < (1 << 26); ++it) {
+    for (int it = 0; it < limit; ++it) {
         uint32_t done;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n"
@@ -253,6 +253,15 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                      smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
+}
+
+// After a wait that gave up at chunk k of n: one thread waits, again with a limit, for the copies
+// in flight in the ring of ST stages (chunk j in stage (seq + j) % ST), which must not land in
+// shared memory that the CTA has given back.
+template <int ST> __device__ __noinline__ void ring_drain(uint64_t *full, uint32_t seq, int k, int n)
+{
+    for (int j = k; j < k + ST && j < n; ++j)
+        mbar_wait(&full[(seq + j) % ST], ((seq + j) / ST) & 1u, 1 << 20);
 }
 
 // ---------------------------------------------------------------- per-warp linear algebra

@@ -115,8 +115,10 @@ __global__ void __launch_bounds__(W * 32, 1)
             if (!mbar_wait(&full[s], parity))
                 s_abort = 1;
             if (__syncthreads_or(s_abort)) {
-                if (tid == 0)
+                if (tid == 0) {
                     atomicExch(errorFlag, 1);
+                    ring_drain<STAGES>(full, seq, k, nchunks);
+                }
                 return;
             }
             const double *ch = stage + s * CH;
@@ -287,8 +289,10 @@ __global__ void __launch_bounds__(W * 32, 1)
             if (!mbar_wait(&full[s], parity))
                 s_abort = 1;
             if (__syncthreads_or(s_abort)) {
-                if (tid == 0)
+                if (tid == 0) {
                     atomicExch(errorFlag, 1);
+                    ring_drain<GSTAGES>(full, seq, k, nchunks);
+                }
                 return;
             }
             const double *ch = stage + s * CH;
@@ -422,8 +426,10 @@ __global__ void __launch_bounds__(W * 32, 1)
         if (!mbar_wait(&full[s], parity))
             s_abort = 1;
         if (__syncthreads_or(s_abort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<STAGES>(full, 0, k, nchunks);
+            }
             return;
         }
         const double *ch = stage + s * CH;
@@ -529,8 +535,10 @@ __global__ void __launch_bounds__(256, 1)
         if (!mbar_wait(&full[s], parity))
             s_abort = 1;
         if (__syncthreads_or(s_abort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<GSTAGES>(full, 0, k, nchunks);
+            }
             return;
         }
         const double *ch = stage + s * CH;

@@ -285,8 +285,10 @@ __global__ void __launch_bounds__(RW * 32, 2)
         if (!mbar_wait(&full[s], parity))
             s_abort = 1;
         if (__syncthreads_or(s_abort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<GSTAGES>(full, 0, k, nchunks);
+            }
             return;
         }
         const double *ch = stage + s * CH;
@@ -418,8 +420,10 @@ __global__ void __launch_bounds__(RW * 32, 1)
         if (!mbar_wait(&full[s], parity))
             s_abort = 1;
         if (__syncthreads_or(s_abort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<ST>(full, 0, k, nchunks);
+            }
             return;
         }
         const double *ch = stage + s * CH;
@@ -730,8 +734,11 @@ __global__ void __launch_bounds__(RW * 32, KIND == 1 ? 1 : KIND == 2 ? 3 : 2)
         if constexpr (KIND == 2 && ZD)
             if (rd)
                 cp_async_wait<1>(); // this thread's copies of chunk k have landed
-        if (__syncthreads_or(s_abort))
+        if (__syncthreads_or(s_abort)) {
+            if (tid == 0)
+                ring_drain<GSTAGES>(full, 0, k, nchunks);
             break;
+        }
         const unsigned char *stb = smem_raw + s * stg;
         const double *ch = reinterpret_cast<const double *>(stb);
         double z0 = 0.0, z1 = 0.0, ez0 = 0.0, ez1 = 0.0;
@@ -1087,8 +1094,10 @@ __global__ void __launch_bounds__(SYM_PASS_WARPS * 32, NT2 > 16 ? 2 : 4)
         }
         refill_fence();
         if (__syncthreads_or(!ok)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<SYM_STAGES>(full, 0, b, T.nb);
+            }
             return;
         }
         if (tid == 0 && b + SYM_STAGES < T.nb)
@@ -1227,8 +1236,10 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
         }
         refill_fence();
         if (__syncthreads_or(!ok)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                ring_drain<SYM_STAGES>(full, 0, b, T.nb);
+            }
             return;
         }
         if (tid == 0 && b + SYM_STAGES < T.nb)

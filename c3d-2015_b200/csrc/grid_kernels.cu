@@ -353,9 +353,9 @@ __device__ __forceinline__ void fbar_load2(void *dst0, const void *src0, uint32_
                  : "memory");
 }
 // false if the phase did not complete within the iteration limit
-__device__ __forceinline__ bool fbar_wait(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ bool fbar_wait(uint64_t *bar, uint32_t parity, int limit = 1 << 26)
 {
-    for (int it = 0; it < (1 << 26); ++it) {
+    for (int it = 0; it < limit; ++it) {
         uint32_t done;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n"
@@ -366,6 +366,14 @@ __device__ __forceinline__ bool fbar_wait(uint64_t *bar, uint32_t parity)
             return true;
     }
     return false;
+}
+
+// After a wait that gave up at tile k of n: one thread waits, again with a limit, for the copies in
+// flight in the FLUX_STAGES stages (as ring_drain, closure_core.cuh).
+__device__ __noinline__ void fbar_drain(uint64_t *bar, int k, int n)
+{
+    for (int j = k; j < k + FLUX_STAGES && j < n; ++j)
+        fbar_wait(&bar[j % FLUX_STAGES], (j / FLUX_STAGES) & 1, 1 << 20);
 }
 
 // psi[(q - q0) nall + c] = exp(alpha_c . m_q) (M_N) or alpha_c . m_q (P_N) for the directions
@@ -407,8 +415,10 @@ __global__ void __launch_bounds__(256)
         if (!fbar_wait(&bar[s], (t / FLUX_STAGES) & 1))
             sAbort = 1;
         if (__syncthreads_or(sAbort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                fbar_drain(bar, t, nt);
+            }
             return;
         }
         const double *B = sB[s];
@@ -516,8 +526,10 @@ __global__ void __launch_bounds__(256)
         if (!fbar_wait(&bar[s], (t / FLUX_STAGES) & 1))
             sAbort = 1;
         if (__syncthreads_or(sAbort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                fbar_drain(bar, t, nt);
+            }
             return;
         }
         const double *dirs = sB[s] + 8 * NT * 32; // c_x, c_y, c_z, w per direction
@@ -609,6 +621,7 @@ __device__ __forceinline__ double axis_flux_m3(double q, double th2, double k1, 
 // DMMAs straight from its registers (k-steps 2v, 2v + 1 of the 32-direction fragment tile, in
 // order), so the flux has the same values as kinetic_dmma_kernel's. One barrier per sub-stage,
 // before its buffers are refilled.
+static_assert(FLUX_STAGES == 2, "kinetic_staged_kernel rings two sub-stages");
 constexpr int KDS = 8;                      // directions per sub-stage
 constexpr int KRUN = 64;                    // longest cell run per CTA
 // doubles staged per direction: the runs back to back (KPER = 4 mod 16, so the four directions
@@ -802,8 +815,10 @@ __global__ void __launch_bounds__(256, 3)
                 dmma_g(acc[jj][0], acc[jj][1], afr[h], B[(h * NT + jj) * 32 + lane]);
         refill_fence();
         if (__syncthreads_or(!ok)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                fbar_drain(pbar, u, nu);
+            }
             return;
         }
         if (u + 2 < nu)
@@ -1076,8 +1091,10 @@ __global__ void __launch_bounds__(256)
         if (!fbar_wait(&bar[st], (t / FLUX_STAGES) & 1))
             sAbort = 1;
         if (__syncthreads_or(sAbort)) {
-            if (tid == 0)
+            if (tid == 0) {
                 atomicExch(errorFlag, 1);
+                fbar_drain(bar, t, nt);
+            }
             return;
         }
         const double *w = sP[st] + 8 * NT * 32 + 96;
