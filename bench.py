@@ -179,6 +179,54 @@ def closure_flops(nm, nq, iters, trials, hessian="gaunt", certified=0):
     return (iters - certified) * per_iter + certified * per_cert + trials * per_trial
 
 
+# The octant form (c3d-2015_b200/csrc/sym.cuh): per cell and octant direction, of which there are
+# nq / 8, the FP64 FLOPs the kernels do, padding of the class tiles included.
+def _octant_classes(deg):
+    """Members of the 8 parity classes of the harmonics of degree <= deg."""
+    n = [0] * 8
+    for l in range(deg + 1):
+        for m in range(-l, l + 1):
+            a = abs(m)
+            n[((a if m >= 0 else a + 1) & 1) | (2 if m < 0 else 0) | (4 * ((l + a) & 1))] += 1
+    return n
+
+
+def _octant_tiles(deg):
+    return sum((n + 7) // 8 for n in _octant_classes(deg))
+
+
+def octant_pass_flops(nm, nq, deg):
+    """One cell's pass: exponents (DMMA steps of 4 class members, a transform), 8 exponentials (1
+    FLOP each) and weights, a transform, and the projection onto the class tiles of degree deg
+    (None: the sum alone)."""
+    N = int(round(nm ** 0.5)) - 1
+    steps = sum((n + 3) // 4 for n in _octant_classes(N))
+    return nq / 8.0 * (8 * steps + 24 + 8 + 8 + 24 + (0 if deg is None else 16 * _octant_tiles(deg)))
+
+
+def octant_closure_flops(nm, nq, st, solved, mixed):
+    """The closure's FP64 FLOPs on the octant kernels (solved: the share of the counted cells that
+    were solved, not copied from their images). FP64: a probe per cell, a pass per first visit that
+    the certificate did not end and per trial (its moments serve the next visit). Mixed: a pass per
+    FP64 Hessian, per trial the sum alone, per reduced-precision Hessian every direction's exponent
+    (2 nm nq), exponential and first-order moments (2 nm nq)."""
+    N = int(round(nm ** 0.5)) - 1
+    f = st.cells * solved * octant_pass_flops(nm, nq, N)
+    f += (st.totalIters - st.certified) * nm ** 3 / 3.0
+    if not mixed:
+        return f + (st.trials + st.cells - st.certified) * octant_pass_flops(nm, nq, 2 * N)
+    return (f + st.hessFp64 * octant_pass_flops(nm, nq, 2 * N)
+            + st.trials * octant_pass_flops(nm, nq, None)
+            + (st.hessBf16 + st.hessTf32x3) * (4 * nm * nq + nq))
+
+
+def octant_stencil_flops(nm, nq):
+    """The symmetric stencil per cell: 60 for the three axes' limited differences per direction, per
+    octant direction a transform and the projection onto the class tiles."""
+    N = int(round(nm ** 0.5)) - 1
+    return 60.0 * nq + nq / 8.0 * (24 + 16 * _octant_tiles(N))
+
+
 def _hbm_peak_gbs():
     try:
         with open(os.path.join(REPO, "MEASURED_PEAKS.json")) as f:
@@ -913,17 +961,23 @@ def b200_arm(args):
         else:
             flops = closure_flops(nm, nq, sst.totalIters, sst.trials, args.hessian, sst.certified)
         per_launch_s = ms[0] * 1e-3 / max(1, closure_launches)
+        n_ = CONFIGS[cfg]["n"]
+        face_ghosts = 12 * n_ * n_  # two layers on each of the six faces
+        octf, octc = ctypes.c_int(), ctypes.c_int()
+        c3d.check(c3d.lib().c3d_octant_info(solver.ctx_handle, ctypes.byref(octf),
+                                            ctypes.byref(octc), None), "octant_info")
+        full_flops = flops  # over all directions
+        if octc.value:
+            flops = octant_closure_flops(nm, nq, sst, 1.0 - face_ghosts / solver.nall,
+                                         precision == 1)
         achieved = flops / max(1, closure_launches) / per_launch_s / 1e12
         closure_roofline = dict(
-            bound="tensor",
+            bound="fp64 pipe",
             pipe=("fp64 (DMMA m8n8k4 + DFMA); the mixed closure's BF16 / 3xTF32 moments run on "
                   "tcgen05 beside it (lowp_tflops)" if precision == 1
                   else "fp64 (DMMA m8n8k4 + DFMA)"),
             achieved=achieved, peak=peak, unit="TFLOP/s", frac=achieved / peak if peak else None,
-            traffic=(profile_traffic("sym_kernels_m6_64")
-                     if args.engine == "rounds" and args.hessian == "gaunt" else None),
-            traffic_source="profiles/sym_kernels_m6_64.txt: the probe pass's DRAM bytes at 64^3 "
-                           "(ncu) scaled by solved cells to 128^3",
+            traffic=None, traffic_source="not captured for all kernels of a closure",
             peak_source="in-run cuBLAS DGEMM 8192^3 via torch (FP64 is not in "
                         "MEASURED_PEAKS.json)",
             kernel=(("closure work-list rounds: sym_probe_kernel<7,22> (first visits) + "
@@ -937,6 +991,11 @@ def b200_arm(args):
             flops_per_launch=flops / max(1, closure_launches),
             ms_per_launch=ms[0] / max(1, closure_launches),
             share_of_step=ms[0] / split["max_ms"])
+        if octc.value:
+            closure_roofline["equivalent_unsymmetrised"] = dict(
+                tflops=full_flops / max(1, closure_launches) / per_launch_s / 1e12,
+                note="the same closure's FLOPs over all directions, of which the octant form does "
+                     "about a sixth")
         if low is not None:
             closure_roofline["lowp_tflops"] = low / max(1, closure_launches) / per_launch_s / 1e12
             closure_roofline["kernel"] = (
@@ -973,21 +1032,22 @@ def b200_arm(args):
                               "matches the C oracle to 1e-12 (tests)")
         # the dominant kernel: the kinetic flux's stencil + projection (sym_flux_kernel),
         # one launch per flux call when the closure handed its ansatz over (psi of all
-        # directions within the 32 GiB budget). Algorithmic work per (cell, direction):
-        # 2 nm FLOPs of projection + 60 of the three axes' limited upwind differences; bytes:
-        # psi of the interior cells and the two face-ghost layers read once, the flux written.
-        n_ = CONFIGS[cfg]["n"]
-        face_ghosts = 12 * n_ * n_  # two layers on each of the six faces
-        handoff = solver.nall * nq * 8 <= (32 << 30)
+        # directions within the 32 GiB budget). FLOPs: octant_stencil_flops, or over all directions
+        # 2 nm of projection + 60 of the limited differences each; bytes: psi of the interior cells
+        # and the two face-ghost layers read once, the flux written.
+        handoff = solver.nall * ((nq + 31) // 32 * 32) * 8 <= (32 << 30)
         flux_ms = ms[1] / max(1, int(cnt[1]))
-        stencil_flops = float((2 * nm + 60) * nq) * cells
+        full_stencil = float((2 * nm + 60) * nq) * cells
+        stencil_flops = octant_stencil_flops(nm, nq) * cells if octf.value else full_stencil
         stencil_bytes = 8.0 * ((cells + face_ghosts) * nq + cells * nm)
         achieved_k = stencil_flops / (flux_ms * 1e-3) / 1e12
         traffic_k = profile_traffic("sym_kernels_m6_64", "dram_bytes_per_launch:")
         if traffic_k is not None:
             traffic_k *= cells / 64 ** 3  # ncu capture at 64^3, scaled by (cell, direction) pairs
         roofline = dict(
-            bound="tensor", pipe="fp64 (DMMA m8n8k4 projection + DFMA/ALU limiter)",
+            bound="fp64 pipe",
+            pipe="fp64 (DMMA m8n8k4 projection + DFMA/ALU limiter): the shared FP64 pipe 47% busy, "
+                 "the ALU 51%, issue 0.62 per clock and scheduler (ncu)",
             kernel="sym_flux_kernel<6,4> (kinetic flux: MUSCL stencil + projection)",
             achieved=achieved_k, peak=peak, unit="TFLOP/s",
             frac=achieved_k / peak if peak else None,
@@ -998,7 +1058,10 @@ def b200_arm(args):
             peak_source="in-run cuBLAS DGEMM 8192^3 via torch (FP64 is not in "
                         "MEASURED_PEAKS.json)",
             flops_per_launch=stencil_flops,
-            flops_per_cell_direction=2 * nm + 60,
+            flops_per_cell_direction=stencil_flops / cells / nq,
+            equivalent_unsymmetrised=dict(
+                flops_per_launch=full_stencil, tflops=full_stencil / (flux_ms * 1e-3) / 1e12,
+                note="with the projection over all directions, which the octant form does not do"),
             ms_per_launch=flux_ms, stencil_only=handoff,
             share_of_step=ms[1] / split["max_ms"],
             hbm=dict(algorithmic_bytes_per_launch=stencil_bytes,
@@ -1006,8 +1069,7 @@ def b200_arm(args):
                      peak_gbs=HBM_PEAK_GBS,
                      frac=stencil_bytes / (flux_ms * 1e-3) / 1e9 / HBM_PEAK_GBS,
                      peak_source="MEASURED_PEAKS.json hbm_gbs (of measured)"),
-            note="FP64-pipe and issue bound (ncu: FP64 pipe, ALU and shared-memory wavefronts "
-                 "busy, DRAM idle most of the launch); the closure is second "
+            note="bound by the FP64 pipe's latency and issue, DRAM 30% (ncu); the closure is second "
                  "(closure_roofline)")
         # CPU baseline: the reference closure on a bounded sample of this workload's cells
         cpu = None
