@@ -20,13 +20,13 @@ def test_octant_classes_hold_every_harmonic(N):
 
 
 def test_m6_counts_are_the_kernels():
-    """M_6, 1568 directions: a probe expands a cell with 15 DMMA steps and projects onto 9 tiles (18
-    DMMAs per block of 8 octant directions and 8 cells), a pass onto 24; 33 DMMAs of 512 FLOPs per block are
-    8 * 64 * 33 / 64 = 264 FLOPs per cell and octant direction."""
+    """M_6, classes of 10, 6 (six times) and 3 members: per block of 8 octant directions and 8 cells a
+    probe expands with 3 + 6 * 2 + 1 = 16 DMMAs and projects onto 2 + 7 = 9 tiles, twice; a pass onto
+    24. A DMMA has 512 FLOPs, a block 64 pairs of cell and octant direction."""
     nm, nq = 49, 1568
     other = nq / 8 * (24 + 8 + 8 + 24)
-    assert bench.octant_pass_flops(nm, nq, 6) - other == nq / 8 * 33 * 512 / 64
-    assert bench.octant_pass_flops(nm, nq, 12) - other == nq / 8 * (15 + 48) * 512 / 64
+    assert bench.octant_pass_flops(nm, nq, 6) - other == nq / 8 * (16 + 2 * 9) * 512 / 64
+    assert bench.octant_pass_flops(nm, nq, 12) - other == nq / 8 * (16 + 2 * 24) * 512 / 64
     assert bench.octant_stencil_flops(nm, nq) == nq * 60 + nq / 8 * (24 + 9 * 16)
 
 
