@@ -633,9 +633,8 @@ static c3d_status ensure_rounds(c3d_ctx *c, long long n)
 
 // gridRecords: the closure covers the context's grid (directly or through cellMap), so the
 // per-cell gamma and |g| records of the context (nall entries) receive its results.
-// The work-list closure of n cells (engine 0): buffers sized, the launch description filled;
-// the hand-off's refresh count is cleared on st (the stream the closure will run on, or the
-// stream capturing it).
+// The work-list closure of n cells (engine 0): buffers sized, the launch description filled for
+// st (the stream the closure will run on, or the stream capturing it).
 static c3d_status rounds_setup(c3d_ctx *c, long long n, double *u, double *alpha, int *iters,
                                int *iterGamma, int *regIdx, int *status, const int *cellMap,
                                bool gridRecords, cudaStream_t st, RoundsLaunch &R)
@@ -1584,7 +1583,7 @@ c3d_status c3d_autotune(c3d_ctx *c, int *qChunk, int *runLen, double *msPerCall)
     }
     std::vector<int> ls{0};
     if (c->symPsi.no == 0 && c->g.nz % 32 == 0 && c->g.nz > 32)
-        ls.push_back(32); // (the symmetric stencil has one tile shape)
+        ls.push_back(32); // (the symmetric stencil takes its tiles by the grid's size)
     const int q0 = c->qChunk, l0 = c->runLen;
     const bool timing = c->timing;
     c->psiReady = false; // every timed call forms the ansatz

@@ -6,14 +6,14 @@
 //   init kernel    per cell: scale u and alpha (preProcess, src/opt/optBatch.cpp:312-331),
 //                  start the first Newton iteration, append the cell to the work list;
 //   pass kernel    per listed cell: exponents alpha.m_q and either the extended moments
-//                  of the Gaunt form (one DMMA GEMM for the 8 cells of a CTA, shared
-//                  staged M2^T chunks) or the direct Hessian tiles, or the trial's f;
-//   Newton kernel  one warp per listed cell: assemble H, Cholesky, condition estimate,
+//                  of the Gaunt form (DMMA, 8 cells per warp over the staged octant tables, or 16
+//                  per CTA over staged M2^T chunks) or the direct Hessian tiles, or the trial's f;
+//   Newton kernel  8, 16 or 32 lanes per listed cell: assemble H, Cholesky, condition estimate,
 //                  direction, stop tests, Armijo (solveTheRest, src/opt/optBatch.cpp:143-283)
 //                  with the state machine shared with the persistent kernels; cells that
 //                  need another pass are appended to the next round's list.
 // Separating the passes (tensor-pipe work, small shared memory) from the per-cell logic
-// (latency-bound, one warp per cell) lets each run at its own occupancy; a cell that
+// (latency-bound, serial chains per cell) lets each run at its own occupancy; a cell that
 // needs many iterations only ever occupies the short lists of later rounds.
 #include "closure_core.cuh"
 
@@ -1356,8 +1356,10 @@ __global__ void __launch_bounds__(SYM_PROBE_WARPS * 32, 4)
 // 1 BF16, 2 3xTF32, 3 probe).
 // GAUNT: the CTA assembles H_ij = sum_k beta_ijk mom_k (i >= j, the CSR terms of beta in
 // the order of src/opt/fobj.cpp:81-99, laid out per tile slot by c3d_set_gaunt) for its
-// cells that need a Hessian in one sweep over the tile slots per four cells. The cells' moments sit in the slots' g..rinv vectors, which a Hessian visit
-// recomputes afterwards. Otherwise the pass wrote H in tiles to hBuf.
+// cells that need a Hessian in one sweep over the tile slots per four cells. The cells' moments
+// sit in the slots' g..rinv vectors, which a Hessian visit recomputes afterwards. Otherwise the pass
+// wrote H in tiles to hBuf. fused: the symmetric passes' list 0 (moments at trial points, bounds of
+// e^{alpha.m} behind the moments).
 template <int NT, int NT2, bool GAUNT, int MODE>
 __global__ void __launch_bounds__(NEWTON_THREADS)
     rounds_newton_kernel(ClosureParams P, double m0, const int *__restrict__ list, int n,

@@ -85,7 +85,8 @@ __host__ __device__ inline int sym_direction(int Q, int o)
 //                                    4 zeros of the group's directions (the kinetic flux)
 //   w     [block][position]          weights of the octant directions (0 past the last)
 //   idx   [tile][8]                  column of each class member, -1 padding
-// Degree: expo, flux and projN/idxN the basis', proj2/idx2 twice that (Gaunt form).
+// Degrees: expo and stepIdx the basis' N; proj and idx N (the flux, the probe) or 2N (the Hessian
+// passes of the Gaunt form).
 struct SymTables {
     int no, nb; // octant directions, blocks
     const double *expo, *proj, *w;

@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(128)
 // ---------------------------------------------------------------- stencil and projection
 
 // Slope of the limited reconstruction at a value with differences dm (to its upwind neighbour),
-// dp (to its downwind one) and dc across both, times 4: minmod(th dp, dc / 2, th dm)
-// (src/flux_kinetic.cpp:45-61) scaled by 2, th2 = 2 th >= 0, for dm and dp of one sign (dc then
+// dp (to its downwind one) and dc across both, times 2: 2 minmod(th dp, dc / 2, th dm) =
+// minmod(th2 dp, dc, th2 dm) (src/flux_kinetic.cpp:45-61), th2 = 2 th >= 0, for dm and dp of one sign (dc then
 // has it too, and min(th |dm|, th |dp|) = th min(|dm|, |dp|)); otherwise it is 0. (The selects as
 // predicated FP64 operations: 24 instructions fewer per cell and direction, 7% slower, since 12
 // more go to the FP64 pipe.)
@@ -125,7 +125,7 @@ __device__ __forceinline__ void sym_add_same(double &f, double q, double s, doub
 
 // Limited upwind difference along one axis in upwind coordinates, v2, v1 the upwind
 // neighbours, v0 the cell, w1 the downwind neighbour:
-//   f = (v0 + s(v1, v0, w1) / 2) - (v1 + s(v2, v1, v0) / 2),
+//   f = (v0 + s(v1, v0, w1) / 2) - (v1 + s(v2, v1, v0) / 2)  (s / 2 = sym_slope / 4),
 // summed from the difference v0 - v1, which the slopes need too, so that a zero slope is a
 // predicated-off FMA instead of a select.
 // A direction of the opposite sign gives the mirror image with f and the cosine both negated,

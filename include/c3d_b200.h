@@ -260,7 +260,11 @@ c3d_status c3d_set_engine(c3d_ctx *ctx, int engine);
  * moments, and the cell keeps them for the rest of the closure, so that the last steps
  * converge quadratically as in mode 0 and the moments track mode 0's closely. Values <= 0
  * select the defaults. For N <= 2 the Hessian moments stay FP64 (the tensor-core tile would
- * be mostly padding). */
+ * be mostly padding).
+ * Mode 1 costs time on the octant kernels (c3d_octant_info), whose FP64 passes are cheaper than
+ * the reduced-precision ones: it runs at 0.96 of mode 0's rate on an M_6 128^3 step, 0.77 on
+ * standalone vectors of the orders 1 to 7 and 0.71 on the serving workload; a visit's pass at
+ * N = 7 takes 18 ns (BF16) or 33 (3xTF32) against 6.5. */
 c3d_status c3d_set_precision(c3d_ctx *ctx, int mode, double condBf16, double condMixedMax,
                              int mixedIterMax, double polish);
 
@@ -329,8 +333,9 @@ c3d_status c3d_set_limits(c3d_ctx *ctx, long long maxRounds, long long passBudge
  * image's bit for bit -- checked on the device before each closure -- its solve would
  * reproduce the image's; the closure then solves the other cells and copies multipliers,
  * regularised moments and records to the face ghosts, whose records also enter the closure
- * statistics. Results and statistics are identical either way. No counterpart in the
- * reference. */
+ * statistics. Results and statistics are identical either way. Not used on grids with an axis
+ * of one cell, whose outer ghost layer holds what the inner one held before the last exchange
+ * (src/comm.cpp:281-323). No counterpart in the reference. */
 c3d_status c3d_set_ghost_mirroring(c3d_ctx *ctx, int on);
 
 /* Standalone batched closure of n independent moment vectors (device

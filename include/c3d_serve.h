@@ -3,8 +3,8 @@
  * process): independent transport problems, each given as input.deck text, are admitted
  * against a device-memory budget and keep their state on the device from submission to
  * completion. One scheduling thread advances every admitted problem by one time step per pass,
- * the M_N problems together in ONE launch: a CUDA graph whose parallel branches are their RK
- * steps (c3d_group_step), rebuilt when the set of problems changes. While the GPU runs a pass
+ * the M_N problems together in ONE launch: a CUDA graph that holds their RK steps one after
+ * another (c3d_group_step), rebuilt when the set of problems changes. While the GPU runs a pass
  * the thread admits the requests that arrived (in arrival order, while the active problems'
  * estimated footprints leave room), which join the next pass; problems that took their last
  * step leave after it. Each problem's result is what c3d_solver_run gives for it alone, bit for
